@@ -49,3 +49,23 @@ def test_exact_sum_at_grid_points_equals_inverse_transform(torch):
     got = p.exact_sum(cube, torch.as_tensor(pos).cuda()).cpu().numpy()
     ref = u[:, idx[:, 0], idx[:, 1], idx[:, 2]].T
     assert np.abs(got - ref).max() / np.abs(ref).max() < 1e-12
+
+
+# edges of the points' tiles (128 per block up to kc = 93, 64 beyond) and of the kz tiles of 8 and
+# ky steps of 4 (kc = 5, 32, 120): FP64 products of at most 2 kc + 1 terms of size |u| each row, so
+# the difference stays within a few hundred roundings of the sum of magnitudes
+@pytest.mark.parametrize("N,npts", [(16, 1), (16, 129), (96, 127), (96, 300), (360, 65)])
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_exact_sum_tile_edges(torch, N, npts, prec):
+    from lucky_droplets_b200.spectral import Plan
+    p = Plan(N, prec)
+    g = torch.Generator(device="cuda").manual_seed(N)
+    cube = p.empty_cube(3)  # modes outside the mask and a kz = 0 plane without symmetry included
+    cube.real.normal_(generator=g)
+    cube.imag.normal_(generator=g)
+    rng = np.random.default_rng(npts)
+    pos = rng.uniform(-1.0, 2 * np.pi + 1.0, (npts, 3))
+    masked = p.to_cube(p.from_cube(cube))
+    got = p.exact_sum(cube, torch.as_tensor(pos).cuda()).cpu().numpy()
+    ref = X.exact_sum(p.from_cube(masked).cpu().numpy().astype(np.complex128), pos)
+    assert np.abs(got - ref).max() / np.abs(ref).max() < 1e-12
