@@ -14,9 +14,9 @@
 //   wide      droplets with 2 r > cell width ("wide"; none when the cell width is at least twice
 //             the largest radius) also search the cells within 2 r of them for the partners
 //             with ri + rj > cell width, which the neighbour search leaves out: counted by the
-//             block of the column visit that meets them, emitted by the block of the emit pass
+//             warp of the count pass that meets them, emitted by the block of the emit pass
 //   emit      pairs at offset + t in the fixed visiting order (copied from the record, or searched
-//             again for droplets with more partners), then mapped to droplet ids (i < j)
+//             again for droplets with more partners), as droplet ids (i < j)
 // The FP64 arithmetic (wrap, cell index, minimum image, squared distance) is done with explicit
 // round-to-nearest operations and no fused multiply-add, in the same order as the CPU rule, so
 // the pair list is bit-exact given identical inputs.
@@ -94,27 +94,30 @@ __device__ __forceinline__ void sorted_slot(long long s, unsigned k, unsigned i,
 
 constexpr int kSmallCell = 64;  // cells up to this occupancy are placed by rank counting
 
-// Thread per droplet (index order): its place in the sorted order is its cell's start plus the
-// number of the cell's droplets with a smaller index, counted over the cell's unordered run;
-// writes the sorted index, key and copies there.  Cells above kSmallCell droplets are left to
-// k_cell_big (the droplet in the run's first slot appends the cell to `big`).
+// Thread per slot of the unordered runs: the slot's droplet goes to its cell's start plus the
+// number of the cell's droplets with a smaller index, counted over the run; the sorted index, key
+// and copies are written there.  By slots, the writes (56 bytes a droplet) stay inside the cell and
+// only the droplet's own data are read from scattered addresses: 1e6 droplets in random order 53 ->
+// 33 us against a thread per droplet (already sorted ones 22 -> 20).  Cells above kSmallCell droplets are left to k_cell_big (the
+// thread of the run's first slot appends the cell to `big`).
 __global__ void k_cell_place(const unsigned* __restrict__ key, const int* __restrict__ cs,
                              const unsigned* __restrict__ run, long long n, const double* __restrict__ pos,
                              const double* __restrict__ rad, double L, unsigned* __restrict__ sval,
                              unsigned* __restrict__ skey, double4* __restrict__ sp, float4* __restrict__ spf,
                              unsigned* __restrict__ big, unsigned* __restrict__ nbig) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const unsigned i = run[t];
     const unsigned k = key[i];
     const int s0 = cs[k], s1 = cs[k + 1];
     if (s1 - s0 > kSmallCell) {
-      if (run[s0] == (unsigned)i) big[atomicAdd(nbig, 1u)] = k;
+      if (s0 == (int)t) big[atomicAdd(nbig, 1u)] = k;
       continue;
     }
     int r = 0;
-    for (int j = s0; j < s1; ++j) r += run[j] < (unsigned)i ? 1 : 0;
+    for (int j = s0; j < s1; ++j) r += run[j] < i ? 1 : 0;
     const int s = s0 + r;
-    sval[s] = (unsigned)i;
-    sorted_slot(s, k, (unsigned)i, pos, rad, L, skey, sp, spf);
+    sval[s] = i;
+    sorted_slot(s, k, i, pos, rad, L, skey, sp, spf);
   }
 }
 
@@ -168,20 +171,50 @@ k_rs_hist(const unsigned* __restrict__ key, long long n, int shift, unsigned* __
   hist[threadIdx.x * (long long)nblocks + blockIdx.x] = cnt[threadIdx.x];
 }
 
-// Multi-block exclusive scan, phase 1: each block scans a tile of SCAN_TILE counts in place and
-// writes the tile total to sums[blockIdx.x].
+// Multi-block exclusive scan in two launches: the totals of the tiles of SCAN_TILE counts, then
+// every block adds up the totals before its own tile (at most SCAN_TILE of them, a few per thread)
+// and scans its tile in place.
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_PER = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_PER;
 
+// sum of v over the block (every thread gets it); w: 32 words of shared memory
+__device__ __forceinline__ unsigned scan_block_sum(unsigned v, unsigned* w) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = w[threadIdx.x & 31];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  return v;
+}
+
 __global__ void __launch_bounds__(SCAN_THREADS)
-k_scan_tiles(unsigned* __restrict__ a, long long m, unsigned* __restrict__ sums) {
+k_scan_totals(const unsigned* __restrict__ a, long long m, unsigned* __restrict__ sums) {
+  __shared__ unsigned w[32];
+  const long long base = (long long)blockIdx.x * SCAN_TILE;
+  unsigned v = 0;
+#pragma unroll
+  for (int q = 0; q < SCAN_PER; ++q) {
+    const long long i = base + q * SCAN_THREADS + threadIdx.x;
+    v += i < m ? a[i] : 0u;
+  }
+  v = scan_block_sum(v, w);
+  if (threadIdx.x == 0) sums[blockIdx.x] = v;
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS)
+k_scan_tiles(unsigned* __restrict__ a, long long m, const unsigned* __restrict__ sums) {
   __shared__ unsigned buf[SCAN_TILE];
   __shared__ unsigned wsum[SCAN_THREADS / 32];
   const long long base = (long long)blockIdx.x * SCAN_TILE;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   for (int i = t; i < SCAN_TILE; i += SCAN_THREADS) buf[i] = base + i < m ? a[base + i] : 0u;
-  __syncthreads();
+  unsigned tiles = 0;
+  for (int i = t; i < (int)blockIdx.x; i += SCAN_THREADS) tiles += sums[i];
+  tiles = scan_block_sum(tiles, wsum);  // its barriers make buf visible too
   unsigned v[SCAN_PER];
   unsigned run = 0;
 #pragma unroll
@@ -196,28 +229,21 @@ k_scan_tiles(unsigned* __restrict__ a, long long m, unsigned* __restrict__ sums)
   if (lane == 31) wsum[w] = x;
   __syncthreads();
   if (w == 0) {
-    unsigned ws = lane < SCAN_THREADS / 32 ? wsum[lane] : 0u;
+    unsigned ws = wsum[lane];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned y = __shfl_up_sync(0xffffffffu, ws, o);
       if (lane >= o) ws += y;
     }
-    if (lane < SCAN_THREADS / 32) wsum[lane] = ws;
+    wsum[lane] = ws;
   }
   __syncthreads();
-  const unsigned before = (x - run) + (w ? wsum[w - 1] : 0u);
+  const unsigned before = tiles + (x - run) + (w ? wsum[w - 1] : 0u);
 #pragma unroll
   for (int q = 0; q < SCAN_PER; ++q) buf[t * SCAN_PER + q] = before + v[q];
-  if (t == SCAN_THREADS - 1) sums[blockIdx.x] = before + run;
   __syncthreads();
   for (int i = t; i < SCAN_TILE; i += SCAN_THREADS)
     if (base + i < m) a[base + i] = buf[i];
-}
-
-// phase 3: add the scanned tile totals
-__global__ void k_scan_add(unsigned* __restrict__ a, long long m, const unsigned* __restrict__ sums) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < m) a[i] += sums[i / SCAN_TILE];
 }
 
 // Stable scatter: items are ranked in index order within the tile (round by round, warp by warp).
@@ -385,101 +411,27 @@ __device__ __forceinline__ bool near_f(const float4 a, const float4 b, float L, 
   return dx * dx + dy * dy + dz * dz < r * r;
 }
 
-// Block per (cell column (cx, cy), part), nc >= 3; thread per droplet of the column (the part's
-// share of them).  Its partners are searched among the cell itself (partners after it in the
-// sorted order) and the 13 forward neighbours, visited in a fixed order r = 0..13:
+// The count pass (nc >= 3), thread per sorted droplet.  Its partners are searched among the cell
+// itself (droplets after it in the sorted order) and the 13 forward neighbours, visited in a fixed
+// order r = 0..13:
 //   r = 0: the cell itself; r = 1: (0, 0, +1); r = 2..13: columns q = 1..4 (offsets (0,+1),
 //   (+1,-1), (+1,0), (+1,+1)) at dz = -1, 0, +1,
 // and in sorted order inside each target cell, so every unordered pair is tested exactly once.
-// The five columns' cell starts, their periodic shifts and (when they fit in cap_smem rows) their
-// FP32 positions are staged in shared memory; the home cell comes from the sorted key and the
-// neighbour cells by compare-and-wrap, so the visit needs no integer division.  The periodic
-// image of a neighbour cell is fixed (a colliding pair is closer than one cell, nc >= 3): the
-// home position is shifted once per target cell; a wrong image only lengthens the distance (the
-// FP64 rule decides).  Each droplet stores its partner count and its first KEEP partners (sorted
-// indices) in scr; k_emit_pairs writes the pairs from the scanned counts, searching again only
-// for droplets with more than KEEP partners.
-constexpr int COL_THREADS = 256;
+// The cells z-1, z, z+1 of a column are one contiguous sorted range, or at the z faces two (the
+// wrapped cell apart), so that a droplet walks five ranges, rarely ten, whose ends are loaded
+// together.  The periodic image of a neighbour cell is fixed (a colliding pair is closer than one
+// cell, nc >= 3): the home position is shifted once per range; a wrong image only lengthens the
+// distance (the FP64 rule decides).
+// The lanes of a warp are neighbours in the sorted order, so their ranges overlap and the
+// candidates come from L1; staging a column's droplets in shared memory, a block per column, left
+// the blocks waiting at their barriers (1e6 droplets in 82^3 cells: 117 us, 82 now; 4.4e5 droplets
+// in 16 boxes of one per cell: 67 us, mostly block set-up, 29 now).  The FP32 pre-test's hits are queued per thread in shared
+// memory and put to the FP64 rule together after the walk, instead of one lane at a time.
+// Each droplet stores its partner count and its first KEEP partners (sorted indices) in scr;
+// k_emit_pairs writes the pairs from the scanned counts, searching again only for droplets with
+// more than KEEP partners.
+constexpr int VISIT_THREADS = 128, VISIT_BLOCKS = 8;
 constexpr int KEEP = 16;  // partners recorded per droplet (more: searched again by k_emit_pairs)
-constexpr int kColSmemRows = 12288;  // 192 KB of staged FP32 rows per block at most
-
-__device__ __forceinline__ void col_offset(int q, int& ox, int& oy) {
-  ox = q < 2 ? 0 : 1;
-  oy = q == 0 ? 0 : (q == 1 ? 1 : q - 3);
-}
-
-// The visit of one droplet (sorted index i, t-th of its column); STAGED: positions from colbuf.
-// Returns whether the droplet is wide (2 r > cw: its partners beyond the neighbour cells are
-// counted by the block afterwards).
-template <bool STAGED>
-__device__ __forceinline__ bool col_visit(int i, int t, const double4* __restrict__ sp, const float4* __restrict__ spf,
-                                          const float4* colbuf, const int* cst, const int* dl, const float* shx,
-                                          const float* shy, int cz, int nc, double L, double cw, float Lf,
-                                          float margin, unsigned* __restrict__ cnt, int* __restrict__ scr) {
-  const float4 mf = STAGED ? colbuf[t] : spf[i];
-  const float mar = margin + 1e-6f * mf.w;
-  unsigned c = 0;
-  // away from the z faces the three cells z-1, z, z+1 of a column are one contiguous sorted range
-  // with no periodic shift along z: 5 ranges (the own column from i + 1 through cell z + 1, then
-  // the four forward columns), visited in exactly the order of the 14 cells
-  const bool interior = cz >= 1 && cz <= nc - 2;
-  const int nseg = interior ? 5 : 14;
-#pragma unroll 1
-  for (int r = 0; r < nseg; ++r) {
-    int q, g0, g1;
-    float sz;
-    if (interior) {
-      q = r;
-      sz = 0.f;
-      g0 = r == 0 ? i + 1 : cst[q * (nc + 1) + cz - 1];
-      g1 = cst[q * (nc + 1) + cz + 2];
-    } else {
-      q = r < 2 ? 0 : 1 + (r - 2) / 3;
-      const int dz = r < 2 ? r : (r - 2) % 3 - 1;
-      const int zr = cz + dz;
-      const int zz = zr < 0 ? zr + nc : (zr >= nc ? zr - nc : zr);
-      sz = zr >= nc ? -Lf : (zr < 0 ? Lf : 0.f);
-      g0 = r == 0 ? i + 1 : cst[q * (nc + 1) + zz];
-      g1 = cst[q * (nc + 1) + zz + 1];
-    }
-    const float ax = mf.x + shx[q], ay = mf.y + shy[q], az = mf.z + sz;
-    const int d = dl[q];
-    // two candidates at a time on packed FP32 pairs (each half rounds as the scalar operation);
-    // b - a instead of a - b: the squares are the same
-    const float2 nax = make_float2(-ax, -ax), nay = make_float2(-ay, -ay), naz = make_float2(-az, -az);
-    const float2 mw = make_float2(mf.w, mf.w), mr = make_float2(mar, mar);
-    int g = g0;
-    for (; g + 1 < g1; g += 2) {
-      const float4 b0 = STAGED ? colbuf[g - d] : spf[g];
-      const float4 b1 = STAGED ? colbuf[g + 1 - d] : spf[g + 1];
-      const float2 dx = __fadd2_rn(make_float2(b0.x, b1.x), nax), dy = __fadd2_rn(make_float2(b0.y, b1.y), nay),
-                   dz = __fadd2_rn(make_float2(b0.z, b1.z), naz);
-      const float2 rr = __fadd2_rn(__fadd2_rn(mw, make_float2(b0.w, b1.w)), mr);
-      const float2 d2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-      const float2 r2 = __fmul2_rn(rr, rr);
-      if (d2.x < r2.x && overlap_near(sp[i], sp[g], L, cw)) {
-        if (c < KEEP) scr[(long long)KEEP * i + c] = g;
-        ++c;
-      }
-      if (d2.y < r2.y && overlap_near(sp[i], sp[g + 1], L, cw)) {
-        if (c < KEEP) scr[(long long)KEEP * i + c] = g + 1;
-        ++c;
-      }
-    }
-    if (g < g1) {
-      const float4 b = STAGED ? colbuf[g - d] : spf[g];
-      const float dxf = ax - b.x, dyf = ay - b.y, dzf = az - b.z;
-      const float rr = mf.w + b.w + mar;
-      if (dxf * dxf + dyf * dyf + dzf * dzf < rr * rr && overlap_near(sp[i], sp[g], L, cw)) {
-        if (c < KEEP) scr[(long long)KEEP * i + c] = g;
-        ++c;
-      }
-    }
-  }
-  cnt[i] = c;
-  // FP32 radius first (rounding is monotone: r > cw / 2 implies float(r) >= float(cw / 2))
-  return mf.w >= (float)(0.5 * cw) && sp[i].w > 0.5 * cw;
-}
 
 // ---- wide droplets ------------------------------------------------------------------------------
 // A pair with ri + rj > cw (cw the cell width) has at least one droplet with 2 r > cw, a wide
@@ -488,10 +440,16 @@ __device__ __forceinline__ bool col_visit(int i, int t, const double4* __restric
 // cw) + 1 cells of its own along each axis (all nc when 2 R + 1 >= nc), since its partner is closer
 // than rs + rt <= 2 rs.  The owner's pairs follow the pairs of its neighbour-cell search in its
 // run of the output.  Work items of a wide droplet: the 14 cells of the neighbour search (emit
-// only), then the cells of the wide search in (x, y, z) order; the block that meets a wide droplet
-// (the column visit for the count, the emit pass for the pairs) takes its items in contiguous
-// runs, one run per thread, counts, scans the counts and writes, so the order is that of a serial
-// visit.
+// only), then the cells of the wide search in (x, y, z) order; the warp that meets a wide droplet
+// in the count pass, and the block of the emit pass, shares out its items.
+
+// droplet ids (i, j), i < j, at place o of the pair list
+__device__ __forceinline__ void put_pair(int* __restrict__ pairs, long long o, long long cap, unsigned a, unsigned b) {
+  if (o < cap) {
+    pairs[2 * o] = (int)(a < b ? a : b);
+    pairs[2 * o + 1] = (int)(a < b ? b : a);
+  }
+}
 
 struct WideCell {
   long long kb;  // the box's first cell
@@ -515,8 +473,8 @@ __device__ __forceinline__ WideCell wide_cell(unsigned key, int nc, double r, do
 template <bool WRITE>
 __device__ unsigned wide_item(int it, bool with_near, int s, const WideCell& w, const double4& me, const float4& mf,
                               const double4* __restrict__ sp, const float4* __restrict__ spf, const int* __restrict__ cs,
-                              int nc, double L, double cw, float Lf, float hf, float mar, int* __restrict__ pairs,
-                              long long o, long long cap) {
+                              int nc, double L, double cw, float Lf, float hf, float mar,
+                              const unsigned* __restrict__ sval, int* __restrict__ pairs, long long o, long long cap) {
   unsigned c = 0;
   if (with_near && it < 14) {  // the neighbour search of k_emit_pairs, segment r = it
     const int r = it;
@@ -530,7 +488,7 @@ __device__ unsigned wide_item(int it, bool with_near, int s, const WideCell& w, 
     for (int g = r == 0 ? s + 1 : cs[k]; g < g1; ++g) {
       if (!near_f(mf, spf[g], Lf, hf, mar)) continue;
       if (!overlap_near(me, sp[g], L, cw)) continue;
-      if (WRITE && o + c < cap) { pairs[2 * (o + c)] = s; pairs[2 * (o + c) + 1] = g; }
+      if (WRITE) put_pair(pairs, o + c, cap, sval[s], sval[g]);
       ++c;
     }
     return c;
@@ -548,233 +506,222 @@ __device__ unsigned wide_item(int it, bool with_near, int s, const WideCell& w, 
     if (!(__dadd_rn(me.w, b.w) > cw)) continue;  // reported by the neighbour search
     if (b.w > 0.5 * cw && (b.w > me.w || (b.w == me.w && g < s))) continue;  // g owns the pair
     if (!overlap(me, b, L)) continue;
-    if (WRITE && o + c < cap) { pairs[2 * (o + c)] = s; pairs[2 * (o + c) + 1] = g; }
+    if (WRITE) put_pair(pairs, o + c, cap, sval[s], sval[g]);
     ++c;
   }
   return c;
 }
 
-// Block-wide exclusive scan of one count per thread (NTH threads, all of them calling); returns
-// the prefix, *total the sum.
-template <int NTH>
-__device__ __forceinline__ unsigned block_excl_scan(unsigned v, unsigned* wsum, unsigned* total) {
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+// Exclusive scan of one count per lane; *total the sum.
+__device__ __forceinline__ unsigned warp_excl_scan(unsigned v, unsigned* total) {
+  const int lane = threadIdx.x & 31;
   unsigned x = v;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const unsigned y = __shfl_up_sync(0xffffffffu, x, d);
     if (lane >= d) x += y;
   }
-  if (lane == 31) wsum[wp] = x;
-  __syncthreads();
-  unsigned before = 0, all = 0;
-#pragma unroll
-  for (int q = 0; q < NTH / 32; ++q) {
-    before += q < wp ? wsum[q] : 0u;
-    all += wsum[q];
-  }
-  __syncthreads();
-  *total = all;
-  return before + x - v;
+  *total = __shfl_sync(0xffffffffu, x, 31);
+  return x - v;
 }
 
-// The block's wide droplets (sorted indices in list[0..nw)), one after another: the partners of
-// the wide search are added to each droplet's count and its record is marked (scr = -1), so that
-// the emit pass writes its pairs by wide_emit_block.
-template <int NTH>
-__device__ void wide_count_block(const unsigned* list, int nw, const double4* __restrict__ sp,
-                                 const float4* __restrict__ spf, const unsigned* __restrict__ skey,
-                                 const int* __restrict__ cs, int nc, double L, double cw, unsigned* __restrict__ cnt,
-                                 int* __restrict__ scr, unsigned* wsum) {
+// The partners of wide droplet s beyond the neighbour cells, counted by the warp.
+__device__ unsigned wide_count(int s, const double4* __restrict__ sp, const float4* __restrict__ spf,
+                               const unsigned* __restrict__ skey, const int* __restrict__ cs, int nc, double L,
+                               double cw) {
   const float Lf = (float)L, hf = 0.5f * Lf, margin = (float)(1e-6 * L);
-  for (int e = 0; e < nw; ++e) {
-    const int s = (int)list[e];
-    const double4 me = sp[s];
-    const float4 mf = spf[s];
-    const WideCell w = wide_cell(skey[s], nc, me.w, cw);
-    const int items = w.ax * w.ax * w.ax;
-    const int per = (items + NTH - 1) / NTH;
-    unsigned c = 0;
-    for (int it = threadIdx.x * per; it < items && it < (int)(threadIdx.x + 1) * per; ++it)
-      c += wide_item<false>(it, false, s, w, me, mf, sp, spf, cs, nc, L, cw, Lf, hf, margin + 1e-6f * mf.w, nullptr,
-                            0, 0);
-    unsigned total;
-    block_excl_scan<NTH>(c, wsum, &total);
-    if (threadIdx.x == 0) {
-      cnt[s] += total;
-      scr[(long long)KEEP * s] = -1;
-    }
-  }
+  const double4 me = sp[s];
+  const float4 mf = spf[s];
+  const WideCell w = wide_cell(skey[s], nc, me.w, cw);
+  const int items = w.ax * w.ax * w.ax;
+  unsigned c = 0, total;
+  for (int it = threadIdx.x & 31; it < items; it += 32)
+    c += wide_item<false>(it, false, s, w, me, mf, sp, spf, cs, nc, L, cw, Lf, hf, margin + 1e-6f * mf.w, nullptr,
+                          nullptr, 0, 0);
+  warp_excl_scan(c, &total);
+  return total;
 }
 
-// All pairs of the block's wide droplets (neighbour search, then wide search) at off[s]...
-template <int NTH>
-__device__ void wide_emit_block(const unsigned* list, int nw, const double4* __restrict__ sp,
-                                const float4* __restrict__ spf, const unsigned* __restrict__ skey,
-                                const int* __restrict__ cs, int nc, double L, double cw,
-                                const unsigned* __restrict__ off, int* __restrict__ pairs, long long cap,
-                                unsigned* wsum) {
-  const float Lf = (float)L, hf = 0.5f * Lf, margin = (float)(1e-6 * L);
-  for (int e = 0; e < nw; ++e) {
-    const int s = (int)list[e];
-    const double4 me = sp[s];
-    const float4 mf = spf[s];
+__global__ void __launch_bounds__(VISIT_THREADS, VISIT_BLOCKS)
+k_visit(const double4* __restrict__ sp, const float4* __restrict__ spf, const unsigned* __restrict__ skey,
+        const int* __restrict__ cs, int nc, double L, double cw, int n, unsigned* __restrict__ cnt,
+        int* __restrict__ scr) {
+  __shared__ int queue[KEEP][VISIT_THREADS];
+  const int tid = threadIdx.x;
+  unsigned c = 0;     // partners confirmed (the first KEEP in scr)
+  bool wide = false;  // partners beyond the neighbour cells, counted by the warp below
+  const long long ii = (long long)blockIdx.x * VISIT_THREADS + tid;
+  if (ii == 0) cnt[n] = 0u;
+  if (ii < n) {
+    const int i = (int)ii;
+    const float Lf = (float)L, margin = (float)(1e-6 * L);
+    // home cell: column (box, cx, cy) and height
+    const unsigned unc = (unsigned)nc;
+    const unsigned key = skey[i], col = key / unc, cz = key - col * unc, cy = col % unc, cx = (col / unc) % unc;
+    const float4 mf = spf[i];
     const float mar = margin + 1e-6f * mf.w;
-    const WideCell w = wide_cell(skey[s], nc, me.w, cw);
-    const int items = 14 + w.ax * w.ax * w.ax;
-    const int per = (items + NTH - 1) / NTH;
-    const int i0 = threadIdx.x * per, i1 = i0 + per < items ? i0 + per : items;
-    unsigned c = 0;
-    for (int it = i0; it < i1; ++it)
-      c += wide_item<false>(it, true, s, w, me, mf, sp, spf, cs, nc, L, cw, Lf, hf, mar, nullptr, 0, 0);
-    unsigned total;
-    long long o = (long long)off[s] + block_excl_scan<NTH>(c, wsum, &total);
-    for (int it = i0; it < i1; ++it)
-      o += wide_item<true>(it, true, s, w, me, mf, sp, spf, cs, nc, L, cw, Lf, hf, mar, pairs, o, cap);
-  }
-}
-
-template <int CT>  // threads per block: fewer for sparse columns (a multi-box collider's small boxes)
-__global__ void __launch_bounds__(CT)
-k_col_pairs(const double4* __restrict__ sp, const float4* __restrict__ spf, const unsigned* __restrict__ skey,
-            const int* __restrict__ cs, int nc, int parts, double L, double cw, int cap_smem,
-            unsigned* __restrict__ cnt, int* __restrict__ scr) {
-  extern __shared__ __align__(16) unsigned char cp_smem[];
-  float4* colbuf = reinterpret_cast<float4*>(cp_smem);
-  int* cst = reinterpret_cast<int*>(cp_smem + sizeof(float4) * (size_t)cap_smem);  // 5 x (nc + 1) cell starts
-  __shared__ long long kq[5];
-  __shared__ int lo[5], so[6], dl[5];
-  __shared__ float shx[5], shy[5];
-  __shared__ unsigned wlist[CT], nwide, wsum[CT / 32];
-  if (threadIdx.x == 0) nwide = 0u;
-  const long long colg = blockIdx.x / parts;  // (box, cx, cy) of a multi-box collider
-  const int part = (int)(blockIdx.x % parts);
-  const long long ncol = (long long)nc * nc;
-  const long long bbase = (colg / ncol) * ncol * nc;  // the box's first cell
-  const long long col = colg % ncol;
-  const int cx = (int)(col / nc), cy = (int)(col % nc);
-  const float Lf = (float)L, margin = (float)(1e-6 * L);
-  if (threadIdx.x < 5) {
-    int ox, oy;
-    col_offset(threadIdx.x, ox, oy);
-    kq[threadIdx.x] = bbase + ((long long)((cx + ox) % nc) * nc + (cy + oy + nc) % nc) * nc;
-    shx[threadIdx.x] = (cx + ox >= nc) ? -Lf : 0.f;
-    shy[threadIdx.x] = (cy + oy >= nc) ? -Lf : ((cy + oy < 0) ? Lf : 0.f);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < 5 * (nc + 1); e += CT) {
-    const int q = e / (nc + 1), z = e - q * (nc + 1);
-    cst[e] = cs[kq[q] + z];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
+    // first cells of the five columns, and the shifts of the home position that bring it next to
+    // their periodic images
+    const bool xw = cx + 1 == unc, yu = cy + 1 == unc, yd = cy == 0;
+    const unsigned colx = col + unc - (xw ? unc * unc : 0u);
+    const unsigned up = 1u - (yu ? unc : 0u), down = (yd ? unc : 0u) - 1u;  // to the next and the previous cy
+    const unsigned cq[5] = {col, col + up, colx + down, colx, colx + up};
+    const float sx = xw ? -Lf : 0.f, su = yu ? -Lf : 0.f, sd = yd ? Lf : 0.f;
+    // range A: cells from max(z - 1, 0) to min(z + 1, nc - 1) of each column (own column: after the
+    // droplet itself); range B: the wrapped cell at a z face
+    const bool bottom = cz == 0, top = cz + 1 == unc;
+    int a0[5], a1[5];
+#pragma unroll
     for (int q = 0; q < 5; ++q) {
-      lo[q] = cst[q * (nc + 1)];
-      so[q] = acc;
-      acc += cst[q * (nc + 1) + nc] - lo[q];
+      const int* c = cs + (size_t)cq[q] * unc;
+      a0[q] = q == 0 ? i + 1 : c[bottom ? 0 : cz - 1];
+      a1[q] = c[top ? unc : cz + 2];
     }
-    so[5] = acc;
-  }
-  __syncthreads();
-  const bool staged = so[5] <= cap_smem;  // block-uniform
-  if (threadIdx.x < 5) dl[threadIdx.x] = staged ? lo[threadIdx.x] - so[threadIdx.x] : 0;
-  if (staged) {
+    unsigned pend = 0;  // candidates queued
+    auto flush = [&]() {
+      for (unsigned e = 0; e < pend; ++e) {
+        const int g = queue[e][tid];
+        if (overlap_near(sp[i], sp[g], L, cw)) {
+          if (c < KEEP) scr[(long long)KEEP * i + c] = g;
+          ++c;
+        }
+      }
+      pend = 0;
+    };
+    auto hit = [&](int g) {
+      if (pend == KEEP) flush();
+      queue[pend++][tid] = g;
+    };
+    auto walk = [&](int g, int g1, float ax, float ay, float az) {
+      // two candidates at a time on packed FP32 pairs (each half rounds as the scalar operation);
+      // b - a instead of a - b: the squares are the same
+      const float2 nax = make_float2(-ax, -ax), nay = make_float2(-ay, -ay), naz = make_float2(-az, -az);
+      const float2 mw = make_float2(mf.w, mf.w), mr = make_float2(mar, mar);
+      for (; g < g1; g += 2) {
+        const bool two = g + 1 < g1;
+        const float4 b0 = spf[g], b1 = spf[two ? g + 1 : g];
+        const float2 dx = __fadd2_rn(make_float2(b0.x, b1.x), nax), dy = __fadd2_rn(make_float2(b0.y, b1.y), nay),
+                     dz = __fadd2_rn(make_float2(b0.z, b1.z), naz);
+        const float2 rr = __fadd2_rn(__fadd2_rn(mw, make_float2(b0.w, b1.w)), mr);
+        const float2 d2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+        const float2 r2 = __fmul2_rn(rr, rr);
+        const bool h0 = d2.x < r2.x, h1 = two && d2.y < r2.y;
+        if (h0 || h1) {
+          if (h0) hit(g);
+          if (h1) hit(g + 1);
+        }
+      }
+    };
+#pragma unroll
     for (int q = 0; q < 5; ++q) {
-      const int n_q = so[q + 1] - so[q];
-      for (int t = threadIdx.x; t < n_q; t += CT) colbuf[so[q] + t] = spf[lo[q] + t];
+      const float ax = mf.x + (q < 2 ? 0.f : sx);
+      const float ay = mf.y + (q == 0 || q == 3 ? 0.f : (q == 2 ? sd : su));
+      // the wrapped cell below comes before range A (dz = -1), the one above after it (dz = +1); the
+      // own column's search starts at the droplet itself and has no cell below
+      if (q > 0 && bottom) {
+        const int* w = cs + (size_t)cq[q] * unc + unc - 1;
+        walk(w[0], w[1], ax, ay, mf.z + Lf);
+      }
+      walk(a0[q], a1[q], ax, ay, mf.z);
+      if (top) {
+        const int* w = cs + (size_t)cq[q] * unc;
+        walk(w[0], w[1], ax, ay, mf.z - Lf);
+      }
     }
+    flush();
+    cnt[i] = c;
+    // FP32 radius first: rounding is monotone, r > cw / 2 implies float(r) >= float(cw / 2)
+    wide = mf.w >= (float)(0.5 * cw) && sp[i].w > 0.5 * cw;
   }
-  __syncthreads();
-  const int len0 = so[1] - so[0];
-  // rounds of CT droplets; after each, the block counts the round's wide droplets' partners
-  // beyond the neighbour cells together
-  for (int t0 = part * CT; t0 < len0; t0 += parts * CT) {
-    const int t = t0 + threadIdx.x;
-    if (t < len0) {
-      const int i = lo[0] + t;
-      const int cz = (int)(skey[i] - (unsigned)kq[0]);
-      const bool wide =
-          staged ? col_visit<true>(i, t, sp, spf, colbuf, cst, dl, shx, shy, cz, nc, L, cw, Lf, margin, cnt, scr)
-                 : col_visit<false>(i, t, sp, spf, colbuf, cst, dl, shx, shy, cz, nc, L, cw, Lf, margin, cnt, scr);
-      if (wide) wlist[atomicAdd(&nwide, 1u)] = (unsigned)i;
+  for (unsigned m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    const unsigned more = wide_count(__shfl_sync(0xffffffffu, (int)ii, src), sp, spf, skey, cs, nc, L, cw);
+    if ((tid & 31) == src) {  // marked, so that the emit pass writes its pairs by wide_emit
+      cnt[ii] = c + more;
+      scr[(long long)KEEP * ii] = -1;
     }
-    __syncthreads();
-    const int nw = (int)nwide;  // block-uniform
-    if (nw) wide_count_block<CT>(wlist, nw, sp, spf, skey, cs, nc, L, cw, cnt, scr, wsum);
-    __syncthreads();
-    if (threadIdx.x == 0) nwide = 0u;
-    __syncthreads();
   }
 }
 
 // Pairs of sorted droplet i at off[i]..: copied from scr when it has at most KEEP partners,
-// otherwise found again from global memory in the same visiting order.  The block takes rounds
-// of EMIT_THREADS droplets; the round's wide droplets (scr marked by the column visit) are
-// emitted by the whole block after the round (wide_emit_block).
+// otherwise found again from global memory in the same visiting order; wide droplets (scr marked by
+// the count pass) by the whole block afterwards, since the pass is short and a wide droplet's
+// search a chain of dependent loads.
 constexpr int EMIT_THREADS = 256;
+
+// All pairs of wide droplet s (neighbour search, then wide search) at place o..., by the block: each
+// thread takes a contiguous run of the work items, so the order is that of a serial visit.
+__device__ void wide_emit(int s, long long o, const double4* __restrict__ sp, const float4* __restrict__ spf,
+                          const unsigned* __restrict__ skey, const int* __restrict__ cs, int nc, double L, double cw,
+                          const unsigned* __restrict__ sval, int* __restrict__ pairs, long long cap, unsigned* wsum) {
+  const float Lf = (float)L, hf = 0.5f * Lf, margin = (float)(1e-6 * L);
+  const double4 me = sp[s];
+  const float4 mf = spf[s];
+  const float mar = margin + 1e-6f * mf.w;
+  const WideCell w = wide_cell(skey[s], nc, me.w, cw);
+  const int items = 14 + w.ax * w.ax * w.ax;
+  const int per = (items + EMIT_THREADS - 1) / EMIT_THREADS;
+  const int i0 = (int)threadIdx.x * per, i1 = i0 + per < items ? i0 + per : items;
+  unsigned c = 0, total;
+  for (int it = i0; it < i1; ++it)
+    c += wide_item<false>(it, true, s, w, me, mf, sp, spf, cs, nc, L, cw, Lf, hf, mar, nullptr, nullptr, 0, 0);
+  const unsigned before = warp_excl_scan(c, &total);
+  if ((threadIdx.x & 31) == 31) wsum[threadIdx.x >> 5] = total;
+  __syncthreads();
+  o += before;
+  for (int q = 0; q < (int)(threadIdx.x >> 5); ++q) o += wsum[q];
+  __syncthreads();
+  for (int it = i0; it < i1; ++it)
+    o += wide_item<true>(it, true, s, w, me, mf, sp, spf, cs, nc, L, cw, Lf, hf, mar, sval, pairs, o, cap);
+}
 
 __global__ void __launch_bounds__(EMIT_THREADS)
 k_emit_pairs(const double4* __restrict__ sp, const float4* __restrict__ spf, const unsigned* __restrict__ skey,
-             const int* __restrict__ cs, int nc, double L, double cw, long long n, const unsigned* __restrict__ off,
-             const int* __restrict__ scr, int* __restrict__ pairs, long long cap) {
+             const unsigned* __restrict__ sval, const int* __restrict__ cs, int nc, double L, double cw, int n,
+             const unsigned* __restrict__ off, const int* __restrict__ scr, int* __restrict__ pairs, long long cap) {
   __shared__ unsigned wlist[EMIT_THREADS], nwide, wsum[EMIT_THREADS / 32];
   if (threadIdx.x == 0) nwide = 0u;
   __syncthreads();
   const float Lf = (float)L, hf = 0.5f * Lf, margin = (float)(1e-6 * L);
-  for (long long base = (long long)blockIdx.x * EMIT_THREADS; base < n; base += (long long)gridDim.x * EMIT_THREADS) {
-    const long long ii = base + threadIdx.x;
-    const int i = (int)ii;
-    const unsigned cnt = ii < n ? off[i + 1] - off[i] : 0u;
-    if (cnt > 0 && scr[(long long)KEEP * i] < 0) {
-      wlist[atomicAdd(&nwide, 1u)] = (unsigned)i;
-    } else if (cnt > 0 && cnt <= (unsigned)KEEP) {
-      const long long o0 = off[i];
-      for (unsigned k = 0; k < cnt; ++k)
-        if (o0 + k < cap) { pairs[2 * (o0 + k)] = i; pairs[2 * (o0 + k) + 1] = scr[(long long)KEEP * i + k]; }
-    } else if (cnt > 0) {
-      const unsigned key = skey[i];
-      const unsigned nc3 = (unsigned)nc * nc * nc;
-      const long long kb = (long long)(key / nc3) * nc3;  // the box's first cell
-      const int cz = (int)(key % (unsigned)nc), cy = (int)((key / nc) % nc), cx = (int)((key / ((unsigned)nc * nc)) % nc);
-      const float4 mf = spf[i];
-      const float mar = margin + 1e-6f * mf.w;
-      const double4 me = sp[i];
-      long long o = off[i];
-      for (int r = 0; r < 14; ++r) {
-        int q, dz;
-        if (r < 2) { q = 0; dz = r; }
-        else { q = 1 + (r - 2) / 3; dz = (r - 2) % 3 - 1; }
-        const int z = (cz + dz + nc) % nc;
-        const int ox = q < 2 ? 0 : 1;
-        const int oy = q == 0 ? 0 : (q == 1 ? 1 : q - 3);
-        const long long k = kb + ((long long)((cx + ox) % nc) * nc + (cy + oy + nc) % nc) * nc + z;
-        const int g1 = cs[k + 1];
-        for (int g = r == 0 ? i + 1 : cs[k]; g < g1; ++g) {
-          if (!near_f(mf, spf[g], Lf, hf, mar)) continue;
-          if (!overlap_near(me, sp[g], L, cw)) continue;
-          if (o < cap) { pairs[2 * o] = i; pairs[2 * o + 1] = g; }
-          ++o;
-        }
+  const long long ii = (long long)blockIdx.x * EMIT_THREADS + threadIdx.x;
+  const int i = (int)ii;
+  const unsigned o0 = ii < n ? off[i] : 0u, cnt = ii < n ? off[i + 1] - o0 : 0u;
+  const bool wide = cnt > 0 && scr[(long long)KEEP * i] < 0;
+  if (wide) wlist[atomicAdd(&nwide, 1u)] = (unsigned)i;
+  if (!wide && cnt > 0 && cnt <= (unsigned)KEEP) {
+    const unsigned id = sval[i];
+    for (unsigned k = 0; k < cnt; ++k) put_pair(pairs, o0 + (long long)k, cap, id, sval[scr[(long long)KEEP * i + k]]);
+  } else if (!wide && cnt > 0) {
+    const unsigned key = skey[i];
+    const unsigned nc3 = (unsigned)nc * nc * nc;
+    const long long kb = (long long)(key / nc3) * nc3;  // the box's first cell
+    const int cz = (int)(key % (unsigned)nc), cy = (int)((key / nc) % nc), cx = (int)((key / ((unsigned)nc * nc)) % nc);
+    const float4 mf = spf[i];
+    const float mar = margin + 1e-6f * mf.w;
+    const double4 me = sp[i];
+    long long o = o0;
+    for (int r = 0; r < 14; ++r) {
+      int q, dz;
+      if (r < 2) { q = 0; dz = r; }
+      else { q = 1 + (r - 2) / 3; dz = (r - 2) % 3 - 1; }
+      const int z = (cz + dz + nc) % nc;
+      const int ox = q < 2 ? 0 : 1;
+      const int oy = q == 0 ? 0 : (q == 1 ? 1 : q - 3);
+      const long long k = kb + ((long long)((cx + ox) % nc) * nc + (cy + oy + nc) % nc) * nc + z;
+      const int g1 = cs[k + 1];
+      for (int g = r == 0 ? i + 1 : cs[k]; g < g1; ++g) {
+        if (!near_f(mf, spf[g], Lf, hf, mar)) continue;
+        if (!overlap_near(me, sp[g], L, cw)) continue;
+        put_pair(pairs, o, cap, sval[i], sval[g]);
+        ++o;
       }
     }
-    __syncthreads();
-    const int nw = (int)nwide;  // block-uniform
-    if (nw) wide_emit_block<EMIT_THREADS>(wlist, nw, sp, spf, skey, cs, nc, L, cw, off, pairs, cap, wsum);
-    __syncthreads();
-    if (threadIdx.x == 0) nwide = 0u;
-    __syncthreads();
   }
-}
-
-// sorted-array indices -> droplet indices, (i, j) with i < j
-__global__ void k_map_pairs(const unsigned* __restrict__ total, long long cap, const unsigned* __restrict__ sval,
-                            int* __restrict__ pairs) {
-  const long long m = (long long)*total < cap ? (long long)*total : cap;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x) {
-    const int a = (int)sval[pairs[2 * e]], b = (int)sval[pairs[2 * e + 1]];
-    pairs[2 * e] = a < b ? a : b;
-    pairs[2 * e + 1] = a < b ? b : a;
+  __syncthreads();
+  const int nw = (int)nwide;  // block-uniform
+  for (int e = 0; e < nw; ++e) {
+    const int s = (int)wlist[e];
+    wide_emit(s, (long long)off[s], sp, spf, skey, cs, nc, L, cw, sval, pairs, cap, wsum);
   }
 }
 
@@ -842,12 +789,8 @@ namespace {
 int scan_u32(ld_collider* c, unsigned* a, long long m, cudaStream_t s) {
   const long long tiles = (m + SCAN_TILE - 1) / SCAN_TILE;
   if (tiles > SCAN_TILE) return ld_fail(LD_ERR_UNSUPPORTED, "scan of %lld elements", m);
+  if (tiles > 1) k_scan_totals<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(a, m, c->sums);
   k_scan_tiles<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(a, m, c->sums);
-  if (tiles > 1) {
-    unsigned* sums2 = c->sums + tiles;
-    k_scan_tiles<<<1, SCAN_THREADS, 0, s>>>(c->sums, tiles, sums2);
-    k_scan_add<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(a, m, c->sums);
-  }
   LD_LAUNCH_CHECK();
   return LD_OK;
 }
@@ -981,52 +924,16 @@ int ld_collide_boxes(ld_collider* c, const double* pos, const double* radius, co
     }
   }
   ProfScope ps(c->trace, KID_COLL_PAIRS, s);
-  LD_CUDA_CHECK(cudaMemsetAsync(c->cnt + n, 0, 4, s));
   if (nc >= 3) {
-    // block per cell column (and part); pairs come out as sorted-array indices and are mapped
-    // back to droplet indices by k_map_pairs
-    const long long ncol = (long long)nc * nc * c->nbox;  // cell columns of every box
-    const long long per_col = (n + ncol - 1) / ncol;
-    const long long parts = per_col > 512 ? (per_col + 511) / 512 : 1;
-    const size_t starts_bytes = sizeof(int) * 5 * (size_t)(nc + 1);
-    if (ncol * parts > 0x7fffffffLL || starts_bytes > 64 * 1024)
-      return ld_fail(LD_ERR_UNSUPPORTED, "ld_collide: too many cells per side (%d)", nc);
-    long long want = 5 * per_col + (5 * per_col) / 4 + 256;  // typical staged rows, with headroom
-    const long long room = (long long)((220 * 1024 - starts_bytes) / sizeof(float4));
-    if (want > kColSmemRows) want = kColSmemRows;
-    if (want > room) want = room;
-    const int cap_smem = (int)want;
-    const size_t smem = sizeof(float4) * (size_t)cap_smem + starts_bytes;
-    // blocks of 64, 128 or 192 threads where columns hold few droplets (the boxes of an ensemble;
-    // about 150 per column at 1e6 droplets in 82^3 cells), 256 otherwise: threads without a
-    // droplet would only wait at the block's barriers
-    if (per_col <= 64) {
-      LD_CUDA_CHECK(cudaFuncSetAttribute(k_col_pairs<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_col_pairs<64><<<(unsigned)(ncol * parts), 64, smem, s>>>(c->sp, c->spf, c->key, c->start, nc, (int)parts, L,
-                                                                 cw, cap_smem, c->cnt, c->scr);
-    } else if (per_col <= 128) {
-      LD_CUDA_CHECK(cudaFuncSetAttribute(k_col_pairs<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_col_pairs<128><<<(unsigned)(ncol * parts), 128, smem, s>>>(c->sp, c->spf, c->key, c->start, nc, (int)parts, L,
-                                                                   cw, cap_smem, c->cnt, c->scr);
-    } else if (per_col <= 192) {
-      LD_CUDA_CHECK(cudaFuncSetAttribute(k_col_pairs<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      // shared memory, not registers, would otherwise hold it to 5 blocks per SM
-      LD_CUDA_CHECK(cudaFuncSetAttribute(k_col_pairs<192>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-      k_col_pairs<192><<<(unsigned)(ncol * parts), 192, smem, s>>>(c->sp, c->spf, c->key, c->start, nc, (int)parts, L,
-                                                                   cw, cap_smem, c->cnt, c->scr);
-    } else {
-      LD_CUDA_CHECK(cudaFuncSetAttribute(k_col_pairs<COL_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
-      k_col_pairs<COL_THREADS><<<(unsigned)(ncol * parts), COL_THREADS, smem, s>>>(
-          c->sp, c->spf, c->key, c->start, nc, (int)parts, L, cw, cap_smem, c->cnt, c->scr);
-    }
+    k_visit<<<(unsigned)((n + VISIT_THREADS - 1) / VISIT_THREADS), VISIT_THREADS, 0, s>>>(
+        c->sp, c->spf, c->key, c->start, nc, L, cw, (int)n, c->cnt, c->scr);
     if (int rc = scan_u32(c, c->cnt, n + 1, s)) return rc;
-    k_emit_pairs<<<gridn(n, EMIT_THREADS), EMIT_THREADS, 0, s>>>(c->sp, c->spf, c->key, c->start, nc, L, cw, n,
-                                                                 c->cnt, c->scr, pairs, cap);
-    k_map_pairs<<<gridn(cap, 256), 256, 0, s>>>(c->cnt + n, cap, c->val, pairs);
+    k_emit_pairs<<<(unsigned)((n + EMIT_THREADS - 1) / EMIT_THREADS), EMIT_THREADS, 0, s>>>(
+        c->sp, c->spf, c->key, c->val, c->start, nc, L, cw, (int)n, c->cnt, c->scr, pairs, cap);
     if (box_counts)
       k_box_counts_sorted<<<(c->nbox + 255) / 256, 256, 0, s>>>(c->cnt, c->start, nc3, c->nbox, box_counts);
   } else {
+    LD_CUDA_CHECK(cudaMemsetAsync(c->cnt + n, 0, 4, s));
     const int* end = c->start + 1;  // end of cell k = start of cell k + 1
     k_pairs<0, true><<<gridn(n, 128), 128, 0, s>>>(c->sp, c->val, c->key, c->start, end, n, nc, L, c->cnt,
                                                    nullptr, nullptr, 0);
