@@ -12,17 +12,15 @@
 // chained after an inverse one with no exchange in between.
 //
 // Twiddles for stages >= 1 come from a table tw[p] = exp(-2 pi i p / N), p < N, computed on the
-// host in FP64 (and rounded once to the element type).  The radix-R butterflies use the exact
-// constants cos(2 pi m / 16), sin(2 pi m / 16).
+// host in FP64 (and rounded once to the element type), read directly, or through a copy in the
+// thread's own order: registers (TwRegs) or shared memory (TwLane).  The radix-R butterflies use
+// the exact constants cos(2 pi m / 16), sin(2 pi m / 16).
 //
-// Lengths that are not powers of two (N = 2^a 3^b 5^c, E a power of two dividing N) take the
-// mixed-radix Stockham pipeline below (fft_run_mr): stage 0 is radix E in registers as above;
-// the remaining factor N / E is split into radix 8/4/2 stages, then radix 5, then radix 3 stages,
-// each stage's N / R butterflies dealt round-robin to the NT threads (a thread does up to
-// ceil(N / R / NT) of them; the rest idle), every stage reading and writing the exchange buffer;
-// the last stage writes natural order and each thread reads back its own positions, so the
-// register contract is the same.
+// The other lengths N = 12 R2 R3 (360 = 12 5 6, 384 = 12 8 4, 192 = 12 4 4, 96 = 12 4 2) take
+// twelve elements per thread and three in-place stages with two exchanges (fft_run_12).
 #pragma once
+#include <type_traits>
+
 #include "ld_common.cuh"
 
 namespace ld {
@@ -138,32 +136,24 @@ struct SyncWarp {
 };
 
 // Shared-memory slot of element p of a row buffer (sstride = 1) when PAD is set.
-//   8-byte elements (complex float): p ^ mask(p / 16), a permutation inside each 128-byte line
-//   (16 elements) keyed by the line index: the contiguous reads of every stage stay on whole
-//   lines (two wavefronts per warp) and the stride-E writes of stage 0 and the grouped writes of
-//   the middle stages spread over the banks.  A warp's 8-byte accesses are served half a warp at
-//   a time, so the sixteen elements of each half must fall in distinct bank pairs: mask = the
-//   line index (p >> 4) & 15 achieves it for every access but the stage-1 writes of N = 256,
-//   E = 8 (two-way conflicts), which the mixed mask below removes for that size.
+//   8-byte elements (complex float), rows of 16 threads or more: p ^ (p / 16 mod 16), a permutation
+//   inside each 128-byte line (16 elements) keyed by the line index: the contiguous reads of every
+//   stage stay on whole lines and the stride-E writes of stage 0 and the grouped writes of the
+//   middle stages spread over the banks, so that the sixteen elements of each half-warp fall in
+//   distinct bank pairs.  Rows of 2 to 8 threads (E = 8): one spare slot per 8 elements (p + p / 8),
+//   conflict-free for two rows of 8 threads side by side that start 8 slots apart (mod 16).
 //   16-byte elements (complex double): one spare slot per E elements (p + p / E), which spreads
 //   the stride-E writes; a warp needs four wavefronts for these anyway.
 // Without PAD: p (column buffers, sstride = columns per block).
 template <typename T, int N, int E, bool PAD> __device__ __forceinline__ int sidx(int p) {
   if constexpr (!PAD) {
     return p;
-  } else if constexpr (sizeof(T) == 4 && N == 256 && E == 8) {
-    // 256-point rows of 32 threads (the fused z pass at 256^3): the line index b mixed with b << 1
-    // (checked over that row's accesses of 8-byte elements — stage-0 and stage-1 writes, stage-1
-    // and stage-2 reads, the forward pair's split — by enumerating each half-warp's bank pairs)
-    const int b = (p >> 4) & 15;
-    return p ^ ((b ^ (b << 1)) & 15);
-  } else if constexpr (sizeof(T) == 4) {
+  } else if constexpr (sizeof(T) == 4 && N / E >= 16) {
     return p ^ ((p >> 4) & 15);
   } else {
     return p + (p >> ilog2(E));
   }
 }
-
 // In-place length-3 and length-5 DFTs (forward sign exp(-2 pi i jk / R); INV conjugates).  The
 // constants are cos and sin of 2 pi / 3, 2 pi / 5 and 4 pi / 5.
 template <typename T, bool INV> __device__ __forceinline__ void dft3(cplx<T>* x) {
@@ -199,88 +189,176 @@ template <typename T, bool INV> __device__ __forceinline__ void dft5(cplx<T>* x)
   x[3] = csub(t2, iu2);
 }
 
-// Any radix of the mixed-radix pipeline: 2, 4, 8, 16 (bit-reversed passes), 3 or 5.
+// In-place length-3 P DFT, P = 2 or 4, by the prime-factor map: no twiddles, input n = 3 a + P b mod
+// 3 P and output k = K3 a' + KP b' mod 3 P, with K3 = 1 mod P and 0 mod 3, KP = 1 mod 3 and 0 mod P.
+template <typename T, int P, bool INV> __device__ __forceinline__ void dft3p(cplx<T>* x) {
+  constexpr int R = 3 * P, K3 = P == 4 ? 9 : 3, KP = 4;
+  cplx<T> y[R];
+#pragma unroll
+  for (int a = 0; a < P; ++a) {
+    cplx<T> t[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) t[b] = x[(3 * a + P * b) % R];
+    dft3<T, INV>(t);
+#pragma unroll
+    for (int b = 0; b < 3; ++b) y[P * b + a] = t[b];
+  }
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    dft<T, P, INV>(y + P * b);
+#pragma unroll
+    for (int a = 0; a < P; ++a) x[(K3 * a + KP * b) % R] = y[P * b + a];
+  }
+}
+
+// Any radix of the mixed-radix pipeline: 2, 4, 8, 16 (bit-reversed passes), 3, 5, 6 or 12.
 template <typename T, int R, bool INV> __device__ __forceinline__ void dft_any(cplx<T>* x) {
   if constexpr (R == 3) dft3<T, INV>(x);
   else if constexpr (R == 5) dft5<T, INV>(x);
+  else if constexpr (R == 6) dft3p<T, 2, INV>(x);
+  else if constexpr (R == 12) dft3p<T, 4, INV>(x);
   else dft<T, R, INV>(x);
 }
 
 __host__ __device__ constexpr bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
-// radix of the next stage for a remaining factor m: 8, 4, 2 first, then 5, then 3
-__host__ __device__ constexpr int mr_pick(int m) {
-  return m % 8 == 0 ? 8 : (m % 4 == 0 ? 4 : (m % 2 == 0 ? 2 : (m % 5 == 0 ? 5 : (m % 3 == 0 ? 3 : m))));
-}
-// remaining factor before stage s (s >= 1) of a length-N pipeline whose stage 0 is radix E
-__host__ __device__ constexpr int mr_rest(int N, int E, int s) {
-  return s <= 1 ? N / E : mr_rest(N, E, s - 1) / mr_pick(mr_rest(N, E, s - 1));
-}
-__host__ __device__ constexpr int mr_nstages(int m) { return m <= 1 ? 0 : 1 + mr_nstages(m / mr_pick(m)); }
-// m is a product of 2s, 3s and 5s
-__host__ __device__ constexpr bool mr_ok(int m) {
-  return m == 1 || (m > 1 && ((m % 2 == 0 && mr_ok(m / 2)) || (m % 3 == 0 && mr_ok(m / 3)) || (m % 5 == 0 && mr_ok(m / 5))));
-}
 
-template <int N, int E> struct MrShape {
-  static_assert(is_pow2(E) && E >= 2 && E <= 16 && N % E == 0, "stage 0: a power-of-two radix dividing N");
-  static_assert(mr_ok(N / E), "N / E must factor into 2, 3 and 5");
-  static constexpr int NT = N / E;
-  static constexpr int S = 1 + mr_nstages(N / E);
-  static __host__ __device__ constexpr int radix(int s) { return s == 0 ? E : mr_pick(mr_rest(N, E, s)); }
-  static __host__ __device__ constexpr int ns(int s) { return N / mr_rest(N, E, s); }  // product of earlier radices
+// Lengths N = 12 R2 R3: with k1 = 0..11, a = 0..R3-1, b and c = 0..R2-1, d = 0..R3-1,
+//   stage 1  thread j = a + R3 b: radix 12 over x[j + NT m] -> k1, twiddle W_N^(j k1);
+//   stage 2  for every (k1, a): radix R2 over b -> c, twiddle W_NT^(a c), in place;
+//   stage 3  for every (k1, c): radix R3 over a -> d, output k = k1 + 12 c + 12 R2 d.
+// The exchange buffer holds (k1, a + R3 c) at slot S(k1) + a + R3 c.  Stage 3's butterflies t = k1 +
+// 12 c = j + NT q leave their outputs at j + NT (q + (12 / R3) d), the thread's own positions (the
+// register contract), and stage 2 works in place, so two barriers separate the three stages.
+// S(k1) = PITCH k1 + (k1 >> SH) makes the accesses of all stages free of bank conflicts (360 in
+// FP64: 10% more than conflict-free), found by enumerating the bank groups of each half-warp
+// (FP32) or quarter-warp (FP64) over pitches and skews; ROW is the row buffer's length, rows of a
+// warp side by side included in the enumeration.
+template <typename T, int N> struct Len12 {
+  static_assert(N == 360 || N == 384 || N == 192 || N == 96, "length 12 R2 R3");
+  static constexpr int NT = N / 12;
+  static constexpr int R2 = N == 360 ? 5 : (N == 384 ? 8 : 4), R3 = N == 360 ? 6 : (N == 96 ? 2 : 4);
+  static constexpr bool F32 = sizeof(T) == 4;
+  static constexpr int PITCH = NT + (N == 96 ? 2 : (N == 360 ? (F32 ? 8 : 0) : 4));
+  static constexpr int SH = F32 ? (N == 360 ? 3 : 2) : (N == 360 ? 2 : (N == 96 ? 3 : 1));
+  static constexpr int ROW = 11 * PITCH + (11 >> SH) + NT;
 };
 
-// Stage s >= 1 of the mixed-radix pipeline.
-template <typename T, int N, int E, bool INV, bool PAD, int s, class Sync>
-__device__ __forceinline__ void fft_stage_mr(cplx<T>* a, cplx<T>* sbuf, int sstride, int j,
-                                             const cplx<T>* __restrict__ tw, Sync sync) {
-  using Sh = MrShape<N, E>;
-  constexpr int NT = Sh::NT;
-  constexpr int R = Sh::radix(s);
-  constexpr int Ns = Sh::ns(s);
-  constexpr int NB = N / R;                  // butterflies of this stage
-  constexpr int Q = (NB + NT - 1) / NT;      // butterflies per thread
-  constexpr bool FULL = Q * NT == NB;
-  constexpr bool LAST = s == Sh::S - 1;
-  cplx<T> x[Q * R];
+// The twiddles a thread uses, numbered: powers of two stage by stage (s >= 1), then by butterfly q,
+// then by r = 1..R-1; N = 12 R2 R3: W_N^(j k1) for k1 = 1..11, then W_NT^(a c) for c = 1..R2-1 (a = j
+// mod R3 for every butterfly of thread j).
+template <int N, int E, bool P2> struct Pipe_;
+template <int N, int E> struct Pipe_<N, E, true> {
+  using Sh = FftShape<N, E>;
+  static constexpr int NT = N / E, S = Sh::S;
+  static __host__ __device__ constexpr int per(int s) { return E / Sh::radix(s); }
+  static __host__ __device__ constexpr int first(int s) {
+    return s <= 1 ? 0 : first(s - 1) + per(s - 1) * (Sh::radix(s - 1) - 1);
+  }
+  static constexpr int COUNT = first(S);
+  // f(number, table index) over thread j's twiddles
+  template <class F, int s = 1> static __device__ __forceinline__ void each(int j, F f) {
+    if constexpr (s < S) {
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const int b = j + NT * q;
-    if (FULL || b < NB) {
+      for (int q = 0; q < per(s); ++q)
 #pragma unroll
-      for (int r = 0; r < R; ++r) x[q * R + r] = sbuf[sidx<T, N, E, PAD>(b + r * NB) * sstride];
+        for (int r = 1; r < Sh::radix(s); ++r)
+          f(first(s) + q * (Sh::radix(s) - 1) + r - 1, r * ((j + NT * q) % Sh::ns(s)) * (N / (Sh::ns(s) * Sh::radix(s))));
+      each<F, s + 1>(j, f);
+    }
+  }
+};
+template <int N, int E> struct Pipe_<N, E, false> {
+  using L = Len12<float, N>;
+  static constexpr int COUNT = 11 + L::R2 - 1;
+  template <class F> static __device__ __forceinline__ void each(int j, F f) {
+#pragma unroll
+    for (int k = 1; k < 12; ++k) f(k - 1, j * k);
+#pragma unroll
+    for (int c = 1; c < L::R2; ++c) f(10 + c, 12 * (j % L::R3) * c);
+  }
+};
+template <int N, int E> using Pipe = Pipe_<N, E, is_pow2(N)>;
+
+// A thread's twiddles in registers (loaded once, used by every transform of a persistent kernel).
+template <typename T, int N, int E> struct TwRegs {
+  cplx<T> w[Pipe<N, E>::COUNT];
+  __device__ __forceinline__ void load(const cplx<T>* __restrict__ tab, int j) {
+    Pipe<N, E>::each(j, [&](int n, int p) { w[n] = tab[p]; });
+  }
+};
+// The same in shared memory, twiddle n of thread j at p[n * NT] (p already at j): contiguous over
+// the threads of a row, where the table's own order would touch a line per thread.
+template <typename T, int N, int E> struct TwLane {
+  const cplx<T>* p;
+  static constexpr int ELEMS = Pipe<N, E>::COUNT * (N / E);
+  static __device__ __forceinline__ void fill(cplx<T>* dst, const cplx<T>* __restrict__ tab, int tid, int nthreads) {
+    for (int j = tid; j < N / E; j += nthreads)
+      Pipe<N, E>::each(j, [&](int n, int q) { dst[n * (N / E) + j] = tab[q]; });
+  }
+};
+// Twiddle number n (table index p) from any of the sources, conjugated for the inverse.
+template <typename T, int N, int E, bool INV> __device__ __forceinline__ cplx<T> tw_at(const cplx<T>* tw, int n, int p) {
+  (void)n;
+  return twid<T, INV>(tw, p);
+}
+template <typename T, int N, int E, bool INV>
+__device__ __forceinline__ cplx<T> tw_at(const TwRegs<T, N, E>& tw, int n, int p) {
+  (void)p;
+  cplx<T> w = tw.w[n];
+  if (INV) w.y = -w.y;
+  return w;
+}
+template <typename T, int N, int E, bool INV>
+__device__ __forceinline__ cplx<T> tw_at(const TwLane<T, N, E>& tw, int n, int p) {
+  (void)p;
+  cplx<T> w = tw.p[n * (N / E)];
+  if (INV) w.y = -w.y;
+  return w;
+}
+
+// The three stages of a length N = 12 R2 R3 (see Len12); without PAD the slots are a + R3 c + NT k1.
+template <typename T, int N, bool INV, bool PAD, class Tw, class Sync>
+__device__ __forceinline__ void fft_run_12(cplx<T>* a, cplx<T>* sbuf, int sstride, int j, const Tw& tw, Sync sync) {
+  using L = Len12<T, N>;
+  constexpr int NT = L::NT, R2 = L::R2, R3 = L::R3, Q2 = (12 + R2 - 1) / R2, Q3 = 12 / R3;
+  auto S = [](int k1) { return PAD ? L::PITCH * k1 + (k1 >> L::SH) : NT * k1; };
+  dft3p<T, 4, INV>(a);
+#pragma unroll
+  for (int k = 0; k < 12; ++k)
+    sbuf[(S(k) + j) * sstride] = k ? cmul(a[k], tw_at<T, N, 12, INV>(tw, k - 1, j * k)) : a[k];
+  sync();
+#pragma unroll
+  for (int q = 0; q < Q2; ++q) {
+    const int u = j + NT * q;
+    if (Q2 * R2 == 12 || u < 12 * R3) {
+      const int i = u % R3;
+      cplx<T>* p = sbuf + (S(u / R3) + i) * sstride;
+      cplx<T> x[R2];
+#pragma unroll
+      for (int b = 0; b < R2; ++b) x[b] = p[b * R3 * sstride];
+      dft_any<T, R2, INV>(x);
+#pragma unroll
+      for (int c = 0; c < R2; ++c)
+        p[c * R3 * sstride] = c ? cmul(x[c], tw_at<T, N, 12, INV>(tw, 10 + c, 12 * i * c)) : x[c];
     }
   }
   sync();
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const int b = j + NT * q;
-    if (FULL || b < NB) {
-      const int k = b % Ns;
+  for (int q = 0; q < Q3; ++q) {
+    const int t = j + NT * q;
+    const cplx<T>* p = sbuf + (S(t % 12) + R3 * (t / 12)) * sstride;
+    cplx<T> x[R3];
 #pragma unroll
-      for (int r = 1; r < R; ++r) x[q * R + r] = cmul(x[q * R + r], twid<T, INV>(tw, r * k * (N / (Ns * R))));
-      dft_any<T, R, INV>(x + q * R);
-      // Stockham output position (b / Ns) Ns R + k + r Ns; in the last stage b < Ns, which is
-      // natural order b + r NB
-      const int base = LAST ? b : (b / Ns) * Ns * R + k;
-      constexpr int step = LAST ? NB : Ns;
+    for (int i = 0; i < R3; ++i) x[i] = p[i * sstride];
+    dft_any<T, R3, INV>(x);
 #pragma unroll
-      for (int r = 0; r < R; ++r) sbuf[sidx<T, N, E, PAD>(base + r * step) * sstride] = x[q * R + r];
-    }
-  }
-  sync();
-  if constexpr (!LAST) {
-    fft_stage_mr<T, N, E, INV, PAD, s + 1>(a, sbuf, sstride, j, tw, sync);
-  } else {
-#pragma unroll
-    for (int m = 0; m < E; ++m) a[m] = sbuf[sidx<T, N, E, PAD>(j + NT * m) * sstride];
+    for (int d = 0; d < R3; ++d) a[q + Q3 * d] = x[d];
   }
 }
 
 // Stage s >= 1 of the Stockham pipeline (compile-time recursion over the stages).
-template <typename T, int N, int E, bool INV, bool PAD, int s, class Sync>
-__device__ __forceinline__ void fft_stage(cplx<T>* a, cplx<T>* sbuf, int sstride, int j,
-                                          const cplx<T>* __restrict__ tw, Sync sync) {
+template <typename T, int N, int E, bool INV, bool PAD, int s, class Tw, class Sync>
+__device__ __forceinline__ void fft_stage(cplx<T>* a, cplx<T>* sbuf, int sstride, int j, const Tw& tw, Sync sync) {
   using Sh = FftShape<N, E>;
   constexpr int NT = Sh::NT;
   constexpr int S = Sh::S;
@@ -300,7 +378,8 @@ __device__ __forceinline__ void fft_stage(cplx<T>* a, cplx<T>* sbuf, int sstride
     const int b = j + NT * q;
     const int k = b % Ns;
 #pragma unroll
-    for (int r = 1; r < R; ++r) x[q * R + r] = cmul(x[q * R + r], twid<T, INV>(tw, r * k * (N / (Ns * R))));
+    for (int r = 1; r < R; ++r) x[q * R + r] = cmul(x[q * R + r], tw_at<T, N, E, INV>(tw, Pipe<N, E>::first(s) + q * (R - 1) + r - 1,
+                                                                            r * k * (N / (Ns * R))));
     dft<T, R, INV>(x + q * R);
     if constexpr (s < S - 1) {
       const int base = (b / Ns) * Ns * R + k;
@@ -319,12 +398,11 @@ __device__ __forceinline__ void fft_stage(cplx<T>* a, cplx<T>* sbuf, int sstride
 
 // Full FFT of length N; see the register contract at the top of this file.  The caller must
 // not touch sbuf between fft_run() calls without a barrier: the last stage reads it.
-template <typename T, int N, int E, bool INV, bool PAD, class Sync>
-__device__ __forceinline__ void fft_run(cplx<T>* a, cplx<T>* sbuf, int sstride, int j,
-                                        const cplx<T>* __restrict__ tw, Sync sync) {
-  dft<T, E, INV>(a);  // stage 0: radix E, Ns = 1, no twiddles
+template <typename T, int N, int E, bool INV, bool PAD, class Tw, class Sync>
+__device__ __forceinline__ void fft_run(cplx<T>* a, cplx<T>* sbuf, int sstride, int j, const Tw& tw, Sync sync) {
   if constexpr (is_pow2(N)) {
     using Sh = FftShape<N, E>;
+    dft<T, E, INV>(a);  // stage 0: radix E, Ns = 1, no twiddles
     if constexpr (Sh::S > 1) {
 #pragma unroll
       for (int r = 0; r < E; ++r) sbuf[sidx<T, N, E, PAD>(j * E + r) * sstride] = a[r];
@@ -332,11 +410,8 @@ __device__ __forceinline__ void fft_run(cplx<T>* a, cplx<T>* sbuf, int sstride, 
       fft_stage<T, N, E, INV, PAD, 1>(a, sbuf, sstride, j, tw, sync);
     }
   } else {
-    static_assert(MrShape<N, E>::S > 1, "mixed-radix lengths have later stages");
-#pragma unroll
-    for (int r = 0; r < E; ++r) sbuf[sidx<T, N, E, PAD>(j * E + r) * sstride] = a[r];
-    sync();
-    fft_stage_mr<T, N, E, INV, PAD, 1>(a, sbuf, sstride, j, tw, sync);
+    static_assert(E == 12, "lengths 12 R2 R3 take twelve elements per thread");
+    fft_run_12<T, N, INV, PAD>(a, sbuf, sstride, j, tw, sync);
   }
 }
 

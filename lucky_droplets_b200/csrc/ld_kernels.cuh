@@ -39,32 +39,46 @@ template <typename T> __device__ __forceinline__ vec4<T> mk4(T a, T b, T c, T d)
   vec4<T> v; v.x = a; v.y = b; v.z = c; v.w = d; return v;
 }
 
-// Launch shapes by N.  Powers of two: as tuned.  Mixed-radix N = 2^a 3^b 5^c (a >= 3): eight
-// elements per thread (stage 0 radix 8) in both kinds of pass; column passes with a CTA of 8
-// columns (64-byte FP32 / 128-byte FP64 row segments; N/8 x 8 threads leave the FP64 update pass,
-// which holds three transformed columns, enough registers); z passes with as many row units per
-// CTA as fit 256 threads (a power of two, so that N^2 rows split evenly); their rows span warps,
-// so they exchange with block-wide barriers.  (Measured at 360^3 in FP64 against four elements
-// per thread, two or three CTAs per SM and a block-pipelined variant with bulk-copy prefetch:
-// this shape was the fastest of them.)
+// Launch shapes of the column passes by N.  Powers of two: as tuned.  N = 12 R2 R3: twelve elements
+// per thread, a CTA of 8 columns (64-byte FP32 / 128-byte FP64 row segments).
 template <int N> struct Cfg {
   static constexpr bool P2 = is_pow2(N);
   // column passes: E elements per thread, TB columns per CTA
-  static constexpr int EC = P2 ? ((N == 32 || N == 64) ? 8 : 16) : 8;
+  static constexpr int EC = P2 ? ((N == 32 || N == 64) ? 8 : 16) : 12;
   static constexpr int NTC = N / EC;
   static constexpr int TB = P2 ? (N == 16 ? 64 : (N == 32 ? 32 : 16)) : 8;
   static constexpr int COL_THREADS = TB * NTC;
-  // z passes: E elements per thread, NTZ threads per row
-  static constexpr int EZ = P2 ? (N >= 512 ? 16 : 8) : 8;
-  static constexpr int NTZ = N / EZ;
-  static constexpr int ZROWS = P2 ? 256 / NTZ : (256 / NTZ >= 16 ? 16 : (256 / NTZ >= 8 ? 8 : (256 / NTZ >= 4 ? 4 : (256 / NTZ >= 2 ? 2 : 1))));
-  static constexpr int ZTHREADS = ZROWS * NTZ;  // row units per CTA x threads per row
-  static constexpr int LOGEZ = ilog2(EZ);
   // the dealiased cube of a plan of size N (ld_plan_create: kc = N / 3, rows padded to 8)
   static constexpr int KC = N / 3;
   static constexpr int MY = 2 * KC + 1;
   static constexpr int MZP = (KC + 1 + 7) / 8 * 8;
-  static constexpr int ZBUF = N + N / EZ;       // padded row buffer (bank-conflict free)
+};
+
+// Shapes of the z passes (contiguous rows).  A row lies inside one warp (N / E <= 32), so
+// that its exchanges are warp-level, and a warp takes R rows side by side.  What bounds these
+// passes is the shared-memory data path, so E is chosen for few exchanges per transform:
+//   powers of two: E = 16 for FP32 rows of 128 and 256 (256 = 16 x 16: one exchange where E = 8
+//   needs two), E = 8 for rows of 16..64 and for FP64 (the fused pass keeps three transforms of E
+//   elements in registers), E = 16 for 512;
+//   N = 12 R2 R3: E = 12, rows of 8, 16, 30 or 32 lanes and two exchanges inside a warp, where E = 8
+//   spread a row of 360 over 45 threads (block-wide barriers) and four exchanges.
+template <typename T, int N> struct ZCfg {
+  static constexpr bool P2 = is_pow2(N);
+  static constexpr int E = !P2 ? 12 : (N >= 512 || (sizeof(T) == 4 && (N == 128 || N == 256)) ? 16 : 8);
+  static constexpr int NT = N / E;                         // threads per row
+  static constexpr int R = 32 / NT;                        // rows per warp (360: lanes 30, 31 repeat lanes 0, 1)
+  static constexpr int ZBUF = P2 ? N + N / E : Len12<T, P2 ? 96 : N>::ROW;  // padded row buffer
+  // One-shot kernels (C2R, R2C of one pair of rows per unit): a short FP32 row of 128 has too few
+  // threads with E = 16 (reference-layout transforms of 128^3: 82 us against 76)
+  static constexpr int E1 = sizeof(T) == 4 && N == 128 ? 8 : E;
+  static constexpr int THREADS1 = 256;
+  static constexpr int UNITS1 = THREADS1 / 32 * (32 / (N / E1));  // row units per block
+  static constexpr int ZBUF1 = P2 ? N + N / E1 : ZBUF;
+  // twiddles of the fused pass: in registers where three transforms and they fit (FP64 powers of
+  // two; FP32 512, whose eight warps per SM run at 255 registers), else in shared memory in lane
+  // order (FP32 256 at 168 registers and three CTAs per SM: 430 us a right-hand side, 451 with the
+  // twiddles in registers, 440 with them and two CTAs)
+  static constexpr bool TWREG = sizeof(T) == 4 ? N == 512 : Pipe<N, E>::COUNT <= 13;
 };
 
 // ------------------------------------------------------------------------------------------
@@ -558,26 +572,24 @@ k_xfwd_update(UpdArgs<T> A, int ncols, const cplx<T>* __restrict__ tw) {
 }
 
 // ------------------------------------------------------------------------------------------
-// z passes (contiguous axis): one thread group of NTZ threads per row unit, inside one warp
+// z passes (contiguous axis): NT threads per row unit, inside one warp
 // ------------------------------------------------------------------------------------------
-// Exchange barrier of the z passes: warp-level when the row units of a warp lie inside it (a row
-// per warp at N >= 256; at N = 64 and 128 four and two rows per warp, every lane of the warp
-// taking part in every exchange), block-wide for rows that span warps (mixed-radix lengths) and
-// for N <= 32 (where the warp-level form gave wrong results in the fused pass).
-template <int N>
-using ZSync = typename std::conditional<(Cfg<N>::NTZ == 32 || (N >= 64 && Cfg<N>::P2 && 32 % Cfg<N>::NTZ == 0)),
-                                        SyncWarp, SyncBlock>::type;
-// Row-buffer slot of element i: the same map as the FFT exchange of the row (sidx with PAD).
-template <typename T, int N> struct ZIdx {
-  static __device__ __forceinline__ int p(int i) { return sidx<T, N, Cfg<N>::EZ, true>(i); }
-};
+// Row unit of this lane within its warp, and the lane within the row.
+template <int N, int E> __device__ __forceinline__ void z_lane(int& unit, int& j) {
+  constexpr int NT = N / E, R = 32 / NT;
+  const int lane = threadIdx.x & 31;
+  unit = lane / NT;
+  j = lane - unit * NT;
+  if (R * NT < 32 && unit >= R) unit = 0;  // the lanes left over repeat the first ones of unit 0
+  __builtin_assume(j >= 0 && j < NT);
+}
 
 // Hermitian-extended load of Y[k] = A[k] + i B[k] (k = j + NT m), A/B spectral rows with Kin
 // valid coefficients; imaginary parts of k = 0 and k = N/2 are dropped (pocketfft c2r).
-template <typename T, int N>
+template <typename T, int N, int E>
 __device__ __forceinline__ void zload_pair(cplx<T>* a, const cplx<T>* A, const cplx<T>* B, int Kin,
                                            int j, T s) {
-  constexpr int NT = Cfg<N>::NTZ, E = Cfg<N>::EZ;
+  constexpr int NT = N / E;
 #pragma unroll
   for (int m = 0; m < E; ++m) {
     const int k = j + NT * m;
@@ -607,13 +619,13 @@ __device__ __forceinline__ void zload_pair(cplx<T>* a, const cplx<T>* A, const c
   }
 }
 
-// After a forward FFT of (a + i b): split Y into A[k], B[k] for k < Kout (zero for k >= Kval).
-// Rows of one warp exchange the mirrored coefficients by shuffles; narrower rows write Y to the
-// row buffer first (the caller must have synced the buffer).
-template <typename T, int N, class Sync>
-__device__ __forceinline__ void zstore_pair(const cplx<T>* a, cplx<T>* sb, cplx<T>* A, cplx<T>* B,
-                                            int Kout, int Kval, int j, bool ok, Sync sync) {
-  constexpr int NT = Cfg<N>::NTZ, E = Cfg<N>::EZ;
+// After a forward FFT of (a + i b): split Y into A[k], B[k] for k < Kout (zero for k >= Kval; B null:
+// A alone).  The mirrored coefficients come by shuffles: Y[N - k] (Y[0] for k = 0) is register
+// E - 1 - m of lane NT - j (j > 0), or register (E - m) % E of lane 0 (j = 0).
+template <typename T, int N, int E>
+__device__ __forceinline__ void zstore_pair(const cplx<T>* a, cplx<T>* A, cplx<T>* B, int Kout, int Kval, int j,
+                                            bool ok) {
+  constexpr int NT = N / E;
   if (B == nullptr) {
 #pragma unroll
     for (int m = 0; m < E; ++m) {
@@ -622,40 +634,19 @@ __device__ __forceinline__ void zstore_pair(const cplx<T>* a, cplx<T>* sb, cplx<
     }
     return;
   }
-  if constexpr (NT == 32) {
-    // a row per warp: Y[N - k] (Y[0] for k = 0) is register E - 1 - m of lane 32 - j (j > 0), or
-    // register (E - m) % E of lane 0 (j = 0), fetched by shuffles instead of through the buffer
-#pragma unroll
-    for (int m = 0; m < E; ++m) {
-      const int k = j + NT * m;
-      cplx<T> z;
-      z.x = __shfl_sync(0xffffffffu, a[E - 1 - m].x, (NT - j) & (NT - 1));
-      z.y = __shfl_sync(0xffffffffu, a[E - 1 - m].y, (NT - j) & (NT - 1));
-      if (j == 0) z = a[(E - m) % E];
-      if (ok && k < Kout) {
-        cplx<T> ra = czero<cplx<T>>(), rb = czero<cplx<T>>();
-        if (k < Kval) {
-          const cplx<T> y = a[m];
-          ra = cmk(T(0.5) * (y.x + z.x), T(0.5) * (y.y - z.y));
-          rb = cmk(T(0.5) * (y.y + z.y), T(-0.5) * (y.x - z.x));
-        }
-        A[k] = ra;
-        B[k] = rb;
-      }
-    }
-    return;
-  }
-#pragma unroll
-  for (int m = 0; m < E; ++m) sb[ZIdx<T, N>::p(j + NT * m)] = a[m];
-  sync();
+  const int lane = threadIdx.x & 31, src = j == 0 ? lane : lane - j + NT - j;
 #pragma unroll
   for (int m = 0; m < E; ++m) {
     const int k = j + NT * m;
+    if (NT * m >= Kout) continue;  // uniform
+    cplx<T> z;
+    z.x = __shfl_sync(0xffffffffu, a[E - 1 - m].x, src);
+    z.y = __shfl_sync(0xffffffffu, a[E - 1 - m].y, src);
+    if (j == 0) z = a[(E - m) % E];
     if (ok && k < Kout) {
       cplx<T> ra = czero<cplx<T>>(), rb = czero<cplx<T>>();
       if (k < Kval) {
         const cplx<T> y = a[m];
-        const cplx<T> z = sb[ZIdx<T, N>::p(k == 0 ? 0 : N - k)];
         ra = cmk(T(0.5) * (y.x + z.x), T(0.5) * (y.y - z.y));
         rb = cmk(T(0.5) * (y.y + z.y), T(-0.5) * (y.x - z.x));
       }
@@ -665,29 +656,40 @@ __device__ __forceinline__ void zstore_pair(const cplx<T>* a, cplx<T>* sb, cplx<
   }
 }
 
+// Row unit of this thread in a one-shot z kernel: unit within the block, lane j within the row,
+// and whether this lane's stores are its own (lanes left over repeat others).
+template <typename T, int N> __device__ __forceinline__ void z_unit(int& unit, int& j, bool& own) {
+  constexpr int E = ZCfg<T, N>::E1, NT = N / E, R = 32 / NT;
+  z_lane<N, E>(unit, j);
+  unit += (threadIdx.x >> 5) * R;
+  own = (threadIdx.x & 31) < R * NT;
+}
+
 // Generic C2R: pairs of rows (2p, 2p+1) of nrows rows per field; spectral rows of stride ss
 // (Kin valid), real rows of stride N.  Scale s (1/N^3 for the 3D inverse).
 template <typename T, int N>
-__global__ void __launch_bounds__(Cfg<N>::ZTHREADS)
+__global__ void __launch_bounds__(256)
 k_z_c2r(const cplx<T>* __restrict__ X, T* __restrict__ x, long long nrows, int ss, int Kin, T s,
         long long xfs, long long Xfs, const cplx<T>* __restrict__ tw) {
-  constexpr int E = Cfg<N>::EZ, NT = Cfg<N>::NTZ;
+  using Z = ZCfg<T, N>;
+  constexpr int E = Z::E1, NT = N / E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
-  const int unit = threadIdx.x / NT, j = threadIdx.x % NT;
-  cplx<T>* sb = sbuf + unit * Cfg<N>::ZBUF;
-  const long long pair = (long long)blockIdx.x * Cfg<N>::ZROWS + unit;
+  int unit, j;
+  bool own;
+  z_unit<T, N>(unit, j, own);
+  cplx<T>* sb = sbuf + unit * Z::ZBUF1;
+  const long long pair = (long long)blockIdx.x * Z::UNITS1 + unit;
   const int f = blockIdx.y;
   const bool ok = 2 * pair < nrows;
   const long long r0 = ok ? 2 * pair : 0;
   const cplx<T>* A = X + f * Xfs + r0 * ss;
   const cplx<T>* B = (r0 + 1 < nrows) ? A + ss : nullptr;
   cplx<T> a[E];
-  if (ok) zload_pair<T, N>(a, A, B, Kin, j, s);
+  if (ok) zload_pair<T, N, E>(a, A, B, Kin, j, s);
   else for (int m = 0; m < E; ++m) a[m] = czero<cplx<T>>();
-  // the row buffer is private to this unit (one warp or part of one): warp-level sync suffices
-  fft_run<T, N, E, true, true>(a, sb, 1, j, tw, ZSync<N>());
-  if (!ok) return;
+  fft_run<T, N, E, true, true>(a, sb, 1, j, tw, SyncWarp());
+  if (!ok || !own) return;
   T* xa = x + f * xfs + r0 * N;
 #pragma unroll
   for (int m = 0; m < E; ++m) {
@@ -699,15 +701,18 @@ k_z_c2r(const cplx<T>* __restrict__ X, T* __restrict__ x, long long nrows, int s
 
 // Generic R2C: pairs of real rows -> spectral rows (stride ss), Kout stored (zeros for k >= Kval).
 template <typename T, int N>
-__global__ void __launch_bounds__(Cfg<N>::ZTHREADS)
+__global__ void __launch_bounds__(256)
 k_z_r2c(const T* __restrict__ x, cplx<T>* __restrict__ X, long long nrows, int ss, int Kout,
         int Kval, long long xfs, long long Xfs, const cplx<T>* __restrict__ tw) {
-  constexpr int E = Cfg<N>::EZ, NT = Cfg<N>::NTZ;
+  using Z = ZCfg<T, N>;
+  constexpr int E = Z::E1, NT = N / E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
-  const int unit = threadIdx.x / NT, j = threadIdx.x % NT;
-  cplx<T>* sb = sbuf + unit * Cfg<N>::ZBUF;
-  const long long pair = (long long)blockIdx.x * Cfg<N>::ZROWS + unit;
+  int unit, j;
+  bool own;
+  z_unit<T, N>(unit, j, own);
+  cplx<T>* sb = sbuf + unit * Z::ZBUF1;
+  const long long pair = (long long)blockIdx.x * Z::UNITS1 + unit;
   const int f = blockIdx.y;
   const bool ok = 2 * pair < nrows;
   const long long r0 = ok ? 2 * pair : 0;
@@ -719,53 +724,36 @@ k_z_r2c(const T* __restrict__ x, cplx<T>* __restrict__ X, long long nrows, int s
     const int n = j + NT * m;
     a[m] = ok ? cmk(xa[n], hasb ? xa[N + n] : T(0)) : czero<cplx<T>>();
   }
-  fft_run<T, N, E, false, true>(a, sb, 1, j, tw, ZSync<N>());
-  ZSync<N>()();
+  fft_run<T, N, E, false, true>(a, sb, 1, j, tw, SyncWarp());
   cplx<T>* A = X + f * Xfs + r0 * ss;
-  zstore_pair<T, N>(a, sb, A, hasb ? A + ss : nullptr, Kout, Kval, j, ok, ZSync<N>());
+  zstore_pair<T, N, E>(a, A, hasb ? A + ss : nullptr, Kout, Kval, j, ok && own);
 }
 
-// One row of the fused z pass: C2R of the six y-transformed fields [u, w] (kz < Kin of each row
-// pointer in[f]), optional store of physical u, u x w (F:299-301), R2C of the three products
-// (kz < Mzp stored, zero beyond Kin) into P + f*fs + row*Mzp.
-// HOIST: the three pairs are loaded before the first transform (rows read from global memory:
-// one load phase per row instead of three); the pipelined pass reads staged rows and loads each
-// pair just before its transform.
-template <typename T, int N, bool HOIST = false>
-__device__ __forceinline__ void zcross_row(const cplx<T>* const* in, cplx<T>* sb, cplx<T>* P, long long fs,
-                                           long long row, T* uphys, int ulayout, int Mzp, int Kin, T s, int j,
-                                           const cplx<T>* __restrict__ tw) {
-  constexpr int E = Cfg<N>::EZ, NT = Cfg<N>::NTZ;
-  using Sy = ZSync<N>;
-  cplx<T> p0[E], p1[E], p2[E];
-  zload_pair<T, N>(p0, in[0], in[1], Kin, j, s);  // pair (u_x, u_y)
-  if constexpr (HOIST) {
-    zload_pair<T, N>(p1, in[2], in[3], Kin, j, s);  // pair (u_z, w_x)
-    zload_pair<T, N>(p2, in[4], in[5], Kin, j, s);  // pair (w_y, w_z)
-  }
-  fft_run<T, N, E, true, true>(p0, sb, 1, j, tw, Sy());
-  Sy()();
-  if constexpr (!HOIST) zload_pair<T, N>(p1, in[2], in[3], Kin, j, s);
-  fft_run<T, N, E, true, true>(p1, sb, 1, j, tw, Sy());
-  Sy()();
-  if constexpr (!HOIST) zload_pair<T, N>(p2, in[4], in[5], Kin, j, s);
-  fft_run<T, N, E, true, true>(p2, sb, 1, j, tw, Sy());
-  Sy()();
-  if (uphys && ulayout == 0) {  // planar (3, N, N, N)
-    const long long NN3 = (long long)N * N * N;
+// The products and forward half of one row of the fused z pass, from the three inverse transforms
+// p0 = (u_x, u_y), p1 = (u_z, w_x), p2 = (w_y, w_z): optional store of physical u, u x w
+// (F:299-301), R2C of the three products into A, B, C (kz < Kout stored, zero beyond Kin).
+template <typename T, int N, class Tw>
+__device__ __forceinline__ void zcross_forward(cplx<T>* p0, cplx<T>* p1, const cplx<T>* p2, cplx<T>* sb, cplx<T>* A,
+                                               cplx<T>* B, cplx<T>* C, long long row, T* uphys, int ulayout, int Kout,
+                                               int Kin, int j, bool own, const Tw& tw) {
+  constexpr int E = ZCfg<T, N>::E, NT = ZCfg<T, N>::NT;
+  if (uphys && own) {
+    if (ulayout == 0) {  // planar (3, N, N, N)
+      const long long NN3 = (long long)N * N * N;
 #pragma unroll
-    for (int m = 0; m < E; ++m) {
-      const int n = j + NT * m;
-      uphys[row * N + n] = p0[m].x;
-      uphys[NN3 + row * N + n] = p0[m].y;
-      uphys[2 * NN3 + row * N + n] = p1[m].x;
-    }
-  } else if (uphys) {  // interleaved (N, N, N, 4): (u, v, w, 0) per grid point
-    vec4<T>* u4 = reinterpret_cast<vec4<T>*>(uphys);
+      for (int m = 0; m < E; ++m) {
+        const int n = j + NT * m;
+        uphys[row * N + n] = p0[m].x;
+        uphys[NN3 + row * N + n] = p0[m].y;
+        uphys[2 * NN3 + row * N + n] = p1[m].x;
+      }
+    } else {  // interleaved (N, N, N, 4): (u, v, w, 0) per grid point
+      vec4<T>* u4 = reinterpret_cast<vec4<T>*>(uphys);
 #pragma unroll
-    for (int m = 0; m < E; ++m) {
-      const int n = j + NT * m;
-      u4[row * N + n] = mk4<T>(p0[m].x, p0[m].y, p1[m].x, T(0));
+      for (int m = 0; m < E; ++m) {
+        const int n = j + NT * m;
+        u4[row * N + n] = mk4<T>(p0[m].x, p0[m].y, p1[m].x, T(0));
+      }
     }
   }
   // products: (u x w) = (uy wz - uz wy, uz wx - ux wz, ux wy - uy wx)
@@ -775,112 +763,121 @@ __device__ __forceinline__ void zcross_row(const cplx<T>* const* in, cplx<T>* sb
     p0[m] = cmk(wz * uy - wy * uz, wx * uz - wz * ux);
     p1[m] = cmk(wy * ux - wx * uy, T(0));
   }
-  fft_run<T, N, E, false, true>(p0, sb, 1, j, tw, Sy());
-  Sy()();
-  zstore_pair<T, N>(p0, sb, P + row * Mzp, P + fs + row * Mzp, Mzp, Kin, j, true, Sy());
-  Sy()();
-  fft_run<T, N, E, false, true>(p1, sb, 1, j, tw, Sy());
-  zstore_pair<T, N>(p1, sb, P + 2 * fs + row * Mzp, (cplx<T>*)nullptr, Mzp, Kin, j, true, Sy());
+  fft_run<T, N, E, false, true>(p0, sb, 1, j, tw, SyncWarp());
+  zstore_pair<T, N, E>(p0, A, B, Kout, Kin, j, own);
+  __syncwarp();
+  fft_run<T, N, E, false, true>(p1, sb, 1, j, tw, SyncWarp());
+  __syncwarp();  // C may lie in the exchange buffer
+  zstore_pair<T, N, E>(p1, C, (cplx<T>*)nullptr, Kout, Kin, j, own);
 }
 
-// Fused z pass, one row unit per NTZ threads, rows read straight from global memory.
-// W: (6, N*N, Mzp) in; P: (3, N*N, Mzp) out.
-// 64-point FP32 rows (the ensemble's boxes): three CTAs per SM (80 registers, no spills; 86 and
-// two CTAs per SM without the bound: ensemble step 1.50 -> 1.42 ms)
-template <typename T, int N>
-__global__ void __launch_bounds__(Cfg<N>::ZTHREADS, (sizeof(T) == 4 && N == 64) ? 3 : 1)
-k_z_cross(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __restrict__ uphys, int ulayout, int Mzp,
-          int kc, T s, const cplx<T>* __restrict__ tw, long long NR) {
-  constexpr int NT = Cfg<N>::NTZ;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
-  const int unit = threadIdx.x / NT, j = threadIdx.x % NT;
-  cplx<T>* sb = sbuf + unit * Cfg<N>::ZBUF;
-  const long long row = (long long)blockIdx.x * Cfg<N>::ZROWS + unit;  // grid covers NR (rows per field) exactly
-  (void)Mzp;
-  (void)kc;
-  constexpr int MZ = Cfg<N>::MZP, KIN = Cfg<N>::KC + 1;  // the plan's cube (checked at launch)
-  const long long fs = NR * MZ;
-  const cplx<T>* in[6];
-#pragma unroll
-  for (int f = 0; f < 6; ++f) in[f] = W + f * fs + row * MZ;
-  zcross_row<T, N, true>(in, sb, P, fs, row, uphys, ulayout, MZ, KIN, s, j, tw);
-}
-
-// Pipelined fused z pass for one warp per row (N >= 256): persistent warps walk the rows with a
-// stride; lane 0 of each warp prefetches the next row's six field rows into a double-buffered
-// shared staging area with bulk asynchronous copies (the TMA engine), completed on per-buffer
-// mbarriers, while the warp transforms the current row.  Waits are bounded: a wait for a row
-// gives up after wait_limit polls (the plan's setting); the warp then raises
+// Fused z pass: persistent warps walk groups of R rows with a
+// stride.  The six field rows of the warp's next group are brought into shared memory by bulk
+// asynchronous copies (the TMA engine), one mbarrier per pair of fields, each issued as soon as
+// the current group's pair sits in registers, so that the transforms cover it.  Waits are bounded:
+// a wait gives up after wait_limit polls (the plan's setting); the warp then raises
 // LD_STATUS_WAIT_TIMEOUT, drains its copies in flight (bounded by kWaitLimit) and returns.  With
-// `stall` set (a test of that path) each warp first waits on a third mbarrier that nothing
-// completes, so the wait runs out while the warp's first copy is in flight.
-// Shared memory per warp: 2 x 6 x Mzp staging + ZBUF exchange elements, then 3 mbarriers.
+// `stall` set (a test of that path) each warp first waits on a fourth mbarrier that nothing
+// completes, so the wait runs out while the warp's first copies are in flight.
+// Shared memory: per warp 6 R rows of Mzp and R exchange rows, then the twiddles in lane order
+// (unless they are in registers), then 4 mbarriers per warp.
 constexpr unsigned kWaitLimit = 1u << 24;
 
-// FP32: 8 warps per CTA, two CTAs per SM at N = 256 (at most 128 registers; the 16-element rows
-// of N = 512 need more); FP64: 4 warps per CTA
+template <typename T, int N> struct ZPipe {
+  using Z = ZCfg<T, N>;
+  static constexpr int WARPS = 4;
+  static constexpr int STAGE = 6 * Z::R * Cfg<N>::MZP;  // elements per warp
+  static constexpr int EX = Z::R * Z::ZBUF;
+  static constexpr int TW = Z::TWREG ? 0 : TwLane<T, N, Z::E>::ELEMS;
+  static constexpr size_t SMEM = sizeof(cplx<T>) * ((size_t)WARPS * (STAGE + EX) + TW) + 32 * WARPS;
+  // CTAs per SM asked of the compiler: 3 E complex values and what a transform needs besides
+  static constexpr int MINB = sizeof(T) == 4 && N != 512 ? 3 : 2;
+};
+
 template <typename T, int N>
-__global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : 128, (sizeof(T) == 4 && N <= 256) ? 2 : 1)
-k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __restrict__ uphys, int ulayout, int Mzp,
-               int kc, T s, const cplx<T>* __restrict__ tw, unsigned* status, unsigned wait_limit,
-               int stall, long long NR) {
-  static_assert(Cfg<N>::NTZ == 32, "one warp per row");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  (void)Mzp;
-  (void)kc;
+__global__ void __launch_bounds__(32 * ZPipe<T, N>::WARPS, ZPipe<T, N>::MINB)
+k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __restrict__ uphys, int ulayout, T s,
+               const cplx<T>* __restrict__ tw, unsigned* status, unsigned wait_limit, int stall, long long NR) {
+  using Z = ZCfg<T, N>;
+  using ZP = ZPipe<T, N>;
+  constexpr int E = Z::E, R = Z::R, WARPS = ZP::WARPS;
   constexpr int MZ = Cfg<N>::MZP, KIN = Cfg<N>::KC + 1;  // the plan's cube (checked at launch)
-  const long long stage_elems = 12LL * MZ;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int unit, j;
+  z_lane<N, E>(unit, j);
+  const bool own = lane < R * Z::NT;
   cplx<T>* base = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* stage = base + warp * stage_elems;
-  cplx<T>* sb = base + nwarps * stage_elems + warp * Cfg<N>::ZBUF;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + nwarps * (stage_elems + Cfg<N>::ZBUF)) + 3 * warp;
+  cplx<T>* stage = base + warp * ZP::STAGE;
+  cplx<T>* sb = base + WARPS * ZP::STAGE + warp * ZP::EX + unit * Z::ZBUF;
+  cplx<T>* tws = base + WARPS * (ZP::STAGE + ZP::EX);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tws + ZP::TW) + 4 * warp;
   const long long fs = NR * MZ;
-  const unsigned rowbytes = (unsigned)(MZ * sizeof(cplx<T>));
-  const long long stride = (long long)gridDim.x * nwarps;
-  long long row = (long long)blockIdx.x * nwarps + warp;
+  const long long stride = (long long)gridDim.x * WARPS * R;
+  long long row = ((long long)blockIdx.x * WARPS + warp) * R;  // NR is a multiple of R
   if (lane == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    mbar_init(&bars[2], 1);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) mbar_init(&bars[q], 1);
     mbar_init_fence();
   }
+  typename std::conditional<Z::TWREG, TwRegs<T, N, E>, TwLane<T, N, E>>::type twr;
+  if constexpr (Z::TWREG) {
+    twr.load(tw, j);
+  } else {
+    TwLane<T, N, E>::fill(tws, tw, threadIdx.x, 32 * WARPS);
+    twr.p = tws + j;
+    __syncthreads();
+  }
   __syncwarp();
-  auto issue = [&](long long r, int b) {
+  auto issue = [&](long long r, int q) {  // fields 2 q, 2 q + 1 of rows r .. r + R - 1
     if (lane == 0) {
+      constexpr unsigned bytes = (unsigned)(R * MZ * sizeof(cplx<T>));
       fence_proxy_async();
-      mbar_expect_tx(&bars[b], 6u * rowbytes);
-#pragma unroll
-      for (int f = 0; f < 6; ++f) bulk_g2s(stage + (6 * b + f) * (long long)MZ, W + f * fs + r * MZ, rowbytes, &bars[b]);
+      mbar_expect_tx(&bars[q], 2u * bytes);
+      bulk_g2s(stage + 2 * q * R * MZ, W + 2 * q * fs + r * MZ, bytes, &bars[q]);
+      bulk_g2s(stage + (2 * q + 1) * R * MZ, W + (2 * q + 1) * fs + r * MZ, bytes, &bars[q]);
     }
   };
-  unsigned ph[2] = {0u, 0u};
-  bool pend[2] = {false, false};
-  if (row < NR) { issue(row, 0); pend[0] = true; }
-  if (stall && row < NR && !mbar_wait_bounded(&bars[2], 0u, wait_limit)) {
+  if (row < NR) {
+    issue(row, 0);
+    issue(row, 1);
+    issue(row, 2);
+  }
+  if (stall && row < NR && !__all_sync(0xffffffffu, mbar_wait_bounded(&bars[3], 0u, wait_limit))) {
     if (lane == 0) atomicOr(status, LD_STATUS_WAIT_TIMEOUT);
-    mbar_wait_bounded(&bars[0], ph[0], kWaitLimit);  // the first row's copy is in flight
+    for (int q = 0; q < 3; ++q) mbar_wait_bounded(&bars[q], 0u, kWaitLimit);  // the first rows' copies are in flight
     return;
   }
-  int b = 0;
-  for (; row < NR; row += stride, b ^= 1) {
-    const long long next = row + stride;
-    if (next < NR) { issue(next, b ^ 1); pend[b ^ 1] = true; }
-    if (!mbar_wait_bounded(&bars[b], ph[b], wait_limit)) {
+  unsigned ph = 0;
+  // pair q of this group into registers, then its next group's copy; false after a time-out (pairs
+  // before q already belong to the next group's phase, when there is one)
+  auto take = [&](cplx<T>* a, int q, long long next) -> bool {
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[q], ph, wait_limit))) {
       if (lane == 0) atomicOr(status, LD_STATUS_WAIT_TIMEOUT);
-      for (int q = 0; q < 2; ++q)
-        if (pend[q]) mbar_wait_bounded(&bars[q], ph[q], kWaitLimit);
-      return;
+      for (int b = 0; b < 3; ++b)
+        if (b >= q) mbar_wait_bounded(&bars[b], ph, kWaitLimit);
+        else if (next < NR) mbar_wait_bounded(&bars[b], ph ^ 1u, kWaitLimit);
+      return false;
     }
-    ph[b] ^= 1u;
-    pend[b] = false;
-    const cplx<T>* st = stage + 6 * b * (long long)MZ;
-    const cplx<T>* in[6];
-#pragma unroll
-    for (int f = 0; f < 6; ++f) in[f] = st + f * MZ;
-    zcross_row<T, N>(in, sb, P, fs, row, uphys, ulayout, MZ, KIN, s, lane, tw);
-    __syncwarp();  // every lane is done with staging buffer b and the exchange buffer
+    const cplx<T>* A = stage + (2 * q * R + unit) * MZ;
+    zload_pair<T, N, E>(a, A, A + R * MZ, KIN, j, s);
+    __syncwarp();  // every lane has read the pair
+    if (next < NR) issue(next, q);
+    return true;
+  };
+  for (; row < NR; row += stride, ph ^= 1u) {
+    const long long next = row + stride;
+    cplx<T> p0[E], p1[E], p2[E];
+    if (!take(p0, 0, next)) return;  // (u_x, u_y)
+    fft_run<T, N, E, true, true>(p0, sb, 1, j, twr, SyncWarp());
+    if (!take(p1, 1, next)) return;  // (u_z, w_x); its __syncwarp frees the exchange buffer
+    fft_run<T, N, E, true, true>(p1, sb, 1, j, twr, SyncWarp());
+    if (!take(p2, 2, next)) return;  // (w_y, w_z)
+    fft_run<T, N, E, true, true>(p2, sb, 1, j, twr, SyncWarp());
+    __syncwarp();
+    cplx<T>* out = P + (row + unit) * MZ;
+    zcross_forward<T, N>(p0, p1, p2, sb, out, out + fs, out + 2 * fs, row + unit, uphys, ulayout, MZ, KIN, j, own, twr);
+    __syncwarp();  // every lane is done with the exchange buffer
   }
 }
 

@@ -79,15 +79,15 @@ int na_run(const float2* fu, float* u, int ncomp, float2* W, const float2* tw, c
   const long long per = NN * Nf;
   const float sc = (float)(1.0 / ((double)N * N * N));
   for (int c = 0; c < ncomp; ++c) {
-    auto xin = O::io(fu + c * per, per, 0, N * Nf, -1);
-    auto xout = O::io(W, per, 0, N * Nf, -1);
+    auto xin = O::io(fu + c * per, per, 0);
+    auto xout = O::io(W, per, 0);
     // the loaders and storers of Ops::irfft_full (plain rows), so both paths run the same kernels
-    if (int rc = O::template colpass<true>(nullptr, KID_XPASS, ld::LdRowsC<float, N, false>{xin},
-                                           ld::StRowsC<float, N, false>{xout}, N * Nf, 1, 1, tw, s))
+    if (int rc = O::template colpass<true>(nullptr, KID_XPASS, ld::LdRowsC<float, N, false, O::RS::XF>{xin},
+                                           ld::StRowsC<float, N, false, O::RS::XF>{xout}, N * Nf, 1, 1, tw, s))
       return rc;
-    auto yio = O::io(W, per, (long long)N * Nf, Nf, -1);
-    if (int rc = O::template colpass<true>(nullptr, KID_YINV, ld::LdRowsC<float, N, false>{yio},
-                                           ld::StRowsC<float, N, false>{yio}, Nf, 1, N, tw, s))
+    auto yio = O::io(W, per, (long long)N * Nf);
+    if (int rc = O::template colpass<true>(nullptr, KID_YINV, ld::LdRowsC<float, N, false, O::RS::YF>{yio},
+                                           ld::StRowsC<float, N, false, O::RS::YF>{yio}, Nf, 1, N, tw, s))
       return rc;
     if (int rc = O::z_c2r(nullptr, W, u + c * NN * N, NN, Nf, Nf, sc, NN * N, per, 1, tw, s)) return rc;
   }

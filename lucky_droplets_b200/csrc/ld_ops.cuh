@@ -35,7 +35,8 @@ template <typename T, int N> struct Ops {
   using C = cplx<T>;
   static constexpr int TB = Cfg<N>::TB;
   static constexpr size_t COL_SMEM = sizeof(C) * N * TB;
-  static constexpr size_t Z_SMEM = sizeof(C) * Cfg<N>::ZROWS * Cfg<N>::ZBUF;
+  using Z = ZCfg<T, N>;
+  static constexpr size_t Z_SMEM = sizeof(C) * Z::UNITS1 * Z::ZBUF1;
 
   template <bool INV, class Ld, class St>
   static int colpass(ld_plan* p, int kid, Ld ld, St st, int ncols, int nf, int nouter, const C* tw, cudaStream_t s) {
@@ -92,8 +93,8 @@ template <typename T, int N> struct Ops {
     ProfScope ps(p, KID_ZC2R, s);
     auto k = k_z_c2r<T, N>;
     if (int rc = set_smem(k, Z_SMEM)) return rc;
-    dim3 grid((unsigned)cdiv(nrows / 2, Cfg<N>::ZROWS), (unsigned)nf);
-    k<<<grid, Cfg<N>::ZTHREADS, Z_SMEM, s>>>(X, x, nrows, ss, Kin, sc, xfs, Xfs, tw);
+    dim3 grid((unsigned)cdiv(nrows / 2, Z::UNITS1), (unsigned)nf);
+    k<<<grid, Z::THREADS1, Z_SMEM, s>>>(X, x, nrows, ss, Kin, sc, xfs, Xfs, tw);
     LD_LAUNCH_CHECK();
     return LD_OK;
   }
@@ -103,8 +104,8 @@ template <typename T, int N> struct Ops {
     ProfScope ps(p, KID_ZR2C, s);
     auto k = k_z_r2c<T, N>;
     if (int rc = set_smem(k, Z_SMEM)) return rc;
-    dim3 grid((unsigned)cdiv(nrows / 2, Cfg<N>::ZROWS), (unsigned)nf);
-    k<<<grid, Cfg<N>::ZTHREADS, Z_SMEM, s>>>(x, X, nrows, ss, Kout, Kval, xfs, Xfs, tw);
+    dim3 grid((unsigned)cdiv(nrows / 2, Z::UNITS1), (unsigned)nf);
+    k<<<grid, Z::THREADS1, Z_SMEM, s>>>(x, X, nrows, ss, Kout, Kval, xfs, Xfs, tw);
     LD_LAUNCH_CHECK();
     return LD_OK;
   }
@@ -214,17 +215,16 @@ template <typename T, int N> struct Ops {
     return LD_OK;
   }
 
-  // ---- pipelined fused z pass (one warp per row) -------------------------------------------------
+  // ---- pipelined fused z pass (rows inside a warp) -----------------------------------------------
   static int zcross_pipe(ld_plan* p, const C* W2, C* W1, T* uout, int ulayout, T sc, cudaStream_t s) {
-    constexpr int WARPS = sizeof(T) == 4 ? 8 : 4;
-    const long long NN = (long long)N * N * p->nbox;  // rows per field, all boxes
-    const size_t smem = (size_t)WARPS * ((size_t)12 * p->Mzp + Cfg<N>::ZBUF) * sizeof(C) + 24 * WARPS;
+    using ZP = ZPipe<T, N>;
+    const long long NR = (long long)N * N * p->nbox;  // rows per field, all boxes
     auto k = k_z_cross_pipe<T, N>;
-    if (int rc = set_smem(k, smem)) return rc;
+    if (int rc = set_smem(k, ZP::SMEM)) return rc;
     static int blocks_per_sm = -1;
     if (blocks_per_sm < 0) {
       int b = 0;
-      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, WARPS * 32, smem);
+      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, ZP::WARPS * 32, ZP::SMEM);
       if (e != cudaSuccess) { ld_set_last_error(e); return LD_ERR_CUDA; }
       blocks_per_sm = b > 0 ? b : 1;
     }
@@ -232,10 +232,10 @@ template <typename T, int N> struct Ops {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     long long grid = (long long)sms * blocks_per_sm;
-    const long long need = (NN + WARPS - 1) / WARPS;
+    const long long need = cdiv(NR, (long long)ZP::WARPS * Z::R);
     if (grid > need) grid = need;
-    k<<<(unsigned)grid, WARPS * 32, smem, s>>>(W2, W1, uout, ulayout, p->Mzp, p->kc, sc, (const C*)p->tw, p->status,
-                                               p->wait_limit, p->wait_stall, NN);
+    k<<<(unsigned)grid, ZP::WARPS * 32, ZP::SMEM, s>>>(W2, W1, uout, ulayout, sc, (const C*)p->tw, p->status,
+                                                       p->wait_limit, p->wait_stall, NR);
     LD_LAUNCH_CHECK();
     return LD_OK;
   }
@@ -308,6 +308,8 @@ template <typename T, int N> struct Ops {
     LdCurl<T, N> lc{y, cs, kc, My, Mzp, 3 * cs};
     auto xout = io(W1, nb * w1s, w1s, My * Mzp, -1);
     if (int rc = colpass<true>(p, KID_XINV, lc, StRowsC<T, N, false>{xout}, My * Mzp, 6, nb, tw, s)) return rc;
+    const T sc = T(1.0 / (double(N) * N * N));
+    const int ulayout = (MODE == UPD_RHS) ? 0 : 1;  // the time steppers feed droplets: interleaved
     // inverse y pass
     auto yin = io(W1, nb * w1s, (long long)My * Mzp, Mzp, kc);
     auto yout = io(W2, nb * w2s, (long long)N * Mzp, Mzp, -1);
@@ -316,18 +318,7 @@ template <typename T, int N> struct Ops {
     // fused z pass: u, w -> u x w  (W2 -> W1 as (3, N*N, Mzp))
     {
       ProfScope ps(p, KID_ZCROSS, s);
-      const T sc = T(1.0 / (double(N) * N * N));
-      const int ulayout = (MODE == UPD_RHS) ? 0 : 1;  // the time steppers feed droplets: interleaved
-      if constexpr (Cfg<N>::NTZ == 32) {
-        if (int rc = zcross_pipe(p, W2, W1, uout, ulayout, sc, s)) return rc;
-      } else {
-        auto k = k_z_cross<T, N>;
-        if (int rc = set_smem(k, Z_SMEM)) return rc;
-        const long long rows = NN * nb;
-        k<<<(unsigned)(rows / Cfg<N>::ZROWS), Cfg<N>::ZTHREADS, Z_SMEM, s>>>(W2, W1, uout, ulayout, Mzp, kc, sc, tw,
-                                                                            rows);
-        LD_LAUNCH_CHECK();
-      }
+      if (int rc = zcross_pipe(p, W2, W1, uout, ulayout, sc, s)) return rc;
     }
     // forward y pass (W1 -> W2 as (3, N, My, Mzp))
     auto fyin = io(W1, nb * w2s, (long long)N * Mzp, Mzp, -1);
