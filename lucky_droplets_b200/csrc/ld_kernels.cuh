@@ -882,6 +882,132 @@ k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __rest
 }
 
 // ------------------------------------------------------------------------------------------
+// plane pass of small grids: inverse y, fused z and forward y of one x plane in shared memory
+// ------------------------------------------------------------------------------------------
+// The six fields' columns kz <= kc of one (box, x) plane fit one SM's shared memory for N <= 64
+// (FP32 also 96): one block transforms them along y, takes the rows through the fused z pass and
+// the three products back along y, so that neither the (6, N, N, Mzp) nor the (3, N, N, Mzp)
+// intermediate goes through global memory and three launches become one.  Larger planes do not
+// fit (128^2 in FP32: 270 KB) and take the separate passes.
+// Row y of the plane holds its NC = 6 (kc + 1) values, columns (field, kz) contiguous; the z
+// transforms of a row exchange inside the row, past the two products stored first.  The row pitch
+// is NT mod 16 elements (FP32; mod 8 in FP64), so that the rows a half-warp (quarter-warp) works on
+// start NT bank groups apart.  Along y a column of length N = R1 R2 takes two steps: R2 threads of
+// radix R1 over y = j + R2 m, the twiddles W^(j k), then R1 threads of radix R2 over j; each step
+// reads and writes the same places, so one block barrier separates them.
+template <typename T, int N> struct PlaneCfg {
+  static constexpr bool OK = N == 16 || N == 32 || N == 64 || (N == 96 && sizeof(T) == 4);
+  static constexpr int M = OK ? N : 64;
+  using Z = ZCfg<T, M>;
+  static constexpr int KIN = Cfg<M>::KC + 1, NC = 6 * KIN;
+  static constexpr int R1 = M == 96 ? 12 : (M == 16 ? 4 : 8), R2 = M / R1;
+  static constexpr int MOD = sizeof(T) == 4 ? 16 : 8;
+  static constexpr int LEAST = NC > 2 * KIN + Z::ZBUF ? NC : 2 * KIN + Z::ZBUF;
+  static constexpr int PITCH = LEAST + ((Z::NT - LEAST) % MOD + MOD) % MOD;
+  static constexpr int THREADS = M == 96 ? 384 : (M == 16 ? 128 : 256);
+  static constexpr int TWZ = TwLane<T, M, Z::E>::ELEMS;
+  static constexpr size_t SMEM = sizeof(cplx<T>) * ((size_t)M * PITCH + TWZ + M);
+  static constexpr int MINB = M == 64 && sizeof(T) == 4 ? 3 : 1;
+};
+
+// W: (6, NO, My, Mzp) in (columns kz <= kc read), P: (3, NO, My, Mzp) out, NO = boxes x N planes
+template <typename T, int N>
+__global__ void __launch_bounds__(PlaneCfg<T, N>::THREADS, PlaneCfg<T, N>::MINB)
+k_plane(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __restrict__ uphys, int ulayout, T s,
+        const cplx<T>* __restrict__ tw, long long NO) {
+  using C = PlaneCfg<T, N>;
+  using Z = ZCfg<T, N>;
+  constexpr int R1 = C::R1, R2 = C::R2, KIN = C::KIN, PITCH = C::PITCH, THREADS = C::THREADS, E = Z::E, NT = Z::NT;
+  constexpr int MY = Cfg<N>::MY, MZ = Cfg<N>::MZP;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* F = reinterpret_cast<cplx<T>*>(smem_raw);
+  cplx<T>* twz = F + N * PITCH;
+  cplx<T>* twy = twz + C::TWZ;
+  const int tid = threadIdx.x;
+  const long long o = blockIdx.x;
+  for (int i = tid; i < N; i += THREADS) twy[i] = tw[i];
+  TwLane<T, N, E>::fill(twz, tw, tid, THREADS);
+  __syncthreads();
+  // y inverse, first step: cube rows from global memory
+  for (int t = tid; t < C::NC * R2; t += THREADS) {
+    const int j = t / C::NC, col = t - j * C::NC, f = col / KIN, c = col - f * KIN;
+    const cplx<T>* src = W + (f * NO + o) * (MY * MZ) + c;
+    cplx<T> a[R1];
+#pragma unroll
+    for (int m = 0; m < R1; ++m) {
+      const int r = crow(j + R2 * m, N, Cfg<N>::KC);
+      a[m] = r < 0 ? czero<cplx<T>>() : src[r * MZ];
+    }
+    dft_any<T, R1, true>(a);
+#pragma unroll
+    for (int k = 0; k < R1; ++k)
+      F[(k + R1 * j) * PITCH + col] = k ? cmul(a[k], twid<T, true>(twy, j * k)) : a[k];
+  }
+  __syncthreads();
+  for (int t = tid; t < C::NC * R1; t += THREADS) {
+    const int k = t / C::NC, col = t - k * C::NC;
+    cplx<T> a[R2];
+#pragma unroll
+    for (int j = 0; j < R2; ++j) a[j] = F[(k + R1 * j) * PITCH + col];
+    dft_any<T, R2, true>(a);
+#pragma unroll
+    for (int j = 0; j < R2; ++j) F[(k + R1 * j) * PITCH + col] = a[j];
+  }
+  __syncthreads();
+  // z rows: NT lanes each, whole warps
+  static_assert(N * NT % 32 == 0 && 32 % NT == 0, "whole rows per warp");
+  for (int t = tid; t < N * NT; t += THREADS) {
+    const int y = t / NT;
+    int j = t % NT;
+    __builtin_assume(j >= 0 && j < NT);
+    cplx<T>* row = F + y * PITCH;
+    cplx<T>* sb = row + 2 * KIN;
+    TwLane<T, N, E> twr;
+    twr.p = twz + j;
+    cplx<T> p0[E], p1[E], p2[E];
+    zload_pair<T, N, E>(p0, row, row + KIN, KIN, j, s);                // (u_x, u_y)
+    zload_pair<T, N, E>(p1, row + 2 * KIN, row + 3 * KIN, KIN, j, s);  // (u_z, w_x)
+    zload_pair<T, N, E>(p2, row + 4 * KIN, row + 5 * KIN, KIN, j, s);  // (w_y, w_z)
+    __syncwarp();
+    fft_run<T, N, E, true, true>(p0, sb, 1, j, twr, SyncWarp());
+    __syncwarp();
+    fft_run<T, N, E, true, true>(p1, sb, 1, j, twr, SyncWarp());
+    __syncwarp();
+    fft_run<T, N, E, true, true>(p2, sb, 1, j, twr, SyncWarp());
+    __syncwarp();
+    zcross_forward<T, N>(p0, p1, p2, sb, row, row + KIN, row + 2 * KIN, o * N + y, uphys, ulayout, KIN, KIN, j, true,
+                         twr);
+  }
+  __syncthreads();
+  // y forward of the three products
+  constexpr int NP = 3 * KIN;
+  for (int t = tid; t < NP * R2; t += THREADS) {
+    const int j = t / NP, col = t - j * NP;
+    cplx<T> a[R1];
+#pragma unroll
+    for (int m = 0; m < R1; ++m) a[m] = F[(j + R2 * m) * PITCH + col];
+    dft_any<T, R1, false>(a);
+#pragma unroll
+    for (int k = 0; k < R1; ++k)
+      F[(j + R2 * k) * PITCH + col] = k ? cmul(a[k], twid<T, false>(twy, j * k)) : a[k];
+  }
+  __syncthreads();
+  for (int t = tid; t < 3 * MZ * R1; t += THREADS) {  // the padding columns are written too: whole sectors
+    const int k = t / (3 * MZ), col = t - k * (3 * MZ), f = col / MZ, c = col - f * MZ;
+    cplx<T> a[R2];
+#pragma unroll
+    for (int j = 0; j < R2; ++j) a[j] = c < KIN ? F[(j + R2 * k) * PITCH + f * KIN + c] : czero<cplx<T>>();
+    dft_any<T, R2, false>(a);
+    cplx<T>* dst = P + (f * NO + o) * (MY * MZ) + c;
+#pragma unroll
+    for (int j = 0; j < R2; ++j) {
+      const int r = crow(k + R1 * j, N, Cfg<N>::KC);
+      if (r >= 0) dst[r * MZ] = a[j];
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------
 // cube <-> reference layout, spectra, forcing, epilogue
 // ------------------------------------------------------------------------------------------
 template <typename T>

@@ -310,21 +310,31 @@ template <typename T, int N> struct Ops {
     if (int rc = colpass<true>(p, KID_XINV, lc, StRowsC<T, N, false>{xout}, My * Mzp, 6, nb, tw, s)) return rc;
     const T sc = T(1.0 / (double(N) * N * N));
     const int ulayout = (MODE == UPD_RHS) ? 0 : 1;  // the time steppers feed droplets: interleaved
-    // inverse y pass
-    auto yin = io(W1, nb * w1s, (long long)My * Mzp, Mzp, kc);
-    auto yout = io(W2, nb * w2s, (long long)N * Mzp, Mzp, -1);
-    if (int rc = colpass_rows<true, true>(p, KID_YINV, yin, StRowsC<T, N, false>{yout}, Mzp, 6, nb * N, tw, s))
-      return rc;
-    // fused z pass: u, w -> u x w  (W2 -> W1 as (3, N*N, Mzp))
-    {
+    if constexpr (PlaneCfg<T, N>::OK) {
+      // y inverse, fused z and y forward of one x plane per block (W1 -> W2 as (3, N, My, Mzp))
+      using PC = PlaneCfg<T, N>;
       ProfScope ps(p, KID_ZCROSS, s);
-      if (int rc = zcross_pipe(p, W2, W1, uout, ulayout, sc, s)) return rc;
+      auto k = k_plane<T, N>;
+      if (int rc = set_smem(k, PC::SMEM)) return rc;
+      k<<<(unsigned)(nb * N), PC::THREADS, PC::SMEM, s>>>(W1, W2, uout, ulayout, sc, tw, (long long)nb * N);
+      LD_LAUNCH_CHECK();
+    } else {
+      // inverse y pass
+      auto yin = io(W1, nb * w1s, (long long)My * Mzp, Mzp, kc);
+      auto yout = io(W2, nb * w2s, (long long)N * Mzp, Mzp, -1);
+      if (int rc = colpass_rows<true, true>(p, KID_YINV, yin, StRowsC<T, N, false>{yout}, Mzp, 6, nb * N, tw, s))
+        return rc;
+      // fused z pass: u, w -> u x w  (W2 -> W1 as (3, N*N, Mzp))
+      {
+        ProfScope ps(p, KID_ZCROSS, s);
+        if (int rc = zcross_pipe(p, W2, W1, uout, ulayout, sc, s)) return rc;
+      }
+      // forward y pass (W1 -> W2 as (3, N, My, Mzp))
+      auto fyin = io(W1, nb * w2s, (long long)N * Mzp, Mzp, -1);
+      auto fyout = io(W2, nb * w1s, (long long)My * Mzp, Mzp, kc);
+      if (int rc = colpass_rows<false, false>(p, KID_YFWD, fyin, StRowsC<T, N, true>{fyout}, Mzp, 3, nb * N, tw, s))
+        return rc;
     }
-    // forward y pass (W1 -> W2 as (3, N, My, Mzp))
-    auto fyin = io(W1, nb * w2s, (long long)N * Mzp, Mzp, -1);
-    auto fyout = io(W2, nb * w1s, (long long)My * Mzp, Mzp, kc);
-    if (int rc = colpass_rows<false, false>(p, KID_YFWD, fyin, StRowsC<T, N, true>{fyout}, Mzp, 3, nb * N, tw, s))
-      return rc;
     // forward x pass + k-space update
     UpdArgs<T> A;
     A.nl = W2; A.nls = nb * w1s;
