@@ -84,75 +84,56 @@ template <typename T, int N> struct ZCfg {
 // ------------------------------------------------------------------------------------------
 // column (strided axis) passes
 // ------------------------------------------------------------------------------------------
-// Plain strided loader/storer: element (f, o, row, col) at f*fs + o*os + row*rs + col, with an
-// optional cube row map (kc >= 0) on the transform axis.
+// Plain strided rows: element (f, o, row, col) at f*fs + o*os + row*RS + col.  The row stride RS is
+// a template constant (every pass has one fixed by N), so that the rows of a thread are one base
+// address and immediate offsets: the y passes spent a third of their instructions on addresses.
 template <typename T> struct RowsIO {
   cplx<T>* p;
   long long fs, os;
-  int rs;
-  int kc;  // < 0: identity row map
-  __device__ __forceinline__ long long at(int f, int o, int r, int col) const {
-    return (long long)f * fs + (long long)o * os + (long long)r * rs + col;
+  __device__ __forceinline__ cplx<T>* at(int f, int o, int col) const {
+    return p + ((long long)f * fs + (long long)o * os + col);
   }
 };
-
-
-// Strided row loader and storer with the row map chosen at run time (io.kc < 0: rows as they are,
-// else compact cube rows through crow).
-template <typename T, int N> struct LdRows {
-  RowsIO<T> io;
-  __device__ __forceinline__ cplx<T> operator()(int f, int o, int n, int col) const {
-    const int r = io.kc < 0 ? n : crow(n, N, io.kc);
-    if (r < 0) return czero<cplx<T>>();
-    return io.p[io.at(f, o, r, col)];
-  }
-};
-
-template <typename T, int N> struct StRows {
-  RowsIO<T> io;
-  __device__ __forceinline__ void operator()(int f, int o, int n, int col, cplx<T> v) const {
-    const int r = io.kc < 0 ? n : crow(n, N, io.kc);
-    if (r < 0) return;
-    io.p[io.at(f, o, r, col)] = v;
-  }
+// Row strides of the passes: y and x passes over cube rows, y and x passes over reference-layout rows
+template <int N> struct RowStride {
+  static constexpr int YC = Cfg<N>::MZP, XC = Cfg<N>::MY * Cfg<N>::MZP;
+  static constexpr int YF = N / 2 + 1, XF = N * (N / 2 + 1);
 };
 
 // Strided row loader: rows mapped to compact cube rows through crow (MAP) or taken as they are.
-template <typename T, int N, bool MAP> struct LdRowsC {
+template <typename T, int N, bool MAP, int RS> struct LdRowsC {
   RowsIO<T> io;
   __device__ __forceinline__ cplx<T> operator()(int f, int o, int n, int col) const {
-    const int r = MAP ? crow(n, N, Cfg<N>::KC) : n;  // io.kc == Cfg<N>::KC for cube rows
+    const int r = MAP ? crow(n, N, Cfg<N>::KC) : n;
     if (r < 0) return czero<cplx<T>>();
-    return io.p[io.at(f, o, r, col)];
+    return io.at(f, o, col)[(long long)r * RS];
   }
 };
 
-
 // Strided row storer: rows mapped to compact cube rows through crow (MAP; rows outside the cube
 // are not written) or taken as they are.
-template <typename T, int N, bool MAP> struct StRowsC {
+template <typename T, int N, bool MAP, int RS> struct StRowsC {
   RowsIO<T> io;
   __device__ __forceinline__ void operator()(int f, int o, int n, int col, cplx<T> v) const {
-    const int r = MAP ? crow(n, N, Cfg<N>::KC) : n;  // io.kc == Cfg<N>::KC for cube rows
+    const int r = MAP ? crow(n, N, Cfg<N>::KC) : n;
     if (r < 0) return;
-    io.p[io.at(f, o, r, col)] = v;
+    io.at(f, o, col)[(long long)r * RS] = v;
   }
 };
 
 // Storer into the cube that also applies the spherical mask round(|k|) <= kc (F:129): the last
 // (x) pass of a forward cube transform.  Columns are the flat (ky, kz) index of a kx plane.
 template <typename T, int N> struct StCube {
-  RowsIO<T> io;  // io.kc = kc (compact rows), io.rs = My * Mzp
-  int Mzp;
+  RowsIO<T> io;
   __device__ __forceinline__ void operator()(int f, int o, int n, int col, cplx<T> v) const {
-    const int kc = io.kc;
+    constexpr int kc = Cfg<N>::KC, Mzp = Cfg<N>::MZP;
     const int r = crow(n, N, kc);
     if (r < 0) return;
     const int kx = n <= kc ? n : n - N;
     const int iy = col / Mzp;
     const int ky = cfreq(iy, kc), kz = col - iy * Mzp;
     if (kz > kc || kx * kx + ky * ky + kz * kz > kc * kc + kc) v = czero<cplx<T>>();
-    io.p[io.at(f, o, r, col)] = v;
+    io.at(f, o, col)[(long long)r * RowStride<N>::XC] = v;
   }
 };
 
@@ -161,7 +142,6 @@ template <typename T, int N> struct StCube {
 template <typename T, int N> struct LdCurl {
   const cplx<T>* u;
   long long cs;  // component stride (cube elements)
-  int kc_, My_, Mzp_;  // the plan's cube; equal to Cfg<N>::KC, MY, MZP, which the loader uses
   long long bs;  // box stride (elements): the outer index is the box of a multi-box plan
   static constexpr int kc = Cfg<N>::KC, My = Cfg<N>::MY, Mzp = Cfg<N>::MZP;
   __device__ __forceinline__ cplx<T> operator()(int f, int o, int n, int col) const {
@@ -197,6 +177,7 @@ k_colfft(Ld ld, St st, int ncols, int nf, const cplx<T>* __restrict__ tw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
   const int c = threadIdx.x % TB, j = threadIdx.x / TB;
+  __builtin_assume(j >= 0 && j < NT);
   const int field = blockIdx.x % nf;
   const int col = (blockIdx.x / nf) * TB + c;
   const bool ok = col < ncols;
@@ -224,6 +205,7 @@ k_colfft5(Ld ld, St st, int ncols, int nf, const cplx<T>* __restrict__ tw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
   const int c = threadIdx.x % TB, j = threadIdx.x / TB;
+  __builtin_assume(j >= 0 && j < NT);
   const int field = blockIdx.x % nf;
   const int col = (blockIdx.x / nf) * TB + c;
   const bool ok = col < ncols;
@@ -249,7 +231,7 @@ constexpr auto colfft_kernel() {
 // rows of the CTA's next item stream into the other shared buffer with 16-byte cp.async copies;
 // the buffer an item was staged in serves as its FFT exchange buffer once its values sit in
 // registers.  Rows the loader's row map drops (r < 0) and columns past ncols are not copied.
-template <typename T, int N, bool INV, class St, bool IN_MAP>
+template <typename T, int N, bool INV, class St, bool IN_MAP, int RS>
 __global__ void __launch_bounds__(Cfg<N>::COL_THREADS, 3)
 k_colfft_pipe(RowsIO<T> in, St st, int ncols, int nf, int nouter, const cplx<T>* __restrict__ tw) {
   constexpr int E = Cfg<N>::EC, TB = Cfg<N>::TB, NT = Cfg<N>::NTC;
@@ -258,6 +240,7 @@ k_colfft_pipe(RowsIO<T> in, St st, int ncols, int nf, int nouter, const cplx<T>*
   cplx<T>* buf0 = reinterpret_cast<cplx<T>*>(smem_raw);
   cplx<T>* buf1 = buf0 + N * TB;
   const int c = threadIdx.x % TB, j = threadIdx.x / TB;
+  __builtin_assume(j >= 0 && j < NT);
   // item = (column block cb, field f, outer o), cb fastest; the launcher keeps the item count
   // below 2^31, so items are split with 32-bit unsigned division
   const unsigned ncb = (unsigned)((ncols + TB - 1) / TB);
@@ -274,19 +257,20 @@ k_colfft_pipe(RowsIO<T> in, St st, int ncols, int nf, int nouter, const cplx<T>*
   constexpr int THREADS = Cfg<N>::COL_THREADS;
   static_assert(THREADS % CPR == 0 && (N * CPR) % THREADS == 0, "whole rows per pass of the block");
   const int kq = threadIdx.x % CPR, n0 = threadIdx.x / CPR;
+  __builtin_assume(n0 >= 0 && n0 < THREADS / CPR);
   auto prefetch = [&](const Item& itm, cplx<T>* dst) {
     const int col0 = itm.cb * TB;
     const int w = ncols - col0 < TB ? ncols - col0 : TB;
     const int cpr = w * (int)sizeof(cplx<T>) / 16;
     if (kq < cpr) {
-      const char* src0 = reinterpret_cast<const char*>(in.p + in.at(itm.f, itm.o, 0, col0)) + 16 * kq;
+      const char* src0 = reinterpret_cast<const char*>(in.at(itm.f, itm.o, col0)) + 16 * kq;
       const unsigned d0 = (unsigned)__cvta_generic_to_shared(reinterpret_cast<char*>(dst) + 16 * kq);
 #pragma unroll
       for (int i = 0; i < N * CPR / THREADS; ++i) {
         const int n = n0 + (THREADS / CPR) * i;
-        const int r = IN_MAP ? crow(n, N, in.kc) : n;
+        const int r = IN_MAP ? crow(n, N, Cfg<N>::KC) : n;
         if (r < 0) continue;
-        const char* src = src0 + (long long)r * in.rs * (long long)sizeof(cplx<T>);
+        const char* src = src0 + (long long)r * (RS * (long long)sizeof(cplx<T>));
         const unsigned d = d0 + (unsigned)(n * TB * (int)sizeof(cplx<T>));
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
       }
@@ -308,7 +292,7 @@ k_colfft_pipe(RowsIO<T> in, St st, int ncols, int nf, int nouter, const cplx<T>*
 #pragma unroll
     for (int m = 0; m < E; ++m) {
       const int n = j + NT * m;
-      const int r = IN_MAP ? crow(n, N, in.kc) : n;
+      const int r = IN_MAP ? crow(n, N, Cfg<N>::KC) : n;
       a[m] = (ok && r >= 0) ? cur[n * TB + c] : czero<cplx<T>>();
     }
     __syncthreads();  // every value is in registers: cur becomes the exchange buffer
@@ -358,9 +342,9 @@ template <typename T> struct UpdArgs {
   // vk = y + tps (k (k . rhs) / k^2 + visc nu k^2 y), minus vg = tps g N^3 on the mean of w
   cplx<T>* vk;
   T tps, vg;
-  // RK2 stages: stage the cube rows of the CTA's columns that the update reads (s1 in stage 1,
-  // s2 in stage 2) into shared memory with cp.async while the x transforms run; the launcher
-  // sets it when the (3, Mx, TB) buffer fits beside the exchange buffer at 2 CTAs per SM
+  // stage the cube rows of the CTA's columns that the update reads for every mode (the stage input
+  // s1; s2 in the second RK2 stage) into shared memory with cp.async while the x transforms run; the
+  // launcher sets it when the (3, Mx, TB) buffer fits beside the exchange buffer at 2 CTAs per SM
   int prefetch;
   // final stages (UPD_RK2_2, UPD_RK4_4): the step epilogue's work on the kz > 0 modes (projection
   // and the non-finite / blow-up checks, as k_epilogue does them) is done here, so that the
@@ -409,15 +393,15 @@ k_xfwd_update(UpdArgs<T> A, int ncols, const cplx<T>* __restrict__ tw) {
   }
   cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
   const int c = threadIdx.x % TB, j = threadIdx.x / TB;
+  __builtin_assume(j >= 0 && j < NT);
   const int col = blockIdx.x * TB + c;
   const bool ok = col < ncols;
-  constexpr bool RK2 = MODE == UPD_RK2_1 || MODE == UPD_RK2_2;
   constexpr int Mx = Cfg<N>::MY;  // A.kc == Cfg<N>::KC, A.My == Cfg<N>::MY, A.Mzp == Cfg<N>::MZP
-  cplx<T>* ybuf = sbuf + N * TB;  // (3, Mx, TB) staged rows of s1 (stage 1) or s2 (stage 2)
-  const bool pre = RK2 && A.prefetch;
+  cplx<T>* ybuf = sbuf + N * TB;  // (3, Mx, TB) staged rows of s1 (s2 in the second RK2 stage)
+  const bool pre = A.prefetch;
   if (pre) {
     constexpr int PER = 16 / (int)sizeof(cplx<T>);  // elements per 16-byte chunk
-    const cplx<T>* src = MODE == UPD_RK2_1 ? A.s1 : A.s2;
+    const cplx<T>* src = MODE == UPD_RK2_2 ? A.s2 : A.s1;
     const int col0 = blockIdx.x * TB;
     const int w = ncols - col0 < TB ? ncols - col0 : TB;  // a multiple of 8 (Mzp is)
     const int cpr = w / PER;
@@ -439,7 +423,7 @@ k_xfwd_update(UpdArgs<T> A, int ncols, const cplx<T>* __restrict__ tw) {
   for (int f = 0; f < 3; ++f)
 #pragma unroll
     for (int m = 0; m < E; ++m)
-      res[f][m] = ok ? A.nl[f * A.nls + (long long)(j + NT * m) * ncols + col] : czero<cplx<T>>();
+      res[f][m] = ok ? A.nl[f * A.nls + col + (long long)(j + NT * m) * RowStride<N>::XC] : czero<cplx<T>>();
 #pragma unroll
   for (int f = 0; f < 3; ++f) {
     if (f) __syncthreads();
@@ -479,7 +463,7 @@ k_xfwd_update(UpdArgs<T> A, int ncols, const cplx<T>* __restrict__ tw) {
 #pragma unroll
     for (int cc = 0; cc < 3; ++cc)
       y[cc] = !need_y ? czero<cplx<T>>()
-                      : ((MODE == UPD_RK2_1 && pre) ? ybuf[(cc * Mx + r) * TB + c] : A.s1[cc * A.cs + idx]);
+                      : ((MODE != UPD_RK2_2 && pre) ? ybuf[(cc * Mx + r) * TB + c] : A.s1[cc * A.cs + idx]);
     cplx<T> rhs[3];
     cplx<T> kd = czero<cplx<T>>();  // (k . rhs) / k^2 before the projection
     if (keep) {

@@ -51,19 +51,18 @@ template <typename T, int N> struct Ops {
 
   // Column pass over plain strided rows: the pipelined kernel where two staging buffers fit.
   static constexpr bool PIPE = 2 * COL_SMEM <= 72 * 1024;
-  // IN_MAP: the input rows are compact cube rows (in.kc >= 0), fixed at compile time for the
-  // pipelined kernel
-  template <bool INV, bool IN_MAP, class St>
+  // IN_MAP: the input rows are compact cube rows; RS: their stride
+  template <bool INV, bool IN_MAP, int RS, class St>
   static int colpass_rows(ld_plan* p, int kid, RowsIO<T> in, St st, int ncols, int nf, int nouter, const C* tw,
                           cudaStream_t s, int variant = -2) {
     const int choice = variant != -2 ? variant : p->tune_y[INV ? 0 : 1];
     if constexpr (!PIPE) {
-      return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP>{in}, st, ncols, nf, nouter, tw, s);
+      return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
     } else {
       if (choice == 0 || cdiv(ncols, TB) * (long long)nf * nouter >= (1LL << 31))
-        return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP>{in}, st, ncols, nf, nouter, tw, s);
+        return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
       ProfScope ps(p, kid, s);
-      auto k = k_colfft_pipe<T, N, INV, St, IN_MAP>;
+      auto k = k_colfft_pipe<T, N, INV, St, IN_MAP, RS>;
       if (int rc = set_smem(k, 2 * COL_SMEM)) return rc;
       static int occ = 0;
       if (occ == 0) {
@@ -82,11 +81,8 @@ template <typename T, int N> struct Ops {
     }
   }
 
-  static RowsIO<T> io(const void* p, long long fs, long long os, int rs, int kc) {
-    RowsIO<T> r;
-    r.p = (C*)p; r.fs = fs; r.os = os; r.rs = rs; r.kc = kc;
-    return r;
-  }
+  static RowsIO<T> io(const void* p, long long fs, long long os) { return RowsIO<T>{(C*)p, fs, os}; }
+  using RS = RowStride<N>;
 
   static int z_c2r(ld_plan* p, const C* X, T* x, long long nrows, int ss, int Kin, T sc, long long xfs, long long Xfs,
                    int nf, const C* tw, cudaStream_t s) {
@@ -117,11 +113,11 @@ template <typename T, int N> struct Ops {
     const long long NN = (long long)N * N;
     if (int rc = z_r2c(p, u, fu, NN, Nf, Nf, Nf, NN * N, NN * Nf, ncomp, tw, s)) return rc;
     // y pass in place: columns kz (Nf), rows y, outer x
-    auto yio = io(fu, NN * Nf, (long long)N * Nf, Nf, -1);
-    if (int rc = colpass<false>(p, KID_YFWD, LdRowsC<T, N, false>{yio}, StRowsC<T, N, false>{yio}, Nf, ncomp, N, tw, s)) return rc;
+    auto yio = io(fu, NN * Nf, (long long)N * Nf);
+    if (int rc = colpass<false>(p, KID_YFWD, LdRowsC<T, N, false, RS::YF>{yio}, StRowsC<T, N, false, RS::YF>{yio}, Nf, ncomp, N, tw, s)) return rc;
     // x pass in place: columns (ky, kz) flat, rows x
-    auto xio = io(fu, NN * Nf, 0, N * Nf, -1);
-    return colpass<false>(p, KID_XPASS, LdRowsC<T, N, false>{xio}, StRowsC<T, N, false>{xio}, N * Nf, ncomp, 1, tw, s);
+    auto xio = io(fu, NN * Nf, 0);
+    return colpass<false>(p, KID_XPASS, LdRowsC<T, N, false, RS::XF>{xio}, StRowsC<T, N, false, RS::XF>{xio}, N * Nf, ncomp, 1, tw, s);
   }
 
   static int irfft_full(ld_plan* p, const C* fu, T* u, int ncomp, cudaStream_t s) {
@@ -133,11 +129,11 @@ template <typename T, int N> struct Ops {
     C* W = (C*)p->W2;
     for (int c0 = 0; c0 < ncomp; c0 += chunk) {
       const int nc = ncomp - c0 < chunk ? ncomp - c0 : chunk;
-      auto xin = io(fu + c0 * per, per, 0, N * Nf, -1);
-      auto xout = io(W, per, 0, N * Nf, -1);
-      if (int rc = colpass<true>(p, KID_XPASS, LdRowsC<T, N, false>{xin}, StRowsC<T, N, false>{xout}, N * Nf, nc, 1, tw, s)) return rc;
-      auto yio = io(W, per, (long long)N * Nf, Nf, -1);
-      if (int rc = colpass<true>(p, KID_YINV, LdRowsC<T, N, false>{yio}, StRowsC<T, N, false>{yio}, Nf, nc, N, tw, s)) return rc;
+      auto xin = io(fu + c0 * per, per, 0);
+      auto xout = io(W, per, 0);
+      if (int rc = colpass<true>(p, KID_XPASS, LdRowsC<T, N, false, RS::XF>{xin}, StRowsC<T, N, false, RS::XF>{xout}, N * Nf, nc, 1, tw, s)) return rc;
+      auto yio = io(W, per, (long long)N * Nf);
+      if (int rc = colpass<true>(p, KID_YINV, LdRowsC<T, N, false, RS::YF>{yio}, StRowsC<T, N, false, RS::YF>{yio}, Nf, nc, N, tw, s)) return rc;
       const T sc = T(1.0 / (double(N) * N * N));
       if (int rc = z_c2r(p, W, u + (long long)c0 * NN * N, NN, Nf, Nf, sc, NN * N, per, nc, tw, s)) return rc;
     }
@@ -155,12 +151,12 @@ template <typename T, int N> struct Ops {
     const long long w1s = (long long)N * My * Mzp, w2s = NN * Mzp;
     for (int c0 = 0; c0 < ncomp; c0 += 6) {
       const int nc = ncomp - c0 < 6 ? ncomp - c0 : 6;
-      auto xin = io(uk + c0 * cs, cs, 0, My * Mzp, kc);
-      auto xout = io(W1, w1s, 0, My * Mzp, -1);
-      if (int rc = colpass<true>(p, KID_XPASS, LdRowsC<T, N, true>{xin}, StRowsC<T, N, false>{xout}, My * Mzp, nc, 1, tw, s)) return rc;
-      auto yin = io(W1, w1s, (long long)My * Mzp, Mzp, kc);
-      auto yout = io(W2, w2s, (long long)N * Mzp, Mzp, -1);
-      if (int rc = colpass<true>(p, KID_YINV, LdRowsC<T, N, true>{yin}, StRowsC<T, N, false>{yout}, Mzp, nc, N, tw, s)) return rc;
+      auto xin = io(uk + c0 * cs, cs, 0);
+      auto xout = io(W1, w1s, 0);
+      if (int rc = colpass<true>(p, KID_XPASS, LdRowsC<T, N, true, RS::XC>{xin}, StRowsC<T, N, false, RS::XC>{xout}, My * Mzp, nc, 1, tw, s)) return rc;
+      auto yin = io(W1, w1s, (long long)My * Mzp);
+      auto yout = io(W2, w2s, (long long)N * Mzp);
+      if (int rc = colpass<true>(p, KID_YINV, LdRowsC<T, N, true, RS::YC>{yin}, StRowsC<T, N, false, RS::YC>{yout}, Mzp, nc, N, tw, s)) return rc;
       const T sc = T(1.0 / (double(N) * N * N));
       if (int rc = z_c2r(p, W2, u + (long long)c0 * NN * N, NN, Mzp, kc + 1, sc, NN * N, w2s, nc, tw, s)) return rc;
     }
@@ -178,12 +174,12 @@ template <typename T, int N> struct Ops {
     for (int c0 = 0; c0 < ncomp; c0 += 6) {
       const int nc = ncomp - c0 < 6 ? ncomp - c0 : 6;
       if (int rc = z_r2c(p, u + (long long)c0 * NN * N, W2, NN, Mzp, Mzp, kc + 1, NN * N, w2s, nc, tw, s)) return rc;
-      auto yin = io(W2, w2s, (long long)N * Mzp, Mzp, -1);
-      auto yout = io(W1, w1s, (long long)My * Mzp, Mzp, kc);
-      if (int rc = colpass<false>(p, KID_YFWD, LdRowsC<T, N, false>{yin}, StRowsC<T, N, true>{yout}, Mzp, nc, N, tw, s)) return rc;
-      auto xin = io(W1, w1s, 0, My * Mzp, -1);
-      auto xout = io(uk + c0 * cs, cs, 0, My * Mzp, kc);
-      if (int rc = colpass<false>(p, KID_XPASS, LdRowsC<T, N, false>{xin}, StCube<T, N>{xout, Mzp}, My * Mzp, nc, 1, tw, s)) return rc;
+      auto yin = io(W2, w2s, (long long)N * Mzp);
+      auto yout = io(W1, w1s, (long long)My * Mzp);
+      if (int rc = colpass<false>(p, KID_YFWD, LdRowsC<T, N, false, RS::YC>{yin}, StRowsC<T, N, true, RS::YC>{yout}, Mzp, nc, N, tw, s)) return rc;
+      auto xin = io(W1, w1s, 0);
+      auto xout = io(uk + c0 * cs, cs, 0);
+      if (int rc = colpass<false>(p, KID_XPASS, LdRowsC<T, N, false, RS::XC>{xin}, StCube<T, N>{xout}, My * Mzp, nc, 1, tw, s)) return rc;
     }
     return LD_OK;
   }
@@ -260,11 +256,11 @@ template <typename T, int N> struct Ops {
         auto run = [&]() -> int {
           const int nb = p->nbox;
           if (pass == 0)
-            return colpass_rows<true, true>(p, KID_YINV, io(W1, nb * w1s, (long long)My * Mzp, Mzp, kc),
-                                            StRowsC<T, N, false>{io(W2, nb * w2s, (long long)N * Mzp, Mzp, -1)}, Mzp,
+            return colpass_rows<true, true, RS::YC>(p, KID_YINV, io(W1, nb * w1s, (long long)My * Mzp),
+                                            StRowsC<T, N, false, RS::YC>{io(W2, nb * w2s, (long long)N * Mzp)}, Mzp,
                                             6, nb * N, tw, s, v);
-          return colpass_rows<false, false>(p, KID_YFWD, io(W1, nb * w2s, (long long)N * Mzp, Mzp, -1),
-                                            StRowsC<T, N, true>{io(W2, nb * w1s, (long long)My * Mzp, Mzp, kc)}, Mzp,
+          return colpass_rows<false, false, RS::YC>(p, KID_YFWD, io(W1, nb * w2s, (long long)N * Mzp),
+                                            StRowsC<T, N, true, RS::YC>{io(W2, nb * w1s, (long long)My * Mzp)}, Mzp,
                                             3, nb * N, tw, s, v);
         };
         if (int rc = run()) return rc;  // warm-up
@@ -305,9 +301,9 @@ template <typename T, int N> struct Ops {
     if (nb > 1 && p->sm_vk) return ld_fail(LD_ERR_UNSUPPORTED, "slow-manifold output of a multi-box plan");
     if (int rc = forcing_factor(p, y, prm, s)) return rc;
     // inverse x pass with the curl: 6 fields [u, w]
-    LdCurl<T, N> lc{y, cs, kc, My, Mzp, 3 * cs};
-    auto xout = io(W1, nb * w1s, w1s, My * Mzp, -1);
-    if (int rc = colpass<true>(p, KID_XINV, lc, StRowsC<T, N, false>{xout}, My * Mzp, 6, nb, tw, s)) return rc;
+    LdCurl<T, N> lc{y, cs, 3 * cs};
+    auto xout = io(W1, nb * w1s, w1s);
+    if (int rc = colpass<true>(p, KID_XINV, lc, StRowsC<T, N, false, RS::XC>{xout}, My * Mzp, 6, nb, tw, s)) return rc;
     const T sc = T(1.0 / (double(N) * N * N));
     const int ulayout = (MODE == UPD_RHS) ? 0 : 1;  // the time steppers feed droplets: interleaved
     if constexpr (PlaneCfg<T, N>::OK) {
@@ -320,9 +316,9 @@ template <typename T, int N> struct Ops {
       LD_LAUNCH_CHECK();
     } else {
       // inverse y pass
-      auto yin = io(W1, nb * w1s, (long long)My * Mzp, Mzp, kc);
-      auto yout = io(W2, nb * w2s, (long long)N * Mzp, Mzp, -1);
-      if (int rc = colpass_rows<true, true>(p, KID_YINV, yin, StRowsC<T, N, false>{yout}, Mzp, 6, nb * N, tw, s))
+      auto yin = io(W1, nb * w1s, (long long)My * Mzp);
+      auto yout = io(W2, nb * w2s, (long long)N * Mzp);
+      if (int rc = colpass_rows<true, true, RS::YC>(p, KID_YINV, yin, StRowsC<T, N, false, RS::YC>{yout}, Mzp, 6, nb * N, tw, s))
         return rc;
       // fused z pass: u, w -> u x w  (W2 -> W1 as (3, N*N, Mzp))
       {
@@ -330,9 +326,9 @@ template <typename T, int N> struct Ops {
         if (int rc = zcross_pipe(p, W2, W1, uout, ulayout, sc, s)) return rc;
       }
       // forward y pass (W1 -> W2 as (3, N, My, Mzp))
-      auto fyin = io(W1, nb * w2s, (long long)N * Mzp, Mzp, -1);
-      auto fyout = io(W2, nb * w1s, (long long)My * Mzp, Mzp, kc);
-      if (int rc = colpass_rows<false, false>(p, KID_YFWD, fyin, StRowsC<T, N, true>{fyout}, Mzp, 3, nb * N, tw, s))
+      auto fyin = io(W1, nb * w2s, (long long)N * Mzp);
+      auto fyout = io(W2, nb * w1s, (long long)My * Mzp);
+      if (int rc = colpass_rows<false, false, RS::YC>(p, KID_YFWD, fyin, StRowsC<T, N, true, RS::YC>{fyout}, Mzp, 3, nb * N, tw, s))
         return rc;
     }
     // forward x pass + k-space update
@@ -346,10 +342,9 @@ template <typename T, int N> struct Ops {
     A.kc = kc; A.My = My; A.Mzp = Mzp; A.status = p->status;
     A.vk = (C*)p->sm_vk; A.tps = T(p->sm_tps); A.vg = T(p->sm_tps * p->sm_g * (double)N * N * N);
     A.blowup = T(100.0 * (double)N * N * N);  // the blow-up threshold of the step epilogue (F:618)
-    // RK2 stages stage their cube rows in shared memory when that keeps 2 CTAs per SM
+    // the cube rows the update reads are staged in shared memory when that keeps 2 CTAs per SM
     const size_t pre_bytes = sizeof(C) * 3 * (size_t)(2 * kc + 1) * TB;
-    constexpr bool RK2 = MODE == UPD_RK2_1 || MODE == UPD_RK2_2;
-    A.prefetch = (RK2 && COL_SMEM + pre_bytes <= 112 * 1024) ? 1 : 0;
+    A.prefetch = COL_SMEM + pre_bytes <= 112 * 1024 ? 1 : 0;
     const size_t smem = COL_SMEM + (A.prefetch ? pre_bytes : 0);
     ProfScope ps(p, KID_XFWD_UPD, s);
     auto k = k_xfwd_update<T, N, MODE>;
