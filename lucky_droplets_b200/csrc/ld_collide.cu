@@ -62,6 +62,7 @@ __global__ void k_cell_keys(const double* __restrict__ pos, long long n, double 
 __global__ void k_cell_count(const double* __restrict__ pos, long long n, double L, double cw, int nc,
                              unsigned* __restrict__ key, unsigned* __restrict__ rank, unsigned* __restrict__ occ,
                              const int* __restrict__ box) {
+  ld::grid_dep();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int cx = cell_of(wrapL(pos[3 * i], L), cw, nc);
     const int cy = cell_of(wrapL(pos[3 * i + 1], L), cw, nc);
@@ -74,6 +75,7 @@ __global__ void k_cell_count(const double* __restrict__ pos, long long n, double
 
 __global__ void k_cell_scatter(const unsigned* __restrict__ key, const unsigned* __restrict__ rank,
                                const int* __restrict__ cs, long long n, unsigned* __restrict__ run) {
+  ld::grid_dep();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     run[cs[key[i]] + rank[i]] = (unsigned)i;
 }
@@ -98,13 +100,14 @@ constexpr int kSmallCell = 64;  // cells up to this occupancy are placed by rank
 // number of the cell's droplets with a smaller index, counted over the run; the sorted index, key
 // and copies are written there.  By slots, the writes (56 bytes a droplet) stay inside the cell and
 // only the droplet's own data are read from scattered addresses: 1e6 droplets in random order 53 ->
-// 33 us against a thread per droplet (already sorted ones 22 -> 20).  Cells above kSmallCell droplets are left to k_cell_big (the
-// thread of the run's first slot appends the cell to `big`).
+// 33 us against a thread per droplet (already sorted ones 22 -> 20).  Cells above kSmallCell droplets
+// are left to k_cell_big (the thread of the run's first slot appends the cell to `big`).
 __global__ void k_cell_place(const unsigned* __restrict__ key, const int* __restrict__ cs,
                              const unsigned* __restrict__ run, long long n, const double* __restrict__ pos,
                              const double* __restrict__ rad, double L, unsigned* __restrict__ sval,
                              unsigned* __restrict__ skey, double4* __restrict__ sp, float4* __restrict__ spf,
                              unsigned* __restrict__ big, unsigned* __restrict__ nbig) {
+  ld::grid_dep();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
     const unsigned i = run[t];
     const unsigned k = key[i];
@@ -128,6 +131,7 @@ __global__ void __launch_bounds__(512)
 k_cell_big(const int* __restrict__ cs, const unsigned* __restrict__ big, const unsigned* __restrict__ nbig,
            unsigned* __restrict__ run, const double* __restrict__ pos, const double* __restrict__ rad, double L,
            unsigned* __restrict__ sval, unsigned* __restrict__ skey, double4* __restrict__ sp, float4* __restrict__ spf) {
+  ld::grid_dep();
   const unsigned nb = *nbig;
   for (unsigned b = blockIdx.x; b < nb; b += gridDim.x) {
     const unsigned k = big[b];
@@ -193,6 +197,7 @@ __device__ __forceinline__ unsigned scan_block_sum(unsigned v, unsigned* w) {
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_scan_totals(const unsigned* __restrict__ a, long long m, unsigned* __restrict__ sums) {
+  ld::grid_dep();
   __shared__ unsigned w[32];
   const long long base = (long long)blockIdx.x * SCAN_TILE;
   unsigned v = 0;
@@ -207,6 +212,7 @@ k_scan_totals(const unsigned* __restrict__ a, long long m, unsigned* __restrict_
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_scan_tiles(unsigned* __restrict__ a, long long m, const unsigned* __restrict__ sums) {
+  ld::grid_dep();
   __shared__ unsigned buf[SCAN_TILE];
   __shared__ unsigned wsum[SCAN_THREADS / 32];
   const long long base = (long long)blockIdx.x * SCAN_TILE;
@@ -425,8 +431,9 @@ __device__ __forceinline__ bool near_f(const float4 a, const float4 b, float L, 
 // The lanes of a warp are neighbours in the sorted order, so their ranges overlap and the
 // candidates come from L1; staging a column's droplets in shared memory, a block per column, left
 // the blocks waiting at their barriers (1e6 droplets in 82^3 cells: 117 us, 82 now; 4.4e5 droplets
-// in 16 boxes of one per cell: 67 us, mostly block set-up, 29 now).  The FP32 pre-test's hits are queued per thread in shared
-// memory and put to the FP64 rule together after the walk, instead of one lane at a time.
+// in 16 boxes of one per cell: 67 us, mostly block set-up, 29 now).  The FP32 pre-test's hits are
+// queued per thread in shared memory and put to the FP64 rule together after the walk, instead of
+// one lane at a time.
 // Each droplet stores its partner count and its first KEEP partners (sorted indices) in scr;
 // k_emit_pairs writes the pairs from the scanned counts, searching again only for droplets with
 // more than KEEP partners.
@@ -546,6 +553,7 @@ __global__ void __launch_bounds__(VISIT_THREADS, VISIT_BLOCKS)
 k_visit(const double4* __restrict__ sp, const float4* __restrict__ spf, const unsigned* __restrict__ skey,
         const int* __restrict__ cs, int nc, double L, double cw, int n, unsigned* __restrict__ cnt,
         int* __restrict__ scr) {
+  ld::grid_dep();
   __shared__ int queue[KEEP][VISIT_THREADS];
   const int tid = threadIdx.x;
   unsigned c = 0;     // partners confirmed (the first KEEP in scr)
@@ -679,6 +687,7 @@ __global__ void __launch_bounds__(EMIT_THREADS)
 k_emit_pairs(const double4* __restrict__ sp, const float4* __restrict__ spf, const unsigned* __restrict__ skey,
              const unsigned* __restrict__ sval, const int* __restrict__ cs, int nc, double L, double cw, int n,
              const unsigned* __restrict__ off, const int* __restrict__ scr, int* __restrict__ pairs, long long cap) {
+  ld::grid_dep();
   __shared__ unsigned wlist[EMIT_THREADS], nwide, wsum[EMIT_THREADS / 32];
   if (threadIdx.x == 0) nwide = 0u;
   __syncthreads();
@@ -729,6 +738,7 @@ k_emit_pairs(const double4* __restrict__ sp, const float4* __restrict__ spf, con
 // box b's droplets are the sorted slots start[b nc^3] .. start[(b + 1) nc^3] - 1).
 __global__ void k_box_counts_sorted(const unsigned* __restrict__ off, const int* __restrict__ start, long long nc3,
                                     int nbox, int64_t* __restrict__ bc) {
+  ld::grid_dep();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nbox; b += gridDim.x * blockDim.x)
     bc[b] = (int64_t)off[start[(b + 1) * nc3]] - (int64_t)off[start[b * nc3]];
 }
@@ -744,6 +754,7 @@ __global__ void k_box_counts_ids(const unsigned* __restrict__ off, const int* __
 
 __global__ void k_finish(const unsigned* __restrict__ off, long long n, long long cap, int64_t* __restrict__ count,
                          unsigned* __restrict__ status) {
+  ld::grid_dep();
   const long long tot = off[n];
   *count = tot;
   if (tot > cap && status) atomicOr(status, LD_STATUS_PAIR_OVERFLOW);
@@ -789,9 +800,8 @@ namespace {
 int scan_u32(ld_collider* c, unsigned* a, long long m, cudaStream_t s) {
   const long long tiles = (m + SCAN_TILE - 1) / SCAN_TILE;
   if (tiles > SCAN_TILE) return ld_fail(LD_ERR_UNSUPPORTED, "scan of %lld elements", m);
-  if (tiles > 1) k_scan_totals<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(a, m, c->sums);
-  k_scan_tiles<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(a, m, c->sums);
-  LD_LAUNCH_CHECK();
+  if (tiles > 1) LD_CUDA_CHECK(launch_dep(true, k_scan_totals, dim3((unsigned)tiles), SCAN_THREADS, 0, s, a, m, c->sums));
+  LD_CUDA_CHECK(launch_dep(true, k_scan_tiles, dim3((unsigned)tiles), SCAN_THREADS, 0, s, a, m, c->sums));
   return LD_OK;
 }
 }  // namespace
@@ -914,24 +924,28 @@ int ld_collide_boxes(ld_collider* c, const double* pos, const double* radius, co
       unsigned* occ = reinterpret_cast<unsigned*>(c->start);
       LD_CUDA_CHECK(cudaMemsetAsync(occ, 0, sizeof(unsigned) * (size_t)(ncell + 1), s));
       LD_CUDA_CHECK(cudaMemsetAsync(c->nbig, 0, sizeof(unsigned), s));
-      k_cell_count<<<gridn(n, 256), 256, 0, s>>>(pos, n, L, cw, nc, c->key2, c->val2, occ, box);
+      LD_CUDA_CHECK(launch_dep(true, k_cell_count, dim3(gridn(n, 256)), 256, 0, s, pos, n, L, cw, nc, c->key2, c->val2,
+                               occ, box));
       if (int rc = scan_u32(c, occ, ncell + 1, s)) return rc;
-      k_cell_scatter<<<gridn(n, 256), 256, 0, s>>>(c->key2, c->val2, c->start, n, c->cnt);
-      k_cell_place<<<gridn(n, 256), 256, 0, s>>>(c->key2, c->start, c->cnt, n, pos, radius, L, c->val, c->key, c->sp,
-                                                 c->spf, c->val2, c->nbig);
-      k_cell_big<<<148, 512, 0, s>>>(c->start, c->val2, c->nbig, c->cnt, pos, radius, L, c->val, c->key, c->sp,
-                                     c->spf);
+      LD_CUDA_CHECK(launch_dep(true, k_cell_scatter, dim3(gridn(n, 256)), 256, 0, s, c->key2, c->val2, c->start, n,
+                               c->cnt));
+      LD_CUDA_CHECK(launch_dep(true, k_cell_place, dim3(gridn(n, 256)), 256, 0, s, c->key2, c->start, c->cnt, n, pos,
+                               radius, L, c->val, c->key, c->sp, c->spf, c->val2, c->nbig));
+      LD_CUDA_CHECK(launch_dep(true, k_cell_big, dim3(kSMs), 512, 0, s, c->start, c->val2, c->nbig, c->cnt, pos, radius,
+                               L, c->val, c->key, c->sp, c->spf));
     }
   }
   ProfScope ps(c->trace, KID_COLL_PAIRS, s);
   if (nc >= 3) {
-    k_visit<<<(unsigned)((n + VISIT_THREADS - 1) / VISIT_THREADS), VISIT_THREADS, 0, s>>>(
-        c->sp, c->spf, c->key, c->start, nc, L, cw, (int)n, c->cnt, c->scr);
+    LD_CUDA_CHECK(launch_dep(true, k_visit, dim3((unsigned)((n + VISIT_THREADS - 1) / VISIT_THREADS)), VISIT_THREADS, 0,
+                             s, c->sp, c->spf, c->key, c->start, nc, L, cw, (int)n, c->cnt, c->scr));
     if (int rc = scan_u32(c, c->cnt, n + 1, s)) return rc;
-    k_emit_pairs<<<(unsigned)((n + EMIT_THREADS - 1) / EMIT_THREADS), EMIT_THREADS, 0, s>>>(
-        c->sp, c->spf, c->key, c->val, c->start, nc, L, cw, (int)n, c->cnt, c->scr, pairs, cap);
+    LD_CUDA_CHECK(launch_dep(true, k_emit_pairs, dim3((unsigned)((n + EMIT_THREADS - 1) / EMIT_THREADS)), EMIT_THREADS,
+                             0, s, c->sp, c->spf, c->key, c->val, c->start, nc, L, cw, (int)n, c->cnt, c->scr, pairs,
+                             cap));
     if (box_counts)
-      k_box_counts_sorted<<<(c->nbox + 255) / 256, 256, 0, s>>>(c->cnt, c->start, nc3, c->nbox, box_counts);
+      LD_CUDA_CHECK(launch_dep(true, k_box_counts_sorted, dim3((c->nbox + 255) / 256), 256, 0, s, c->cnt, c->start, nc3,
+                               c->nbox, box_counts));
   } else {
     LD_CUDA_CHECK(cudaMemsetAsync(c->cnt + n, 0, 4, s));
     const int* end = c->start + 1;  // end of cell k = start of cell k + 1
@@ -942,7 +956,7 @@ int ld_collide_boxes(ld_collider* c, const double* pos, const double* radius, co
                                                    c->cnt, pairs, cap);
     if (box_counts) k_box_counts_ids<<<gridn(n, 256), 256, 0, s>>>(c->cnt, box, n, box_counts);
   }
-  k_finish<<<1, 1, 0, s>>>(c->cnt, n, cap, count, c->status);
+  LD_CUDA_CHECK(launch_dep(true, k_finish, dim3(1), 1, 0, s, c->cnt, n, cap, count, c->status));
   LD_LAUNCH_CHECK();
   return LD_OK;
 }

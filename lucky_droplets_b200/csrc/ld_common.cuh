@@ -40,6 +40,18 @@ template <typename C> __device__ __forceinline__ C czero() { C r; r.x = 0; r.y =
 
 template <typename T> __device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
 
+// Programmatic dependent launch (launch_dep): the next kernel in the stream may be scheduled while
+// this one runs; its threads wait in grid_dep_wait until this grid has completed and its writes are
+// visible.  Both are no-ops for a kernel launched without the attribute.  Kernels call grid_dep_wait
+// before they touch anything that another kernel writes or reads, and grid_dep_launch after it, so
+// that whatever runs before a kernel's own wait runs after its last predecessor but one.
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep() {
+  grid_dep_wait();
+  grid_dep_launch();
+}
+
 }  // namespace ld
 
 #define LD_CUDA_CHECK(expr)                                   \

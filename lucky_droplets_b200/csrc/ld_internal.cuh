@@ -80,6 +80,33 @@ struct ProfScope {
   ~ProfScope() { if (p && p->prof) ld_prof_end(p, s); }
 };
 
+// Kernel launch; early: it may begin while its predecessor in the stream finishes (programmatic
+// dependent launch; the kernel waits in grid_dep_wait), which hides the launch latency and the
+// prologue, two to three microseconds per launch.  That pays for short kernels only: blocks that
+// become resident beside a long predecessor pin the SM's split of L1 and shared memory (a right-hand
+// side at 32^3 FP64 23.6 -> 14.4 us, at 256^3 FP32 396 -> 442; 1e6 inferences 381 -> 612).  Hence:
+// the flow's passes with at most one x plane per SM (four boxes of 64^3: 637 us for five ensemble
+// steps without, 702 with it), per-droplet passes of at most 1024 droplets per SM, inference of at
+// most one tile per SM; the generic transforms and the collision search always (transforms at 96^3
+// FP64 78 -> 66 us, 256^3 FP32 503 -> 491; 1e6 droplets 228 -> 204 us).
+constexpr int kSMs = 148;
+inline bool early_droplets(long long n) { return n <= kSMs * 1024; }
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dep(bool early, void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t s,
+                       Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // Launch sequences of one (precision, N) instance; every pointer is a device pointer.
 struct OpsTable {
   int (*rfft_full)(ld_plan*, const void* u, void* fu, int ncomp, cudaStream_t);

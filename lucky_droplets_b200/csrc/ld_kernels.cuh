@@ -171,11 +171,10 @@ template <typename T, int N> struct LdCurl {
 // One CTA = TB columns x NT threads; blockIdx.x = tile * nf + field (fields of a tile launch
 // together so their shared inputs are served from L2), blockIdx.y = outer index.
 template <typename T, int N, bool INV, class Ld, class St>
-__global__ void __launch_bounds__(Cfg<N>::COL_THREADS)
-k_colfft(Ld ld, St st, int ncols, int nf, const cplx<T>* __restrict__ tw) {
+__device__ __forceinline__ void colfft_tile(const Ld& ld, const St& st, int ncols, int nf, const cplx<T>* __restrict__ tw,
+                                            unsigned char* smem) {
   constexpr int E = Cfg<N>::EC, TB = Cfg<N>::TB, NT = Cfg<N>::NTC;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
+  cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem);
   const int c = threadIdx.x % TB, j = threadIdx.x / TB;
   __builtin_assume(j >= 0 && j < NT);
   const int field = blockIdx.x % nf;
@@ -192,38 +191,112 @@ k_colfft(Ld ld, St st, int ncols, int nf, const cplx<T>* __restrict__ tw) {
   }
 }
 
-// The same tile (the same body, written out so that k_colfft keeps its code) with five CTAs per
-// SM, for N = 256 in FP32: 48 registers, no spills, 32 KB of shared memory each, instead of four
-// CTAs at 56 registers.  These one-shot tiles wait on their loads (the inverse x pass with the
-// curl stalls mostly on long scoreboard) and the extra warps hide that latency (x inverse
-// 0.072 -> 0.067 ms).  Elsewhere k_colfft keeps the compiler's own register choice: stating one
-// CTA per SM would let the FP64 tiles grow from about 90 to about 150 registers.
+template <typename T, int N, bool INV, class Ld, class St>
+__global__ void __launch_bounds__(Cfg<N>::COL_THREADS)
+k_colfft(Ld ld, St st, int ncols, int nf, const cplx<T>* __restrict__ tw) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_dep();
+  colfft_tile<T, N, INV>(ld, st, ncols, nf, tw, smem_raw);
+}
+
+// The same tile with five CTAs per SM, for N = 256 in FP32: 48 registers, no spills, 32 KB of shared
+// memory each, instead of four CTAs at 56 registers.  These one-shot tiles wait on their loads and
+// the extra warps hide that latency (x inverse 0.072 -> 0.067 ms).  Elsewhere k_colfft keeps the
+// compiler's own register choice: stating one CTA per SM would let the FP64 tiles grow from about
+// 90 to about 150 registers.
 template <typename T, int N, bool INV, class Ld, class St>
 __global__ void __launch_bounds__(Cfg<N>::COL_THREADS, 5)
 k_colfft5(Ld ld, St st, int ncols, int nf, const cplx<T>* __restrict__ tw) {
-  constexpr int E = Cfg<N>::EC, TB = Cfg<N>::TB, NT = Cfg<N>::NTC;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
-  const int c = threadIdx.x % TB, j = threadIdx.x / TB;
-  __builtin_assume(j >= 0 && j < NT);
-  const int field = blockIdx.x % nf;
-  const int col = (blockIdx.x / nf) * TB + c;
-  const bool ok = col < ncols;
-  const int outer = blockIdx.y;
-  cplx<T> a[E];
-#pragma unroll
-  for (int m = 0; m < E; ++m) a[m] = ok ? ld(field, outer, j + NT * m, col) : czero<cplx<T>>();
-  fft_run<T, N, E, INV, false>(a, sbuf + c, TB, j, tw, SyncBlock());
-  if (ok) {
-#pragma unroll
-    for (int m = 0; m < E; ++m) st(field, outer, j + NT * m, col, a[m]);
-  }
+  grid_dep();
+  colfft_tile<T, N, INV>(ld, st, ncols, nf, tw, smem_raw);
 }
 
 template <typename T, int N, bool INV, class Ld, class St>
 constexpr auto colfft_kernel() {
   if constexpr (N == 256 && sizeof(T) == 4) return k_colfft5<T, N, INV, Ld, St>;
   else return k_colfft<T, N, INV, Ld, St>;
+}
+
+// Sum of 0.5 |u|^2 normalize over the modes listed for shell s (CSR of cube indices), by the block
+// in a fixed order (FP64, deterministic); as_factor: the constant-power factor f0 / (2 E_s) of
+// F:250-254 instead of E_s.  red: 32 doubles of shared memory.
+template <typename T> struct ShellArgs {
+  const cplx<T>* u;
+  long long cs, ubs;  // component stride, box stride of u
+  const int *off, *idx;
+  int Mzp, shell0, nshell;
+  double norm0, f0;
+  int as_factor, obs;  // box stride of out
+  double* out;
+};
+template <typename T> __device__ __forceinline__ void shell_sum(const ShellArgs<T>& A, int s, int box, double* red) {
+  const cplx<T>* u = A.u + box * A.ubs;
+  const int nthr = (int)blockDim.x & ~31;  // whole warps
+  if ((int)threadIdx.x >= nthr) {
+    __syncthreads();
+    return;
+  }
+  double acc = 0.0;
+  for (int t = A.off[s] + threadIdx.x; t < A.off[s + 1]; t += nthr) {
+    const int e = A.idx[t];
+    const double w = (e % A.Mzp) ? 2.0 : 1.0;  // Hermitian weight of F:136 (kz < N/2 here)
+    double m = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      cplx<T> v = u[c * A.cs + e];
+      m += double(v.x) * double(v.x) + double(v.y) * double(v.y);
+    }
+    acc += 0.5 * m * w * A.norm0;
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, d);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double e = red[0];
+    for (int w = 1; w < nthr / 32; ++w) e += red[w];
+    if (A.as_factor) {
+      if (fabs(e) < 1e-10) e = INFINITY;  // F:250
+      e = A.f0 / (2.0 * e);
+    }
+    A.out[box * A.obs + s] = e;
+  }
+}
+
+template <typename T> __global__ void k_shell_sum(ShellArgs<T> A) {
+  __shared__ double red[32];
+  grid_dep();
+  shell_sum(A, A.shell0 + (int)blockIdx.x, (int)blockIdx.y, red);
+}
+
+// The inverse x pass of the right-hand side (curl on load); the blocks past its tiles compute the
+// forcing factors of the stage input, one shell each, which the update pass reads (a launch of its
+// own cost 3.3 us, of 31 us for a right-hand side at 32^3).
+template <typename T, int N, class St>
+__device__ __forceinline__ void xinv_block(const LdCurl<T, N>& ld, const St& st, int ncols, const cplx<T>* __restrict__ tw,
+                                           const ShellArgs<T>& F, unsigned char* smem) {
+  const int tiles = 6 * ((ncols + Cfg<N>::TB - 1) / Cfg<N>::TB);
+  if ((int)blockIdx.x < tiles) colfft_tile<T, N, true>(ld, st, ncols, 6, tw, smem);
+  else shell_sum(F, F.shell0 + (int)blockIdx.x - tiles, (int)blockIdx.y, reinterpret_cast<double*>(smem));
+}
+template <typename T, int N, class St>
+__global__ void __launch_bounds__(Cfg<N>::COL_THREADS)
+k_xinv(LdCurl<T, N> ld, St st, int ncols, const cplx<T>* __restrict__ tw, ShellArgs<T> F) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_dep();
+  xinv_block<T, N>(ld, st, ncols, tw, F, smem_raw);
+}
+template <typename T, int N, class St>
+__global__ void __launch_bounds__(Cfg<N>::COL_THREADS, 5)
+k_xinv5(LdCurl<T, N> ld, St st, int ncols, const cplx<T>* __restrict__ tw, ShellArgs<T> F) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_dep();
+  xinv_block<T, N>(ld, st, ncols, tw, F, smem_raw);
+}
+template <typename T, int N, class St> constexpr auto xinv_kernel() {
+  if constexpr (N == 256 && sizeof(T) == 4) return k_xinv5<T, N, St>;
+  else return k_xinv<T, N, St>;
 }
 
 // Pipelined column pass over plain strided rows: a CTA loops over items (column block, field,
@@ -277,6 +350,7 @@ k_colfft_pipe(RowsIO<T> in, St st, int ncols, int nf, int nouter, const cplx<T>*
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  grid_dep();
   unsigned it = blockIdx.x;
   Item cur_item = split(it);
   if (it < nitems) prefetch(cur_item, buf0);
@@ -382,6 +456,7 @@ __global__ void __launch_bounds__(Cfg<N>::COL_THREADS, (N == 256 && sizeof(T) ==
 k_xfwd_update(UpdArgs<T> A, int ncols, const cplx<T>* __restrict__ tw) {
   constexpr int E = Cfg<N>::EC, TB = Cfg<N>::TB, NT = Cfg<N>::NTC;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_dep();
   if (blockIdx.y) {  // box of a multi-box plan
     const long long bo = blockIdx.y;
     A.nl += bo * A.nl_bs;
@@ -657,6 +732,7 @@ k_z_c2r(const cplx<T>* __restrict__ X, T* __restrict__ x, long long nrows, int s
         long long xfs, long long Xfs, const cplx<T>* __restrict__ tw) {
   using Z = ZCfg<T, N>;
   constexpr int E = Z::E1, NT = N / E;
+  grid_dep();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
   int unit, j;
@@ -690,6 +766,7 @@ k_z_r2c(const T* __restrict__ x, cplx<T>* __restrict__ X, long long nrows, int s
         int Kval, long long xfs, long long Xfs, const cplx<T>* __restrict__ tw) {
   using Z = ZCfg<T, N>;
   constexpr int E = Z::E1, NT = N / E;
+  grid_dep();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* sbuf = reinterpret_cast<cplx<T>*>(smem_raw);
   int unit, j;
@@ -812,6 +889,7 @@ k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __rest
     twr.p = tws + j;
     __syncthreads();
   }
+  grid_dep();
   __syncwarp();
   auto issue = [&](long long r, int q) {  // fields 2 q, 2 q + 1 of rows r .. r + R - 1
     if (lane == 0) {
@@ -911,6 +989,7 @@ k_plane(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __restrict__ 
   const long long o = blockIdx.x;
   for (int i = tid; i < N; i += THREADS) twy[i] = tw[i];
   TwLane<T, N, E>::fill(twz, tw, tid, THREADS);
+  grid_dep();
   __syncthreads();
   // y inverse, first step: cube rows from global memory
   for (int t = tid; t < C::NC * R2; t += THREADS) {
@@ -1037,47 +1116,6 @@ __global__ void k_from_cube(const cplx<T>* __restrict__ cube, cplx<T>* __restric
   }
 }
 
-// Shell sums of 0.5 |u|^2 normalize over the modes listed for each shell (CSR of cube indices);
-// one CTA per shell, fixed-order FP64 reduction (deterministic).  With `factor` != nullptr the
-// block writes the constant-power factor f0 / (2 E_s) of F:250-254 instead of E_s.
-template <typename T>
-__global__ void k_shell_sum(const cplx<T>* __restrict__ u, long long cs, const int* __restrict__ off,
-                            const int* __restrict__ idx, int Mzp, int shell0,
-                            double norm0, double* __restrict__ out, double f0, int as_factor, long long ubs = 0,
-                            int obs = 0) {
-  __shared__ double red[256];
-  u += blockIdx.y * ubs;  // box of a multi-box plan
-  out += blockIdx.y * obs;
-  const int s = shell0 + blockIdx.x;
-  double acc = 0.0;
-  for (int t = off[s] + threadIdx.x; t < off[s + 1]; t += blockDim.x) {
-    const int e = idx[t];
-    const double w = (e % Mzp) ? 2.0 : 1.0;  // Hermitian weight of F:136 (kz < N/2 here)
-    double m = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      cplx<T> v = u[c * cs + e];
-      m += double(v.x) * double(v.x) + double(v.y) * double(v.y);
-    }
-    acc += 0.5 * m * w * norm0;
-  }
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double e = red[0];
-    if (as_factor) {
-      if (fabs(e) < 1e-10) e = INFINITY;  // F:250
-      out[s] = f0 / (2.0 * e);
-    } else {
-      out[s] = e;
-    }
-  }
-}
-
 // End-of-step epilogue (F:596-620) on the cube: symmetrise kz = 0 (the irfft->rfft round trip),
 // div-free projection, NaN and blow-up tests.  One thread per (kx, ky, kz) column element; the
 // kz = 0 pair (k, -k) is handled by the lexicographically smaller member.
@@ -1156,6 +1194,7 @@ __global__ void k_epilogue(cplx<T>* __restrict__ u, long long cs, int kc, int My
 template <typename T>
 __global__ void k_epilogue_plane0(cplx<T>* __restrict__ u, long long cs, int kc, int My, int Mzp, T blowup,
                                   unsigned* status) {
+  grid_dep();
   u += blockIdx.y * 3 * cs;  // box of a multi-box plan
   const long long total = (long long)My * My;
   unsigned flags = 0;
@@ -1366,6 +1405,7 @@ template <typename T, int METHOD, int STAGE>
 __global__ void k_droplet_stage(const vec4<T>* __restrict__ u0, int N, double L, double* __restrict__ pos,
                                 T* __restrict__ vel, const T* __restrict__ tau, T* __restrict__ a1,
                                 long long n, double h, T g, const int* __restrict__ box = nullptr) {
+  grid_dep();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     // the droplet's box of a multi-box plan: its field is box (N, N, N, 4) further on
     const vec4<T>* u = box ? u0 + (long long)box[i] * N * N * N : u0;

@@ -456,6 +456,7 @@ k_mlp_features(const vec4<T>* __restrict__ u4, int N, double L, const double* __
   const int r = lane < 3 * FDROP ? lane / 3 : FDROP - 1;
   const int c = lane < 3 * FDROP ? lane - 3 * r : 0;
   __shared__ __align__(16) float2 fs2[32];  // feature scales as pairs (fs[i], fs[i + 32]), warp-uniform reads
+  grid_dep();
   if (threadIdx.x < 32) fs2[threadIdx.x] = make_float2(params[OFF_FS + threadIdx.x], params[OFF_FS + 32 + threadIdx.x]);
   __syncthreads();
   const float mode = params[OFF_OS + 1];
@@ -620,6 +621,8 @@ k_mlp_forward_tc(const unsigned char* __restrict__ Xg, const float* __restrict__
   unsigned* cnt = reinterpret_cast<unsigned*>(sm + SM_CNT);  // [x_issued 2][x_waited 2][mma_commit 2][mma_wait 2]
   // b1, b2 halved: the epilogues form h = z / 2 = fma(0.5, acc, b / 2), which is exactly
   // 0.5 * (acc + b) (halving is exact), and SiLU(z) = h + h tanh(h); b3 as is
+  // (weights and biases load before the wait for the feature kernel, which does not write them; it
+  // triggers this launch after its own wait, so an update of the weights before it is complete)
   for (int e = tid; e < 2 * H + N3P; e += FT_THREADS)
     bias[e] = e < H ? 0.5f * params[OFF_B1 + e]
                     : (e < 2 * H ? 0.5f * params[OFF_B2 + e - H] : (e - 2 * H < N3 ? params[OFF_B3 + e - 2 * H] : 0.f));
@@ -639,6 +642,7 @@ k_mlp_forward_tc(const unsigned char* __restrict__ Xg, const float* __restrict__
     bulk_g2s(sm + SM_W1, packed + P_TW1, H * K1 * 2, bar_w);
     bulk_g2s(sm + SM_W2, packed + P_TW2, H * H * 2, bar_w);
     bulk_g2s(sm + SM_W3, packed + P_TW3, N3P * H * 2, bar_w);
+    grid_dep_wait();
     if (mine > 0) {  // the first copy is counted at the end (x_issued[0] + 1)
       mbar_expect_tx(&bar_x[0], TILE_X_BYTES);
       bulk_g2s(sm + SM_X, Xg + blockIdx.x * (long long)TILE_X_BYTES, TILE_X_BYTES, &bar_x[0]);
@@ -649,6 +653,7 @@ k_mlp_forward_tc(const unsigned char* __restrict__ Xg, const float* __restrict__
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
+  grid_dep();
   tc_fence_before();
   __syncthreads();  // the barriers are initialised
   tc_fence_after();
@@ -953,12 +958,6 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-
-// Programmatic dependent launch: the next kernel in the stream may start (its CTAs wait in
-// grid_dep_wait until this grid has completed and its writes are visible); both are no-ops for a
-// kernel launched without the attribute.
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // 16-byte asynchronous copy global -> shared; bytes < 16 zero-fills the rest (0: no read)
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, unsigned bytes) {
@@ -1384,6 +1383,7 @@ __global__ void k_mlp_reduce_adam(const float* __restrict__ gpart, const float* 
 template <typename T>
 __global__ void k_droplet_given(int stage, const T* __restrict__ up, double* __restrict__ pos, T* __restrict__ vel,
                                 const T* __restrict__ tau, T* __restrict__ a1, long long n, double h, T g) {
+  grid_dep();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const T vx = vel[3 * i], vy = vel[3 * i + 1], vz = vel[3 * i + 2];
     const T it = T(1) / tau[i];
@@ -1410,6 +1410,7 @@ __global__ void k_droplet_given(int stage, const T* __restrict__ up, double* __r
 template <typename T>
 __global__ void k_droplet_predict(const double* __restrict__ pos, const T* __restrict__ vel, long long n, double h,
                                   double* __restrict__ xs) {
+  grid_dep();
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < 3 * n; e += (long long)gridDim.x * blockDim.x)
     xs[e] = pos[e] + h * double(vel[e]);
 }
@@ -1419,21 +1420,6 @@ template <typename T>
 __global__ void k_interleave3(const T* __restrict__ in, vec4<T>* __restrict__ out, long long m) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < m; i += (long long)gridDim.x * blockDim.x)
     out[i] = mk4<T>(in[i], in[m + i], in[2 * m + i], T(0));
-}
-
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 inline int gridn(long long n, int th) {
@@ -1502,25 +1488,25 @@ int ld_mlp_infer_ws(ld_plan* p, const void* u4, const double* pos, int64_t n, co
                                          (int)SMEM_FWD));
       {
         ProfScope ps(p, KID_MLP_FEAT, s);
-        k_mlp_features<float><<<(unsigned)gf, FTHREADS, 0, s>>>((const float4*)u4, p->N, L,
-                                                                          pos + 3 * b0, nb, params, (bf16*)X, aux);
+        LD_CUDA_CHECK(launch_dep(tiles <= kSMs, k_mlp_features<float>, dim3((unsigned)gf), FTHREADS, 0, s, (const float4*)u4, p->N, L,
+                                 pos + 3 * b0, nb, params, (bf16*)X, aux));
       }
       ProfScope ps(p, KID_MLP_INFER, s);
-      k_mlp_forward_tc<float><<<(unsigned)gm, FT_THREADS, SMEM_FWD, s>>>(X, aux, nb, (const bf16*)packed, params,
-                                                                        (float*)out + 3 * b0, p->status,
-                                                                        p->wait_limit, p->wait_stall);
+      LD_CUDA_CHECK(launch_dep(tiles <= kSMs, k_mlp_forward_tc<float>, dim3((unsigned)gm), FT_THREADS, SMEM_FWD, s, X, aux, nb,
+                               (const bf16*)packed, params, (float*)out + 3 * b0, p->status, p->wait_limit,
+                               p->wait_stall));
     } else {
       LD_CUDA_CHECK(cudaFuncSetAttribute(k_mlp_forward_tc<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)SMEM_FWD));
       {
         ProfScope ps(p, KID_MLP_FEAT, s);
-        k_mlp_features<double><<<(unsigned)gf, FTHREADS, 0, s>>>((const double4*)u4, p->N, L,
-                                                                            pos + 3 * b0, nb, params, (bf16*)X, aux);
+        LD_CUDA_CHECK(launch_dep(tiles <= kSMs, k_mlp_features<double>, dim3((unsigned)gf), FTHREADS, 0, s, (const double4*)u4, p->N, L,
+                                 pos + 3 * b0, nb, params, (bf16*)X, aux));
       }
       ProfScope ps(p, KID_MLP_INFER, s);
-      k_mlp_forward_tc<double><<<(unsigned)gm, FT_THREADS, SMEM_FWD, s>>>(X, aux, nb, (const bf16*)packed,
-                                                                         params, (double*)out + 3 * b0, p->status,
-                                                                         p->wait_limit, p->wait_stall);
+      LD_CUDA_CHECK(launch_dep(tiles <= kSMs, k_mlp_forward_tc<double>, dim3((unsigned)gm), FT_THREADS, SMEM_FWD, s, X, aux, nb,
+                               (const bf16*)packed, params, (double*)out + 3 * b0, p->status, p->wait_limit,
+                               p->wait_stall));
     }
     LD_LAUNCH_CHECK();
   }
@@ -1599,8 +1585,8 @@ int ld_droplet_predict(ld_plan* p, const double* pos, const void* vel, int64_t n
   if (!p || n < 0 || (n > 0 && (!pos || !vel || !xs))) return ld_fail(LD_ERR_ARG, "ld_droplet_predict: bad arguments");
   if (n == 0) return LD_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  if (p->prec == LD_F32) k_droplet_predict<float><<<gridn(3 * n, 256), 256, 0, s>>>(pos, (const float*)vel, n, h, xs);
-  else k_droplet_predict<double><<<gridn(3 * n, 256), 256, 0, s>>>(pos, (const double*)vel, n, h, xs);
+  if (p->prec == LD_F32) LD_CUDA_CHECK(launch_dep(early_droplets(n), k_droplet_predict<float>, dim3(gridn(3 * n, 256)), 256, 0, s, pos, (const float*)vel, n, h, xs));
+  else LD_CUDA_CHECK(launch_dep(early_droplets(n), k_droplet_predict<double>, dim3(gridn(3 * n, 256)), 256, 0, s, pos, (const double*)vel, n, h, xs));
   LD_LAUNCH_CHECK();
   return LD_OK;
 }
@@ -1613,11 +1599,11 @@ int ld_droplet_update(ld_plan* p, int stage, const void* up, double* pos, void* 
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope ps(p, stage == 1 ? KID_DROPLET1 : KID_DROPLET2, s);
   if (p->prec == LD_F32)
-    k_droplet_given<float><<<gridn(n, 256), 256, 0, s>>>(stage, (const float*)up, pos, (float*)vel, (const float*)tau,
-                                                         (float*)a1, n, h, (float)g);
+    LD_CUDA_CHECK(launch_dep(early_droplets(n), k_droplet_given<float>, dim3(gridn(n, 256)), 256, 0, s, stage, (const float*)up, pos, (float*)vel,
+                             (const float*)tau, (float*)a1, n, h, (float)g));
   else
-    k_droplet_given<double><<<gridn(n, 256), 256, 0, s>>>(stage, (const double*)up, pos, (double*)vel,
-                                                          (const double*)tau, (double*)a1, n, h, g);
+    LD_CUDA_CHECK(launch_dep(early_droplets(n), k_droplet_given<double>, dim3(gridn(n, 256)), 256, 0, s, stage, (const double*)up, pos, (double*)vel,
+                             (const double*)tau, (double*)a1, n, h, (double)g));
   LD_LAUNCH_CHECK();
   return LD_OK;
 }
@@ -1659,10 +1645,10 @@ int ld_mlp_train_epoch(const void* X, const float* T, const float* W, const uint
     const double lrk = lr_final > 0.0 ? lr * pow(lr_final / lr, (double)(k < total ? k : total) / (double)total) : lr;
     const float c1 = 1.f - powf(b1, (float)k), c2 = 1.f - powf(b2, (float)k);
     // each launch may begin while the previous one finishes (programmatic dependent launch)
-    LD_CUDA_CHECK(launch_pdl(k_mlp_train_tc, nblk, TR_THREADS, SMEM_TRAIN_TC, s, (const bf16*)X, T, W,
+    LD_CUDA_CHECK(launch_dep(true, k_mlp_train_tc, dim3(nblk), TR_THREADS, SMEM_TRAIN_TC, s, (const bf16*)X, T, W,
                              order + b * batch, (long long)batch, inv_norm, (const bf16*)packed, params, gpart,
                              lpart));
-    LD_CUDA_CHECK(launch_pdl(k_mlp_reduce_adam, gridn(OFF_FS, 256), 256, 0, s, (const float*)gpart,
+    LD_CUDA_CHECK(launch_dep(true, k_mlp_reduce_adam, dim3(gridn(OFF_FS, 256)), 256, 0, s, (const float*)gpart,
                              (const float*)lpart, nblk, inv_norm, params, m, v, (bf16*)packed, (float)lrk, b1, b2,
                              1e-8f, c1, c2, loss_acc));
   }

@@ -38,14 +38,16 @@ template <typename T, int N> struct Ops {
   using Z = ZCfg<T, N>;
   static constexpr size_t Z_SMEM = sizeof(C) * Z::UNITS1 * Z::ZBUF1;
 
+  // whether the flow's passes may begin early: at most one x plane per SM (launch_dep)
+  static bool early(const ld_plan* p) { return (long long)N * p->nbox <= kSMs; }
+
   template <bool INV, class Ld, class St>
   static int colpass(ld_plan* p, int kid, Ld ld, St st, int ncols, int nf, int nouter, const C* tw, cudaStream_t s) {
     ProfScope ps(p, kid, s);
     auto k = colfft_kernel<T, N, INV, Ld, St>();
     if (int rc = set_smem(k, COL_SMEM)) return rc;
     dim3 grid((unsigned)(cdiv(ncols, TB) * nf), (unsigned)nouter);
-    k<<<grid, Cfg<N>::COL_THREADS, COL_SMEM, s>>>(ld, st, ncols, nf, tw);
-    LD_LAUNCH_CHECK();
+    LD_CUDA_CHECK(launch_dep(true, k, grid, Cfg<N>::COL_THREADS, COL_SMEM, s, ld, st, ncols, nf, tw));
     return LD_OK;
   }
 
@@ -75,8 +77,8 @@ template <typename T, int N> struct Ops {
       const long long items = cdiv(ncols, TB) * (long long)nf * nouter;
       const int per_sm = choice > 0 && choice < occ ? choice : occ;
       const long long grid = items < (long long)sms * per_sm ? items : (long long)sms * per_sm;
-      k<<<(unsigned)grid, Cfg<N>::COL_THREADS, 2 * COL_SMEM, s>>>(in, st, ncols, nf, nouter, tw);
-      LD_LAUNCH_CHECK();
+      LD_CUDA_CHECK(launch_dep(early(p), k, dim3((unsigned)grid), Cfg<N>::COL_THREADS, 2 * COL_SMEM, s, in, st, ncols,
+                               nf, nouter, tw));
       return LD_OK;
     }
   }
@@ -90,8 +92,7 @@ template <typename T, int N> struct Ops {
     auto k = k_z_c2r<T, N>;
     if (int rc = set_smem(k, Z_SMEM)) return rc;
     dim3 grid((unsigned)cdiv(nrows / 2, Z::UNITS1), (unsigned)nf);
-    k<<<grid, Z::THREADS1, Z_SMEM, s>>>(X, x, nrows, ss, Kin, sc, xfs, Xfs, tw);
-    LD_LAUNCH_CHECK();
+    LD_CUDA_CHECK(launch_dep(true, k, grid, Z::THREADS1, Z_SMEM, s, X, x, nrows, ss, Kin, sc, xfs, Xfs, tw));
     return LD_OK;
   }
 
@@ -101,8 +102,7 @@ template <typename T, int N> struct Ops {
     auto k = k_z_r2c<T, N>;
     if (int rc = set_smem(k, Z_SMEM)) return rc;
     dim3 grid((unsigned)cdiv(nrows / 2, Z::UNITS1), (unsigned)nf);
-    k<<<grid, Z::THREADS1, Z_SMEM, s>>>(x, X, nrows, ss, Kout, Kval, xfs, Xfs, tw);
-    LD_LAUNCH_CHECK();
+    LD_CUDA_CHECK(launch_dep(true, k, grid, Z::THREADS1, Z_SMEM, s, x, X, nrows, ss, Kout, Kval, xfs, Xfs, tw));
     return LD_OK;
   }
 
@@ -184,16 +184,17 @@ template <typename T, int N> struct Ops {
     return LD_OK;
   }
 
-  // ---- forcing factor for the stage input -----------------------------------------------------
-  static int forcing_factor(ld_plan* p, const C* y, const ld_flow_params* prm, cudaStream_t s) {
-    if (prm->kf_hi < prm->kf_lo || prm->f0 == 0.0) return LD_OK;
-    ProfScope ps(p, KID_FORCING, s);
-    const double norm0 = std::pow(2.0 * M_PI, 3) / std::pow((double)N, 6);
-    dim3 grid((unsigned)(prm->kf_hi - prm->kf_lo + 1), (unsigned)p->nbox);
-    k_shell_sum<T><<<grid, 256, 0, s>>>(y, p->cube_elems(), p->shell_off, p->shell_idx, p->Mzp, prm->kf_lo, norm0,
-                                        p->factor, prm->f0, 1, 3 * p->cube_elems(), p->Nf);
-    LD_LAUNCH_CHECK();
-    return LD_OK;
+  // ---- forcing factors of the stage input y: shells kf_lo..kf_hi (none when nshell = 0) ------------
+  static ShellArgs<T> forcing(ld_plan* p, const C* y, const ld_flow_params* prm) {
+    ShellArgs<T> F;
+    F.u = y; F.cs = p->cube_elems(); F.ubs = 3 * p->cube_elems();
+    F.off = p->shell_off; F.idx = p->shell_idx; F.Mzp = p->Mzp;
+    F.shell0 = prm->kf_lo;
+    F.nshell = prm->kf_hi < prm->kf_lo || prm->f0 == 0.0 ? 0 : prm->kf_hi - prm->kf_lo + 1;
+    F.norm0 = std::pow(2.0 * M_PI, 3) / std::pow((double)N, 6);
+    F.f0 = prm->f0; F.as_factor = 1;
+    F.out = p->factor; F.obs = p->Nf;
+    return F;
   }
 
   // The integrating-factor table exp(-nu h k^2) for the current nu h, built on the stream when
@@ -230,9 +231,8 @@ template <typename T, int N> struct Ops {
     long long grid = (long long)sms * blocks_per_sm;
     const long long need = cdiv(NR, (long long)ZP::WARPS * Z::R);
     if (grid > need) grid = need;
-    k<<<(unsigned)grid, ZP::WARPS * 32, ZP::SMEM, s>>>(W2, W1, uout, ulayout, sc, (const C*)p->tw, p->status,
-                                                       p->wait_limit, p->wait_stall, NR);
-    LD_LAUNCH_CHECK();
+    LD_CUDA_CHECK(launch_dep(early(p), k, dim3((unsigned)grid), ZP::WARPS * 32, ZP::SMEM, s, W2, W1, uout, ulayout, sc,
+                             (const C*)p->tw, p->status, p->wait_limit, p->wait_stall, NR));
     return LD_OK;
   }
 
@@ -299,11 +299,18 @@ template <typename T, int N> struct Ops {
     // the box index next to x (fields (f, box, x, ...)), so that (box, x) is one outer index
     const int nb = p->nbox;
     if (nb > 1 && p->sm_vk) return ld_fail(LD_ERR_UNSUPPORTED, "slow-manifold output of a multi-box plan");
-    if (int rc = forcing_factor(p, y, prm, s)) return rc;
-    // inverse x pass with the curl: 6 fields [u, w]
+    // inverse x pass with the curl, 6 fields [u, w], and the forcing factors
     LdCurl<T, N> lc{y, cs, 3 * cs};
     auto xout = io(W1, nb * w1s, w1s);
-    if (int rc = colpass<true>(p, KID_XINV, lc, StRowsC<T, N, false, RS::XC>{xout}, My * Mzp, 6, nb, tw, s)) return rc;
+    {
+      ProfScope ps(p, KID_XINV, s);
+      using St = StRowsC<T, N, false, RS::XC>;
+      const ShellArgs<T> F = forcing(p, y, prm);
+      auto k = xinv_kernel<T, N, St>();
+      if (int rc = set_smem(k, COL_SMEM)) return rc;
+      const dim3 grid((unsigned)(cdiv(My * Mzp, TB) * 6 + F.nshell), (unsigned)nb);
+      LD_CUDA_CHECK(launch_dep(early(p), k, grid, Cfg<N>::COL_THREADS, COL_SMEM, s, lc, St{xout}, My * Mzp, tw, F));
+    }
     const T sc = T(1.0 / (double(N) * N * N));
     const int ulayout = (MODE == UPD_RHS) ? 0 : 1;  // the time steppers feed droplets: interleaved
     if constexpr (PlaneCfg<T, N>::OK) {
@@ -312,8 +319,8 @@ template <typename T, int N> struct Ops {
       ProfScope ps(p, KID_ZCROSS, s);
       auto k = k_plane<T, N>;
       if (int rc = set_smem(k, PC::SMEM)) return rc;
-      k<<<(unsigned)(nb * N), PC::THREADS, PC::SMEM, s>>>(W1, W2, uout, ulayout, sc, tw, (long long)nb * N);
-      LD_LAUNCH_CHECK();
+      LD_CUDA_CHECK(launch_dep(early(p), k, dim3((unsigned)(nb * N)), PC::THREADS, PC::SMEM, s, W1, W2, uout, ulayout, sc, tw,
+                               (long long)nb * N));
     } else {
       // inverse y pass
       auto yin = io(W1, nb * w1s, (long long)My * Mzp);
@@ -350,8 +357,7 @@ template <typename T, int N> struct Ops {
     auto k = k_xfwd_update<T, N, MODE>;
     if (int rc = set_smem(k, smem)) return rc;
     dim3 ugrid((unsigned)cdiv((long long)My * Mzp, TB), (unsigned)nb);
-    k<<<ugrid, Cfg<N>::COL_THREADS, smem, s>>>(A, My * Mzp, tw);
-    LD_LAUNCH_CHECK();
+    LD_CUDA_CHECK(launch_dep(early(p), k, ugrid, Cfg<N>::COL_THREADS, smem, s, A, My * Mzp, tw));
     return LD_OK;
   }
 
@@ -376,9 +382,8 @@ template <typename T, int N> struct Ops {
     const int gr = grid1d(n, th);
     const double L = 2.0 * M_PI;
     const vec4<T>* u4 = reinterpret_cast<const vec4<T>*>(u);
-    if (stage == 1) k_droplet_stage<T, M, 1><<<gr, th, 0, s>>>(u4, N, L, pos, vel, tau, a1, n, h, T(g), box);
-    else k_droplet_stage<T, M, 2><<<gr, th, 0, s>>>(u4, N, L, pos, vel, tau, a1, n, h, T(g), box);
-    LD_LAUNCH_CHECK();
+    auto k = stage == 1 ? k_droplet_stage<T, M, 1> : k_droplet_stage<T, M, 2>;
+    LD_CUDA_CHECK(launch_dep(early_droplets(n), k, dim3(gr), th, 0, s, u4, N, L, pos, vel, tau, a1, n, h, T(g), box));
     return LD_OK;
   }
 
@@ -425,10 +430,14 @@ template <typename T, int N> struct Table {
   }
   static int shell_spectrum(ld_plan* p, const void* uk, double* ek, cudaStream_t s) {
     ProfScope ps(p, KID_SHELL, s);
-    const double norm0 = std::pow(2.0 * M_PI, 3) / std::pow((double)N, 6);
-    ld::k_shell_sum<T><<<p->Nf, 256, 0, s>>>((const C*)uk, p->cube_elems(), p->shell_off, p->shell_idx, p->Mzp, 0,
-                                             norm0, ek, 0.0, 0);
-    LD_LAUNCH_CHECK();
+    ld::ShellArgs<T> A;
+    A.u = (const C*)uk; A.cs = p->cube_elems(); A.ubs = 0;
+    A.off = p->shell_off; A.idx = p->shell_idx; A.Mzp = p->Mzp;
+    A.shell0 = 0; A.nshell = p->Nf;
+    A.norm0 = std::pow(2.0 * M_PI, 3) / std::pow((double)N, 6);
+    A.f0 = 0.0; A.as_factor = 0;
+    A.out = ek; A.obs = 0;
+    LD_CUDA_CHECK(launch_dep(true, ld::k_shell_sum<T>, dim3((unsigned)p->Nf), 256, 0, s, A));
     return LD_OK;
   }
   static int autotune(ld_plan* p, cudaStream_t s, double* ms) { return O::autotune(p, s, ms); }
@@ -464,8 +473,8 @@ template <typename T, int N> struct Table {
     const double blow = 100.0 * (double)N * N * N;
     const long long plane = (long long)p->My * p->My;
     dim3 grid((unsigned)grid1d(plane, 256), (unsigned)p->nbox);
-    ld::k_epilogue_plane0<T><<<grid, 256, 0, s>>>((C*)uk, p->cube_elems(), p->kc, p->My, p->Mzp, T(blow), p->status);
-    LD_LAUNCH_CHECK();
+    LD_CUDA_CHECK(launch_dep(O::early(p), ld::k_epilogue_plane0<T>, grid, 256, 0, s, (C*)uk, p->cube_elems(), p->kc, p->My, p->Mzp,
+                             T(blow), p->status));
     return LD_OK;
   }
 
