@@ -415,4 +415,164 @@ __device__ __forceinline__ void fft_run(cplx<T>* a, cplx<T>* sbuf, int sstride, 
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// two FP32 transforms of one length side by side, on packed FP32 pairs
+// ------------------------------------------------------------------------------------------
+// Element n of both transforms: x = (re0, re1), y = (im0, im1).  Every operation is one packed
+// instruction for both (add, multiply, fused multiply-add, each half rounding as the scalar one;
+// differences as fma(b, -1, a)), which halves the instructions of the row passes: they issue on two
+// thirds of their cycles and their transforms are two thirds of what they issue.
+struct C2 {
+  float2 x, y;
+};
+__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
+
+// Butterfly u +- v W_16^m of both transforms.
+template <bool INV> __device__ __forceinline__ void butterfly2(C2& p, C2& q, int m) {
+  constexpr float c1 = 0.92387953251128675613f;  // cos(pi/8)
+  constexpr float s1 = 0.38268343236508977173f;  // sin(pi/8)
+  constexpr float c2 = 0.70710678118654752440f;  // cos(pi/4)
+  const C2 u = p, v = q;
+  if (m == 0) {
+    p.x = __fadd2_rn(u.x, v.x);
+    p.y = __fadd2_rn(u.y, v.y);
+    q.x = sub2(u.x, v.x);
+    q.y = sub2(u.y, v.y);
+  } else if (m == 4) {  // v -> -i v (forward), i v (inverse)
+    const float2 ax = __fadd2_rn(u.x, v.y), sx = sub2(u.x, v.y);
+    const float2 ay = __fadd2_rn(u.y, v.x), sy = sub2(u.y, v.x);
+    p.x = INV ? sx : ax;
+    p.y = INV ? ay : sy;
+    q.x = INV ? ax : sx;
+    q.y = INV ? sy : ay;
+  } else if (m == 2 || m == 6) {
+    const float2 s = __fadd2_rn(v.x, v.y), d = sub2(v.x, v.y);
+    // W^2 v = c2 (s, -d) forward, c2 (d, s) inverse; W^6 v = c2 (-d, -s) forward, c2 (-s, d) inverse
+    const float2 a = m == 2 ? (INV ? d : s) : (INV ? s : d), b = m == 2 ? (INV ? s : d) : (INV ? d : s);
+    const float ka = m == 2 ? c2 : -c2, kb = m == 2 ? (INV ? c2 : -c2) : (INV ? c2 : -c2);
+    p.x = __ffma2_rn(a, f2(ka), u.x);
+    p.y = __ffma2_rn(b, f2(kb), u.y);
+    q.x = __ffma2_rn(a, f2(-ka), u.x);
+    q.y = __ffma2_rn(b, f2(-kb), u.y);
+  } else {
+    const float wr = m == 1 ? c1 : (m == 3 ? s1 : (m == 5 ? -s1 : -c1));
+    const float wi = (INV ? 1.f : -1.f) * (m == 1 || m == 7 ? s1 : c1);
+    p.x = __ffma2_rn(v.x, f2(wr), __ffma2_rn(v.y, f2(-wi), u.x));
+    p.y = __ffma2_rn(v.y, f2(wr), __ffma2_rn(v.x, f2(wi), u.y));
+    q.x = __ffma2_rn(v.x, f2(-wr), __ffma2_rn(v.y, f2(wi), u.x));
+    q.y = __ffma2_rn(v.y, f2(-wr), __ffma2_rn(v.x, f2(-wi), u.y));
+  }
+}
+template <int R, int LEN, bool INV> __device__ __forceinline__ void dft_pass2(C2* a) {
+  if constexpr (LEN <= R) {
+#pragma unroll
+    for (int i = 0; i < R; i += LEN)
+#pragma unroll
+      for (int q = 0; q < LEN / 2; ++q) butterfly2<INV>(a[i + q], a[i + q + LEN / 2], q * (16 / LEN));
+    dft_pass2<R, 2 * LEN, INV>(a);
+  }
+}
+template <int R, int I> __device__ __forceinline__ void bitrev_swaps2(C2* a) {
+  if constexpr (I < R) {
+    constexpr int K = bitrev(I, ilog2(R));
+    if constexpr (K > I) {
+      const C2 t = a[I];
+      a[I] = a[K];
+      a[K] = t;
+    }
+    bitrev_swaps2<R, I + 1>(a);
+  }
+}
+template <int R, bool INV> __device__ __forceinline__ void dft2(C2* a) {
+  if constexpr (R > 1) {
+    bitrev_swaps2<R, 0>(a);
+    dft_pass2<R, 2, INV>(a);
+  }
+}
+
+// Exchange buffer of 16-byte elements: p ^ (p / E mod E), conflict-free for the quarter-warps of
+// stage 0's writes (E apart) and of the contiguous reads.
+template <int E> __device__ __forceinline__ int sidx2(int p) { return p ^ ((p / E) & (E - 1)); }
+
+// Twiddles in shared memory as (wr, wr, wi, wi), in lane order: twiddle n of thread j at p[n * NT].
+template <int N, int E> struct TwLane2 {
+  const float4* p;
+  static constexpr int ELEMS = Pipe<N, E>::COUNT * (N / E);
+  static __device__ __forceinline__ void fill(float4* dst, const float2* __restrict__ tab, int tid, int nthreads) {
+    for (int j = tid; j < N / E; j += nthreads)
+      Pipe<N, E>::each(j, [&](int n, int q) {
+        const float2 w = tab[q];
+        dst[n * (N / E) + j] = make_float4(w.x, w.x, w.y, w.y);
+      });
+  }
+};
+// for a single transform beside the packed ones
+template <typename T, int N, int E, bool INV>
+__device__ __forceinline__ float2 tw_at(const TwLane2<N, E>& tw, int n, int p) {
+  (void)p;
+  const float4 w = tw.p[n * (N / E)];
+  return make_float2(w.x, INV ? -w.z : w.z);
+}
+// a W (forward) or a conj(W) (inverse)
+template <bool INV> __device__ __forceinline__ C2 cmul2(const C2& a, float4 w) {
+  const float2 wr = make_float2(w.x, w.y), wi = make_float2(w.z, w.w), nwi = __fmul2_rn(wi, f2(-1.f));
+  C2 r;
+  r.x = __ffma2_rn(a.y, INV ? wi : nwi, __fmul2_rn(a.x, wr));
+  r.y = __ffma2_rn(a.x, INV ? nwi : wi, __fmul2_rn(a.y, wr));
+  return r;
+}
+
+// Exchange slot of element p: row buffers (STRIDE = 1) swizzled, column buffers p STRIDE.
+template <int E, int STRIDE> __device__ __forceinline__ int slot2(int p) { return STRIDE == 1 ? sidx2<E>(p) : p * STRIDE; }
+
+template <int N, int E, bool INV, int STRIDE, int s, class Sync>
+__device__ __forceinline__ void fft_stage2(C2* a, float4* sbuf, int j, const TwLane2<N, E>& tw, Sync sync) {
+  using Sh = FftShape<N, E>;
+  constexpr int NT = Sh::NT, S = Sh::S, R = Sh::radix(s), Ns = Sh::ns(s), Q = E / R;
+  C2 x[E];
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 v = sbuf[slot2<E, STRIDE>(j + NT * q + r * (N / R))];
+      x[q * R + r] = C2{make_float2(v.x, v.y), make_float2(v.z, v.w)};
+    }
+  if constexpr (s < S - 1) sync();
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int b = j + NT * q, k = b % Ns;
+#pragma unroll
+    for (int r = 1; r < R; ++r)
+      x[q * R + r] = cmul2<INV>(x[q * R + r], tw.p[(Pipe<N, E>::first(s) + q * (R - 1) + r - 1) * NT]);
+    dft2<R, INV>(x + q * R);
+    if constexpr (s < S - 1) {
+      const int base = (b / Ns) * Ns * R + k;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const C2 c = x[q * R + r];
+        sbuf[slot2<E, STRIDE>(base + r * Ns)] = make_float4(c.x.x, c.x.y, c.y.x, c.y.y);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[q + r * Q] = x[q * R + r];
+    }
+  }
+  if constexpr (s < S - 1) {
+    sync();
+    fft_stage2<N, E, INV, STRIDE, s + 1>(a, sbuf, j, tw, sync);
+  }
+}
+
+// Both transforms, powers of two: the register contract of fft_run().
+template <int N, int E, bool INV, int STRIDE, class Sync>
+__device__ __forceinline__ void fft_run2(C2* a, float4* sbuf, int j, const TwLane2<N, E>& tw, Sync sync) {
+  dft2<E, INV>(a);
+#pragma unroll
+  for (int r = 0; r < E; ++r)
+    sbuf[slot2<E, STRIDE>(j * E + r)] = make_float4(a[r].x.x, a[r].x.y, a[r].y.x, a[r].y.y);
+  sync();
+  fft_stage2<N, E, INV, STRIDE, 1>(a, sbuf, j, tw, sync);
+}
+
 }  // namespace ld

@@ -76,8 +76,11 @@ template <typename T, int N> struct ZCfg {
   static constexpr int ZBUF1 = P2 ? N + N / E1 : ZBUF;
   // twiddles of the fused pass: in registers where three transforms and they fit (FP64 powers of
   // two; FP32 512, whose eight warps per SM run at 255 registers), else in shared memory in lane
-  // order (FP32 256 at 168 registers and three CTAs per SM: 430 us a right-hand side, 451 with the
-  // twiddles in registers, 440 with them and two CTAs)
+  // order (FP32 128 at 168 registers and three CTAs per SM)
+  // packed transforms: FP32 rows of 256 (right-hand side 388 -> 366 us, warp instructions down by a
+  // quarter); 512 (16 x 16 x 2 at 8 warps per SM: 3.71 -> 3.75 ms), 128 (60.7 -> 64.1 us) and the plane
+  // pass of 64 are not faster with them
+  static constexpr bool PACK = sizeof(T) == 4 && N == 256;
   static constexpr bool TWREG = sizeof(T) == 4 ? N == 512 : Pipe<N, E>::COUNT <= 13;
 };
 
@@ -108,6 +111,12 @@ template <typename T, int N, bool MAP, int RS> struct LdRowsC {
     if (r < 0) return czero<cplx<T>>();
     return io.at(f, o, col)[(long long)r * RS];
   }
+  // columns col, col + 1 (FP32; RS and col even, rows 16-byte aligned)
+  __device__ __forceinline__ float4 two(int f, int o, int n, int col) const {
+    const int r = MAP ? crow(n, N, Cfg<N>::KC) : n;
+    if (r < 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+    return *reinterpret_cast<const float4*>(io.at(f, o, col) + (long long)r * RS);
+  }
 };
 
 // Strided row storer: rows mapped to compact cube rows through crow (MAP; rows outside the cube
@@ -118,6 +127,11 @@ template <typename T, int N, bool MAP, int RS> struct StRowsC {
     const int r = MAP ? crow(n, N, Cfg<N>::KC) : n;
     if (r < 0) return;
     io.at(f, o, col)[(long long)r * RS] = v;
+  }
+  __device__ __forceinline__ void two(int f, int o, int n, int col, float4 v) const {
+    const int r = MAP ? crow(n, N, Cfg<N>::KC) : n;
+    if (r < 0) return;
+    *reinterpret_cast<float4*>(io.at(f, o, col) + (long long)r * RS) = v;
   }
 };
 
@@ -165,6 +179,26 @@ template <typename T, int N> struct LdCurl {
       w = cmuli(csub(cscale(uy, kx), cscale(ux, ky)));
     }
     return w;
+  }
+  // columns col, col + 1 (FP32; col even, u 16-byte aligned): one ky, two neighbouring kz
+  __device__ __forceinline__ float4 two(int f, int o, int n, int col) const {
+    const int r = crow(n, N, kc);
+    if (r < 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const cplx<T>* b = u + (long long)o * bs + (long long)r * My * Mzp + col;
+    auto get = [&](int c) { return *reinterpret_cast<const float4*>(b + c * cs); };
+    if (f < 3) return get(f);
+    const float kx = float(n <= kc ? n : n - N);
+    const int iy = col / Mzp;
+    const float ky = float(cfreq(iy, kc));
+    const float kz = float(col - iy * Mzp);
+    // i (p a - q b) for the two columns
+    auto curl = [](float4 a, float pa0, float pa1, float4 b, float qb0, float qb1) {
+      return make_float4(-(a.y * pa0 - b.y * qb0), a.x * pa0 - b.x * qb0, -(a.w * pa1 - b.w * qb1),
+                         a.z * pa1 - b.z * qb1);
+    };
+    if (f == 3) return curl(get(2), ky, ky, get(1), kz, kz + 1.f);  // i (ky u_z - kz u_y)
+    if (f == 4) return curl(get(0), kz, kz + 1.f, get(2), kx, kx);  // i (kz u_x - kx u_z)
+    return curl(get(1), kx, kx, get(0), ky, ky);                    // i (kx u_y - ky u_x)
   }
 };
 
@@ -216,6 +250,60 @@ template <typename T, int N, bool INV, class Ld, class St>
 constexpr auto colfft_kernel() {
   if constexpr (N == 256 && sizeof(T) == 4) return k_colfft5<T, N, INV, Ld, St>;
   else return k_colfft<T, N, INV, Ld, St>;
+}
+
+// The tile with two neighbouring columns per thread, FP32: 16-byte accesses, and their transforms as
+// packed pairs (C2), which halves the instructions of a pass.  It pays where the one-column tiles
+// queue for issue slots and the load unit (512^3: inverse y 823 -> 736 us, right-hand side 3.70 ->
+// 3.43 ms; 128^3 60.5 -> 58.4 us); at 256^3 the passes wait for memory either way (366 -> 361 us).  The twiddles are put into shared
+// memory in lane order, behind the exchange buffer.
+template <int N> struct Col2 {
+  static constexpr int E = Cfg<N>::EC, NT = Cfg<N>::NTC, PAIRS = Cfg<N>::TB / 2;
+  static constexpr bool OK = is_pow2(N) && E == 16 && N >= 128;
+  static constexpr int THREADS = PAIRS * NT;
+  static constexpr int MINB = 640 / THREADS;  // 96 registers (128: five in four at 256^3; 80: spills)
+  using Tw = TwLane2<is_pow2(N) ? N : 64, is_pow2(N) ? E : 8>;
+  static constexpr size_t BUF = sizeof(float4) * N * PAIRS, SMEM = BUF + sizeof(float4) * Tw::ELEMS;
+};
+__device__ __forceinline__ C2 pair_of(float4 v) { return C2{make_float2(v.x, v.z), make_float2(v.y, v.w)}; }
+__device__ __forceinline__ float4 columns_of(const C2& c) { return make_float4(c.x.x, c.y.x, c.x.y, c.y.y); }
+
+template <int N, bool INV, class Ld, class St>
+__device__ __forceinline__ void colfft_tile2(const Ld& ld, const St& st, int ncols, int nf, const float2* __restrict__ tw,
+                                             unsigned char* smem) {
+  using C = Col2<N>;
+  constexpr int E = C::E, NT = C::NT;
+  float4* sbuf = reinterpret_cast<float4*>(smem);
+  float4* tws = reinterpret_cast<float4*>(smem + C::BUF);
+  const int c = threadIdx.x % C::PAIRS, j = threadIdx.x / C::PAIRS;
+  __builtin_assume(j >= 0 && j < NT);
+  const int field = blockIdx.x % nf;
+  const int col = (blockIdx.x / nf) * Cfg<N>::TB + 2 * c;
+  const bool ok = col < ncols;  // ncols is even
+  const int outer = blockIdx.y;
+  float4 v[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) v[m] = ok ? ld.two(field, outer, j + NT * m, col) : make_float4(0.f, 0.f, 0.f, 0.f);
+  C::Tw::fill(tws, tw, threadIdx.x, C::THREADS);  // before the exchange's first barrier
+  typename C::Tw t;
+  t.p = tws + j;
+  C2 a[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) a[m] = pair_of(v[m]);
+  fft_run2<N, E, INV, C::PAIRS>(a, sbuf + c, j, t, SyncBlock());
+  if (ok) {
+#pragma unroll
+    for (int m = 0; m < E; ++m) st.two(field, outer, j + NT * m, col, columns_of(a[m]));
+  }
+}
+
+
+template <int N, bool INV, class Ld, class St>
+__global__ void __launch_bounds__(Col2<N>::THREADS, Col2<N>::MINB)
+k_colfft2(Ld ld, St st, int ncols, int nf, const float2* __restrict__ tw) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_dep();
+  colfft_tile2<N, INV>(ld, st, ncols, nf, tw, smem_raw);
 }
 
 // Sum of 0.5 |u|^2 normalize over the modes listed for shell s (CSR of cube indices), by the block
@@ -293,6 +381,15 @@ k_xinv5(LdCurl<T, N> ld, St st, int ncols, const cplx<T>* __restrict__ tw, Shell
   extern __shared__ __align__(16) unsigned char smem_raw[];
   grid_dep();
   xinv_block<T, N>(ld, st, ncols, tw, F, smem_raw);
+}
+template <int N, class St>
+__global__ void __launch_bounds__(Col2<N>::THREADS, Col2<N>::MINB)
+k_xinv2(LdCurl<float, N> ld, St st, int ncols, const float2* __restrict__ tw, ShellArgs<float> F) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_dep();
+  const int tiles = 6 * ((ncols + Cfg<N>::TB - 1) / Cfg<N>::TB);
+  if ((int)blockIdx.x < tiles) colfft_tile2<N, true>(ld, st, ncols, 6, tw, smem_raw);
+  else shell_sum(F, F.shell0 + (int)blockIdx.x - tiles, (int)blockIdx.y, reinterpret_cast<double*>(smem_raw));
 }
 template <typename T, int N, class St> constexpr auto xinv_kernel() {
   if constexpr (N == 256 && sizeof(T) == 4) return k_xinv5<T, N, St>;
@@ -379,6 +476,79 @@ k_colfft_pipe(RowsIO<T> in, St st, int ncols, int nf, int nouter, const cplx<T>*
       for (int m = 0; m < E; ++m) st(f, o, j + NT * m, col, a[m]);
     }
     __syncthreads();
+    b ^= 1;
+    cur_item = next_item;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// The pipelined pass with two columns per thread (see colfft_tile2 and k_colfft_pipe).
+template <int N, bool INV, class St, bool IN_MAP, int RS>
+__global__ void __launch_bounds__(Col2<N>::THREADS, 3)
+k_colfft_pipe2(RowsIO<float> in, St st, int ncols, int nf, int nouter, const float2* __restrict__ tw) {
+  using C = Col2<N>;
+  constexpr int E = C::E, NT = C::NT, PAIRS = C::PAIRS, TB = Cfg<N>::TB, THREADS = C::THREADS;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float4* buf0 = reinterpret_cast<float4*>(smem_raw);
+  float4* buf1 = buf0 + N * PAIRS;
+  float4* tws = buf1 + N * PAIRS;
+  const int c = threadIdx.x % PAIRS, j = threadIdx.x / PAIRS;
+  __builtin_assume(j >= 0 && j < NT);
+  C::Tw::fill(tws, tw, threadIdx.x, THREADS);
+  typename C::Tw t;
+  t.p = tws + j;
+  grid_dep();
+  const unsigned ncb = (unsigned)((ncols + TB - 1) / TB);
+  const unsigned nitems = ncb * (unsigned)nf * (unsigned)nouter;
+  struct Item {
+    int cb, f, o;
+  };
+  auto split = [&](unsigned it) {
+    const unsigned rest = it / ncb;
+    const unsigned fo = rest / (unsigned)nf;
+    return Item{(int)(it - rest * ncb), (int)(rest - fo * (unsigned)nf), (int)fo};
+  };
+  // this thread copies what it will transform: its two columns of rows j + NT m
+  auto prefetch = [&](const Item& itm, float4* dst) {
+    if (itm.cb * TB + 2 * c < ncols) {
+      const float2* src = in.at(itm.f, itm.o, itm.cb * TB + 2 * c);
+      const unsigned d = (unsigned)__cvta_generic_to_shared(dst + c);
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const int n = j + NT * m, r = IN_MAP ? crow(n, N, Cfg<N>::KC) : n;
+        if (r < 0) continue;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * PAIRS * n), "l"(src + (long long)r * RS)
+                     : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  unsigned it = blockIdx.x;
+  Item cur_item = split(it);
+  if (it < nitems) prefetch(cur_item, buf0);
+  int b = 0;
+  __syncthreads();  // the twiddles
+  for (; it < nitems; it += gridDim.x) {
+    float4* cur = b ? buf1 : buf0;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const int f = cur_item.f, o = cur_item.o;
+    const int col = cur_item.cb * TB + 2 * c;
+    const bool ok = col < ncols;
+    C2 a[E];
+#pragma unroll
+    for (int m = 0; m < E; ++m) {  // the thread's own copies
+      const int n = j + NT * m, r = IN_MAP ? crow(n, N, Cfg<N>::KC) : n;
+      a[m] = pair_of(ok && r >= 0 ? cur[n * PAIRS + c] : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    __syncthreads();  // every value is in registers: cur becomes the exchange buffer, the other is free
+    const unsigned nx = it + gridDim.x;
+    const Item next_item = split(nx);
+    if (nx < nitems) prefetch(next_item, b ? buf0 : buf1);
+    fft_run2<N, E, INV, PAIRS>(a, cur + c, j, t, SyncBlock());
+    if (ok) {
+#pragma unroll
+      for (int m = 0; m < E; ++m) st.two(f, o, j + NT * m, col, columns_of(a[m]));
+    }
     b ^= 1;
     cur_item = next_item;
   }
@@ -832,6 +1002,55 @@ __device__ __forceinline__ void zcross_forward(cplx<T>* p0, cplx<T>* p1, const c
   zstore_pair<T, N, E>(p1, C, (cplx<T>*)nullptr, Kout, Kin, j, own);
 }
 
+// The fused z pass of an FP32 row of power-of-two length with packed transforms: (u_x, u_y) and
+// (u_z, w_x) transform side by side, (w_y, w_z) alone, the products (two and one) side by side.
+// Hermitian-extended load of two pairs of fields (A0, B0), (A1, B1), as zload_pair.
+template <int N, int E>
+__device__ __forceinline__ void zload_pair2(C2* a, const float2* A0, const float2* B0, const float2* A1, const float2* B1,
+                                            int Kin, int j, float s) {
+  float2 t0[E], t1[E];
+  zload_pair<float, N, E>(t0, A0, B0, Kin, j, s);
+  zload_pair<float, N, E>(t1, A1, B1, Kin, j, s);
+#pragma unroll
+  for (int m = 0; m < E; ++m) a[m] = C2{make_float2(t0[m].x, t1[m].x), make_float2(t0[m].y, t1[m].y)};
+}
+
+// zcross_forward from the packed inverse transforms p = ((u_x, u_z), (u_y, w_x)) and p2 = (w_y, w_z).
+template <int N, int E>
+__device__ __forceinline__ void zcross_forward2(C2* p, const float2* p2, float4* sb, float2* A, float2* B, float2* C,
+                                                long long row, float* uphys, int ulayout, int Kout, int Kin, int j,
+                                                bool own, const TwLane2<N, E>& tw) {
+  constexpr int NT = N / E;
+  if (uphys && own) {
+    const long long NN3 = (long long)N * N * N;
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      const int n = j + NT * m;
+      if (ulayout == 0) {  // planar (3, N, N, N)
+        uphys[row * N + n] = p[m].x.x;
+        uphys[NN3 + row * N + n] = p[m].y.x;
+        uphys[2 * NN3 + row * N + n] = p[m].x.y;
+      } else {  // interleaved (N, N, N, 4)
+        reinterpret_cast<float4*>(uphys)[row * N + n] = make_float4(p[m].x.x, p[m].y.x, p[m].x.y, 0.f);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < E; ++m) {
+    const float ux = p[m].x.x, uy = p[m].y.x, uz = p[m].x.y, wx = p[m].y.y, wy = p2[m].x, wz = p2[m].y;
+    p[m] = C2{make_float2(wz * uy - wy * uz, wy * ux - wx * uy), make_float2(wx * uz - wz * ux, 0.f)};
+  }
+  fft_run2<N, E, false, 1>(p, sb, j, tw, SyncWarp());
+  SyncWarp()();  // A, B, C may lie in the exchange buffer
+  float2 t[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) t[m] = make_float2(p[m].x.x, p[m].y.x);
+  zstore_pair<float, N, E>(t, A, B, Kout, Kin, j, own);
+#pragma unroll
+  for (int m = 0; m < E; ++m) t[m] = make_float2(p[m].x.y, p[m].y.y);
+  zstore_pair<float, N, E>(t, C, (float2*)nullptr, Kout, Kin, j, own);
+}
+
 // Fused z pass: persistent warps walk groups of R rows with a
 // stride.  The six field rows of the warp's next group are brought into shared memory by bulk
 // asynchronous copies (the TMA engine), one mbarrier per pair of fields, each issued as soon as
@@ -846,10 +1065,11 @@ constexpr unsigned kWaitLimit = 1u << 24;
 
 template <typename T, int N> struct ZPipe {
   using Z = ZCfg<T, N>;
+  static constexpr bool PACK = Z::PACK;
   static constexpr int WARPS = 4;
   static constexpr int STAGE = 6 * Z::R * Cfg<N>::MZP;  // elements per warp
-  static constexpr int EX = Z::R * Z::ZBUF;
-  static constexpr int TW = Z::TWREG ? 0 : TwLane<T, N, Z::E>::ELEMS;
+  static constexpr int EX = PACK ? 2 * Z::R * N : Z::R * Z::ZBUF;
+  static constexpr int TW = PACK ? 2 * TwLane<T, N, Z::E>::ELEMS : (Z::TWREG ? 0 : TwLane<T, N, Z::E>::ELEMS);
   static constexpr size_t SMEM = sizeof(cplx<T>) * ((size_t)WARPS * (STAGE + EX) + TW) + 32 * WARPS;
   // CTAs per SM asked of the compiler: 3 E complex values and what a transform needs besides
   static constexpr int MINB = sizeof(T) == 4 && N != 512 ? 3 : 2;
@@ -870,7 +1090,7 @@ k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __rest
   const bool own = lane < R * Z::NT;
   cplx<T>* base = reinterpret_cast<cplx<T>*>(smem_raw);
   cplx<T>* stage = base + warp * ZP::STAGE;
-  cplx<T>* sb = base + WARPS * ZP::STAGE + warp * ZP::EX + unit * Z::ZBUF;
+  cplx<T>* sb = base + WARPS * ZP::STAGE + warp * ZP::EX + unit * (ZP::PACK ? 2 * N : Z::ZBUF);
   cplx<T>* tws = base + WARPS * (ZP::STAGE + ZP::EX);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tws + ZP::TW) + 4 * warp;
   const long long fs = NR * MZ;
@@ -881,12 +1101,16 @@ k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __rest
     for (int q = 0; q < 4; ++q) mbar_init(&bars[q], 1);
     mbar_init_fence();
   }
-  typename std::conditional<Z::TWREG, TwRegs<T, N, E>, TwLane<T, N, E>>::type twr;
-  if constexpr (Z::TWREG) {
+  typename std::conditional<ZP::PACK, TwLane2<N, E>,
+                            typename std::conditional<Z::TWREG, TwRegs<T, N, E>, TwLane<T, N, E>>::type>::type twr;
+  if constexpr (!ZP::PACK && Z::TWREG) {
     twr.load(tw, j);
   } else {
-    TwLane<T, N, E>::fill(tws, tw, threadIdx.x, 32 * WARPS);
-    twr.p = tws + j;
+    using Table = decltype(twr);
+    using Elem = typename std::remove_const<typename std::remove_pointer<decltype(twr.p)>::type>::type;
+    Elem* t = reinterpret_cast<Elem*>(tws);
+    Table::fill(t, tw, threadIdx.x, 32 * WARPS);
+    twr.p = t + j;
     __syncthreads();
   }
   grid_dep();
@@ -911,16 +1135,21 @@ k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __rest
     return;
   }
   unsigned ph = 0;
-  // pair q of this group into registers, then its next group's copy; false after a time-out (pairs
-  // before q already belong to the next group's phase, when there is one)
-  auto take = [&](cplx<T>* a, int q, long long next) -> bool {
+  // waits for pair q of this group; false after a time-out (pairs before q already belong to the next
+  // group's phase when there is one and `moved`)
+  auto arrived = [&](int q, long long next, bool moved) -> bool {
     if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[q], ph, wait_limit))) {
       if (lane == 0) atomicOr(status, LD_STATUS_WAIT_TIMEOUT);
       for (int b = 0; b < 3; ++b)
         if (b >= q) mbar_wait_bounded(&bars[b], ph, kWaitLimit);
-        else if (next < NR) mbar_wait_bounded(&bars[b], ph ^ 1u, kWaitLimit);
+        else if (moved && next < NR) mbar_wait_bounded(&bars[b], ph ^ 1u, kWaitLimit);
       return false;
     }
+    return true;
+  };
+  // pair q of this group into registers, then its next group's copy
+  auto take = [&](cplx<T>* a, int q, long long next) -> bool {
+    if (!arrived(q, next, true)) return false;
     const cplx<T>* A = stage + (2 * q * R + unit) * MZ;
     zload_pair<T, N, E>(a, A, A + R * MZ, KIN, j, s);
     __syncwarp();  // every lane has read the pair
@@ -929,6 +1158,27 @@ k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __rest
   };
   for (; row < NR; row += stride, ph ^= 1u) {
     const long long next = row + stride;
+    cplx<T>* out = P + (row + unit) * MZ;
+    if constexpr (ZP::PACK) {
+      C2 p[E];
+      cplx<T> p2[E];
+      float4* sb4 = reinterpret_cast<float4*>(sb);
+      if (!arrived(0, next, false) || !arrived(1, next, false)) return;
+      const cplx<T>* A = stage + unit * MZ;
+      zload_pair2<N, E>(p, A, A + R * MZ, A + 2 * R * MZ, A + 3 * R * MZ, KIN, j, s);
+      __syncwarp();  // every lane has read the pairs
+      if (next < NR) {
+        issue(next, 0);
+        issue(next, 1);
+      }
+      fft_run2<N, E, true, 1>(p, sb4, j, twr, SyncWarp());
+      if (!take(p2, 2, next)) return;  // (w_y, w_z); its __syncwarp frees the exchange buffer
+      fft_run<T, N, E, true, true>(p2, sb, 1, j, twr, SyncWarp());
+      __syncwarp();
+      zcross_forward2<N, E>(p, p2, sb4, out, out + fs, out + 2 * fs, row + unit, uphys, ulayout, MZ, KIN, j, own, twr);
+      __syncwarp();  // every lane is done with the exchange buffer
+      continue;
+    } else {
     cplx<T> p0[E], p1[E], p2[E];
     if (!take(p0, 0, next)) return;  // (u_x, u_y)
     fft_run<T, N, E, true, true>(p0, sb, 1, j, twr, SyncWarp());
@@ -937,9 +1187,9 @@ k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __rest
     if (!take(p2, 2, next)) return;  // (w_y, w_z)
     fft_run<T, N, E, true, true>(p2, sb, 1, j, twr, SyncWarp());
     __syncwarp();
-    cplx<T>* out = P + (row + unit) * MZ;
     zcross_forward<T, N>(p0, p1, p2, sb, out, out + fs, out + 2 * fs, row + unit, uphys, ulayout, MZ, KIN, j, own, twr);
     __syncwarp();  // every lane is done with the exchange buffer
+    }
   }
 }
 
@@ -969,12 +1219,14 @@ template <typename T, int N> struct PlaneCfg {
   static constexpr int THREADS = M == 96 ? 384 : (M == 16 ? 128 : 256);
   static constexpr int TWZ = TwLane<T, M, Z::E>::ELEMS;
   static constexpr size_t SMEM = sizeof(cplx<T>) * ((size_t)M * PITCH + TWZ + M);
-  static constexpr int MINB = M == 64 && sizeof(T) == 4 ? 3 : 1;
 };
 
 // W: (6, NO, My, Mzp) in (columns kz <= kc read), P: (3, NO, My, Mzp) out, NO = boxes x N planes
-template <typename T, int N>
-__global__ void __launch_bounds__(PlaneCfg<T, N>::THREADS, PlaneCfg<T, N>::MINB)
+// MINB: blocks per SM asked of the compiler.  Many planes of FP32 64 run three per SM at 80 registers
+// (16 boxes, five ensemble steps: 1.50 ms, 1.56 at 96 registers); a few run faster at 96 (one box:
+// right-hand side 21.4 us, 26.2 at 80; four boxes: 621 and 626 us for five steps).
+template <typename T, int N, int MINB>
+__global__ void __launch_bounds__(PlaneCfg<T, N>::THREADS, MINB)
 k_plane(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __restrict__ uphys, int ulayout, T s,
         const cplx<T>* __restrict__ tw, long long NO) {
   using C = PlaneCfg<T, N>;

@@ -31,6 +31,8 @@ inline int grid1d(long long n, int threads) {
   return (int)b;
 }
 
+inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
 template <typename T, int N> struct Ops {
   using C = cplx<T>;
   static constexpr int TB = Cfg<N>::TB;
@@ -51,6 +53,22 @@ template <typename T, int N> struct Ops {
     return LD_OK;
   }
 
+  // The same with two columns per thread (FP32, even row strides and columns, 16-byte aligned rows)
+  static constexpr bool PAIRS = sizeof(T) == 4 && Col2<N>::OK;
+  template <bool INV, class Ld, class St>
+  static int colpass2(ld_plan* p, int kid, Ld ld, St st, int ncols, int nf, int nouter, const C* tw, cudaStream_t s) {
+    ProfScope ps(p, kid, s);
+    auto k = k_colfft2<N, INV, Ld, St>;
+    if (int rc = set_smem(k, Col2<N>::SMEM)) return rc;
+    dim3 grid((unsigned)(cdiv(ncols, TB) * nf), (unsigned)nouter);
+    LD_CUDA_CHECK(launch_dep(early(p), k, grid, Col2<N>::THREADS, Col2<N>::SMEM, s, ld, st, ncols, nf, tw));
+    return LD_OK;
+  }
+  template <bool INV, class St, bool IN_MAP, int RSC> static constexpr auto pipe_kernel() {
+    if constexpr (PAIRS) return k_colfft_pipe2<N, INV, St, IN_MAP, RSC>;
+    else return k_colfft_pipe<T, N, INV, St, IN_MAP, RSC>;
+  }
+
   // Column pass over plain strided rows: the pipelined kernel where two staging buffers fit.
   static constexpr bool PIPE = 2 * COL_SMEM <= 72 * 1024;
   // IN_MAP: the input rows are compact cube rows; RS: their stride
@@ -59,16 +77,23 @@ template <typename T, int N> struct Ops {
                           cudaStream_t s, int variant = -2) {
     const int choice = variant != -2 ? variant : p->tune_y[INV ? 0 : 1];
     if constexpr (!PIPE) {
-      return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
+      if constexpr (PAIRS) return colpass2<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
+      else return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
     } else {
-      if (choice == 0 || cdiv(ncols, TB) * (long long)nf * nouter >= (1LL << 31))
-        return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
+      // untuned plans: one-shot tiles for short columns (right-hand side at 128^3 FP64 105 -> 95 us), except
+      // with two columns per thread (FP32 58 -> 61 us)
+      if (choice == 0 || (choice < 0 && N <= 128 && !PAIRS) || cdiv(ncols, TB) * (long long)nf * nouter >= (1LL << 31)) {
+        if constexpr (PAIRS) return colpass2<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
+        else return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
+      }
       ProfScope ps(p, kid, s);
-      auto k = k_colfft_pipe<T, N, INV, St, IN_MAP, RS>;
-      if (int rc = set_smem(k, 2 * COL_SMEM)) return rc;
+      constexpr int threads = PAIRS ? Col2<N>::THREADS : Cfg<N>::COL_THREADS;
+      constexpr size_t smem = 2 * COL_SMEM + (PAIRS ? sizeof(float4) * Col2<N>::Tw::ELEMS : 0);
+      auto k = pipe_kernel<INV, St, IN_MAP, RS>();
+      if (int rc = set_smem(k, smem)) return rc;
       static int occ = 0;
       if (occ == 0) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, Cfg<N>::COL_THREADS, 2 * COL_SMEM);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, threads, smem);
         if (e != cudaSuccess || occ < 1) occ = 1;
       }
       int dev = 0, sms = 148;
@@ -77,8 +102,7 @@ template <typename T, int N> struct Ops {
       const long long items = cdiv(ncols, TB) * (long long)nf * nouter;
       const int per_sm = choice > 0 && choice < occ ? choice : occ;
       const long long grid = items < (long long)sms * per_sm ? items : (long long)sms * per_sm;
-      LD_CUDA_CHECK(launch_dep(early(p), k, dim3((unsigned)grid), Cfg<N>::COL_THREADS, 2 * COL_SMEM, s, in, st, ncols,
-                               nf, nouter, tw));
+      LD_CUDA_CHECK(launch_dep(early(p), k, dim3((unsigned)grid), threads, smem, s, in, st, ncols, nf, nouter, tw));
       return LD_OK;
     }
   }
@@ -306,10 +330,21 @@ template <typename T, int N> struct Ops {
       ProfScope ps(p, KID_XINV, s);
       using St = StRowsC<T, N, false, RS::XC>;
       const ShellArgs<T> F = forcing(p, y, prm);
-      auto k = xinv_kernel<T, N, St>();
-      if (int rc = set_smem(k, COL_SMEM)) return rc;
       const dim3 grid((unsigned)(cdiv(My * Mzp, TB) * 6 + F.nshell), (unsigned)nb);
-      LD_CUDA_CHECK(launch_dep(early(p), k, grid, Cfg<N>::COL_THREADS, COL_SMEM, s, lc, St{xout}, My * Mzp, tw, F));
+      bool pairs = false;
+      if constexpr (PAIRS) {
+        pairs = aligned16(y);  // the state is the caller's buffer
+        if (pairs) {
+          auto k = k_xinv2<N, St>;
+          if (int rc = set_smem(k, Col2<N>::SMEM)) return rc;
+          LD_CUDA_CHECK(launch_dep(early(p), k, grid, Col2<N>::THREADS, Col2<N>::SMEM, s, lc, St{xout}, My * Mzp, tw, F));
+        }
+      }
+      if (!pairs) {
+        auto k = xinv_kernel<T, N, St>();
+        if (int rc = set_smem(k, COL_SMEM)) return rc;
+        LD_CUDA_CHECK(launch_dep(early(p), k, grid, Cfg<N>::COL_THREADS, COL_SMEM, s, lc, St{xout}, My * Mzp, tw, F));
+      }
     }
     const T sc = T(1.0 / (double(N) * N * N));
     const int ulayout = (MODE == UPD_RHS) ? 0 : 1;  // the time steppers feed droplets: interleaved
@@ -317,7 +352,10 @@ template <typename T, int N> struct Ops {
       // y inverse, fused z and y forward of one x plane per block (W1 -> W2 as (3, N, My, Mzp))
       using PC = PlaneCfg<T, N>;
       ProfScope ps(p, KID_ZCROSS, s);
-      auto k = k_plane<T, N>;
+      auto k = k_plane<T, N, 1>;
+      if constexpr (N == 64 && sizeof(T) == 4) {
+        if (nb * N >= 3 * kSMs) k = k_plane<T, N, 3>;
+      }
       if (int rc = set_smem(k, PC::SMEM)) return rc;
       LD_CUDA_CHECK(launch_dep(early(p), k, dim3((unsigned)(nb * N)), PC::THREADS, PC::SMEM, s, W1, W2, uout, ulayout, sc, tw,
                                (long long)nb * N));
@@ -351,7 +389,8 @@ template <typename T, int N> struct Ops {
     A.blowup = T(100.0 * (double)N * N * N);  // the blow-up threshold of the step epilogue (F:618)
     // the cube rows the update reads are staged in shared memory when that keeps 2 CTAs per SM
     const size_t pre_bytes = sizeof(C) * 3 * (size_t)(2 * kc + 1) * TB;
-    A.prefetch = COL_SMEM + pre_bytes <= 112 * 1024 ? 1 : 0;
+    const bool al = aligned16(MODE == UPD_RK2_2 ? s2 : s1);  // 16-byte copies from the caller's buffers
+    A.prefetch = al && COL_SMEM + pre_bytes <= 112 * 1024 ? 1 : 0;
     const size_t smem = COL_SMEM + (A.prefetch ? pre_bytes : 0);
     ProfScope ps(p, KID_XFWD_UPD, s);
     auto k = k_xfwd_update<T, N, MODE>;

@@ -1,0 +1,72 @@
+"""Forms of the flow's passes that a plan chooses by size, batch or alignment: they agree with the
+forms that the oracle tests cover."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch
+    assert torch.cuda.is_available()
+    return torch
+
+
+def _state(torch, p, seed, nbox=None):
+    """A smooth random cube spectrum, the same for every precision."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    shape = ((nbox,) if nbox else ()) + (3, p.Mx, p.My, p.Mzp)
+    uk = torch.view_as_complex(torch.randn(shape + (2,), dtype=torch.float64, device="cuda", generator=g))
+    k = torch.cat([torch.arange(p.kc + 1), torch.arange(-p.kc, 0)]).double().cuda()
+    kz = torch.arange(p.Mzp).double().cuda()
+    k2 = k[:, None, None] ** 2 + k[None, :, None] ** 2 + kz ** 2
+    uk = uk * torch.where(k2 <= p.kc * p.kc + p.kc, p.N ** 3 / (1.0 + k2), 0.0)
+    return uk.to(p.cdtype)
+
+
+# FP32 tolerance of one RHS evaluation (tests/test_dns_gpu.py)
+TOL = 2e-5
+
+
+@pytest.mark.parametrize("N", [64, 128, 256])
+def test_state_off_the_16_byte_grid(torch, N):
+    """A contiguous state that starts 8 bytes past a 16-byte boundary takes one column per thread and
+    no row prefetch; the same RHS to FP32 rounding, and nothing past the end is read or written."""
+    from lucky_droplets_b200.spectral import Plan
+    p = Plan(N, "f32")
+    uk = _state(torch, p, N)
+    ref = p.velocity_rhs(uk, 0.01, 1.0, (1, 2))
+    off = torch.zeros(uk.numel() + 1, dtype=uk.dtype, device="cuda")[1:].view(uk.shape)
+    out = torch.zeros(uk.numel() + 1, dtype=uk.dtype, device="cuda")[1:].view(uk.shape)
+    off.copy_(uk)
+    assert off.data_ptr() % 16 == 8 and out.data_ptr() % 16 == 8
+    got = p.velocity_rhs(off, 0.01, 1.0, (1, 2), ku=out)
+    assert float(torch.linalg.norm(got - ref) / torch.linalg.norm(ref)) < TOL
+    assert torch.equal(off, uk)
+
+
+@pytest.mark.parametrize("N,nbox", [(64, 3), (64, 8), (32, 5), (16, 2)])
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_boxes_of_a_batch_equal_boxes_alone(torch, N, nbox, prec):
+    """The plane pass of few planes and of many (three blocks per SM from 444 planes of FP32 64)."""
+    from lucky_droplets_b200.spectral import Plan
+    many, one = Plan(N, prec, nbox=nbox), Plan(N, prec)
+    uk = _state(torch, one, N + nbox, nbox)
+    ku = torch.zeros_like(uk)
+    many.velocity_rhs(uk, 0.01, 1.0, (1, 2), ku=ku)
+    for b in range(nbox):
+        assert torch.equal(ku[b], one.velocity_rhs(uk[b].contiguous(), 0.01, 1.0, (1, 2)))
+
+
+@pytest.mark.parametrize("N", [384, 512])
+def test_large_grids_fp32_against_fp64(torch, N):
+    """Two columns per thread with three radix stages (512), the longest 12 R2 R3 rows (384)."""
+    from lucky_droplets_b200.spectral import Plan
+    p32 = Plan(N, "f32")
+    uk = _state(torch, p32, N)
+    got = p32.velocity_rhs(uk, 0.01, 1.0, (1, 2))
+    p64 = Plan(N, "f64")
+    ref = p64.velocity_rhs(uk.to(torch.complex128), 0.01, 1.0, (1, 2))
+    assert float(torch.linalg.norm(got - ref) / torch.linalg.norm(ref)) < TOL
+    assert np.isfinite(float(got.abs().max()))
