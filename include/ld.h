@@ -182,10 +182,10 @@ LD_API int ld_rk4_stage(ld_plan* plan, int stage, void* uk, void* y, void* acc, 
 LD_API int ld_plan_autotune(ld_plan* plan, double* ms, int32_t* choice, void* stream);
 LD_API int ld_plan_set_tuning(ld_plan* plan, const int32_t* choice);
 /* Bounded device waits (no counterpart in the reference, whose failures end in comm.Abort,
- * F:618-620): the waits of the plan's pipelined kernels (the fused z pass at N >= 256, the
- * tensor-core MLP forward) give up after `limit` polls (0: the default, 2^24), raise
- * LD_STATUS_WAIT_TIMEOUT, let the copies and MMAs they issued complete, free their tensor memory
- * and return; the launch and the context stay usable.  stall != 0 tests that path: the first wait
+ * F:618-620): the waits of the plan's pipelined kernels (the fused z pass where it runs
+ * on its own, N >= 128 and FP64 96; the tensor-core MLP forward) give up after `limit` polls
+ * (0: the default, 2^24), raise LD_STATUS_WAIT_TIMEOUT, let the copies and MMAs they issued
+ * complete, free their tensor memory and return; the launch and the context stay usable.  stall != 0 tests that path: the first wait
  * of every warp (z pass) or warp group (MLP forward) is on a barrier that nothing completes, so
  * it runs out after `limit` polls while the first copy is in flight.  stall = 0 for production. */
 LD_API int ld_plan_set_wait_limit(ld_plan* plan, uint32_t limit, int stall);

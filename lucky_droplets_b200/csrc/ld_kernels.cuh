@@ -1177,18 +1177,18 @@ k_z_cross_pipe(const cplx<T>* __restrict__ W, cplx<T>* __restrict__ P, T* __rest
       __syncwarp();
       zcross_forward2<N, E>(p, p2, sb4, out, out + fs, out + 2 * fs, row + unit, uphys, ulayout, MZ, KIN, j, own, twr);
       __syncwarp();  // every lane is done with the exchange buffer
-      continue;
     } else {
-    cplx<T> p0[E], p1[E], p2[E];
-    if (!take(p0, 0, next)) return;  // (u_x, u_y)
-    fft_run<T, N, E, true, true>(p0, sb, 1, j, twr, SyncWarp());
-    if (!take(p1, 1, next)) return;  // (u_z, w_x); its __syncwarp frees the exchange buffer
-    fft_run<T, N, E, true, true>(p1, sb, 1, j, twr, SyncWarp());
-    if (!take(p2, 2, next)) return;  // (w_y, w_z)
-    fft_run<T, N, E, true, true>(p2, sb, 1, j, twr, SyncWarp());
-    __syncwarp();
-    zcross_forward<T, N>(p0, p1, p2, sb, out, out + fs, out + 2 * fs, row + unit, uphys, ulayout, MZ, KIN, j, own, twr);
-    __syncwarp();  // every lane is done with the exchange buffer
+      cplx<T> p0[E], p1[E], p2[E];
+      if (!take(p0, 0, next)) return;  // (u_x, u_y)
+      fft_run<T, N, E, true, true>(p0, sb, 1, j, twr, SyncWarp());
+      if (!take(p1, 1, next)) return;  // (u_z, w_x); its __syncwarp frees the exchange buffer
+      fft_run<T, N, E, true, true>(p1, sb, 1, j, twr, SyncWarp());
+      if (!take(p2, 2, next)) return;  // (w_y, w_z)
+      fft_run<T, N, E, true, true>(p2, sb, 1, j, twr, SyncWarp());
+      __syncwarp();
+      zcross_forward<T, N>(p0, p1, p2, sb, out, out + fs, out + 2 * fs, row + unit, uphys, ulayout, MZ, KIN, j, own,
+                           twr);
+      __syncwarp();  // every lane is done with the exchange buffer
     }
   }
 }
