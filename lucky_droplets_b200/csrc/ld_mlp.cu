@@ -557,7 +557,7 @@ k_mlp_features(const vec4<T>* __restrict__ u4, int N, double L, const double* __
 //   layer 2: 8 MMAs from H and W2; epilogue as above -> H;
 //   layer 3: 8 MMAs (N 16: W3 padded); 4 warps write out = tricubic + scale * os * MLP in the grid
 //   frame.
-// The group's leader issues its MMAs and commits them to the group's mbarrier; group barriers are
+// One lane of the group's first warp issues its MMAs and commits them to the group's mbarrier; group barriers are
 // named barriers.  Every wait is bounded (wait_limit polls, the plan's setting): a wait that runs
 // out raises LD_STATUS_WAIT_TIMEOUT and the group stops; before the CTA frees its tensor memory
 // and exits, one thread waits (bounded by kWaitLimitMlp) for the feature copy and the MMAs that
@@ -605,7 +605,8 @@ k_mlp_forward_tc(const unsigned char* __restrict__ Xg, const float* __restrict__
                  unsigned* __restrict__ status, unsigned wait_limit, int stall) {
   extern __shared__ __align__(1024) unsigned char sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = warp >> 3, gw = warp & 7;             // group, warp within the group
+  const int wu = __shfl_sync(0xffffffffu, warp, 0);   // known to be warp-uniform
+  const int g = wu >> 3, gw = wu & 7;                 // group, warp within the group
   const bool leader = (tid & (FT_GROUP - 1)) == 0;
   float* bias = reinterpret_cast<float*>(sm + SM_BIAS);
   // copy i of the X buffer completes on bar_x[i % 2]: group g waits only on bar_x[g], so every
@@ -616,7 +617,7 @@ k_mlp_forward_tc(const unsigned char* __restrict__ Xg, const float* __restrict__
   uint64_t* bar_w = bar_x + 5;      // the weights' bulk copies
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(sm + SM_TMEM);
   // drain bookkeeping: X copies issued to / waited on each bar_x, MMA commits to / waits on each
-  // bar_mma; each counter has one writer (a group leader; cnt[0] leaves out the first copy, which
+  // bar_mma; each counter has one writer (a lane of a group's first warp; cnt[0] leaves out the first copy, which
   // thread 0 issues before the loop) and thread 0 reads them after the final barrier
   unsigned* cnt = reinterpret_cast<unsigned*>(sm + SM_CNT);  // [x_issued 2][x_waited 2][mma_commit 2][mma_wait 2]
   // b1, b2 halved: the epilogues form h = z / 2 = fma(0.5, acc, b / 2), which is exactly
@@ -682,13 +683,12 @@ k_mlp_forward_tc(const unsigned char* __restrict__ Xg, const float* __restrict__
     }
     failed = group_or(g, !mbar_wait_bounded(&bar_x[g], (unsigned)((i >> 1) & 1), wait_limit));
     if (failed) break;
-    if (leader) {
+    __syncwarp();
+    if (gw == 0 && elect_one()) {
       cnt[2 + g] += 1u;
       tc_fence_after();
-#pragma unroll 1
-      for (int k = 0; k < K1 / 16; ++k)
-        umma_bf16(tmem, umma_desc(sm + SM_X + 2 * k * (TM / 8) * 128, (TM / 8) * 128, 128),
-                  umma_desc(sm + SM_W1 + 2 * k * (H / 8) * 128, (H / 8) * 128, 128), ID1, k > 0);
+      umma_steps<K1 / 16>(tmem, umma_desc(sm + SM_X, (TM / 8) * 128, 128), 2 * (TM / 8) * 128,
+                          umma_desc(sm + SM_W1, (H / 8) * 128, 128), 2 * (H / 8) * 128, ID1);
       umma_commit(&bar_mma[g]);
       cnt[4 + g] += 1u;
     }
@@ -738,18 +738,15 @@ k_mlp_forward_tc(const unsigned char* __restrict__ Xg, const float* __restrict__
         fence_proxy_async_smem();
         tc_fence_before();
         group_sync(g);
-        if (leader) {
+        __syncwarp();
+        if (gw == 0 && elect_one()) {
           tc_fence_after();
           if (layer == 0) {
-#pragma unroll 1
-            for (int k = 0; k < H / 16; ++k)
-              umma_bf16(tmem, umma_desc(Hs + 2 * k * (TM / 8) * 128, (TM / 8) * 128, 128),
-                        umma_desc(sm + SM_W2 + 2 * k * (H / 8) * 128, (H / 8) * 128, 128), ID1, k > 0);
+            umma_steps<H / 16>(tmem, umma_desc(Hs, (TM / 8) * 128, 128), 2 * (TM / 8) * 128,
+                               umma_desc(sm + SM_W2, (H / 8) * 128, 128), 2 * (H / 8) * 128, ID1);
           } else {
-#pragma unroll 1
-            for (int k = 0; k < H / 16; ++k)
-              umma_bf16(tmem + 128, umma_desc(Hs + 2 * k * (TM / 8) * 128, (TM / 8) * 128, 128),
-                        umma_desc(sm + SM_W3 + 2 * k * (N3P / 8) * 128, (N3P / 8) * 128, 128), ID3, k > 0);
+            umma_steps<H / 16>(tmem + 128, umma_desc(Hs, (TM / 8) * 128, 128), 2 * (TM / 8) * 128,
+                               umma_desc(sm + SM_W3, (N3P / 8) * 128, 128), 2 * (N3P / 8) * 128, ID3);
           }
           umma_commit(&bar_mma[g]);
           cnt[4 + g] += 1u;
@@ -1058,10 +1055,8 @@ k_mlp_train_tc(const bf16* __restrict__ Xg, const float* __restrict__ Tg, const 
     if (!ok) break;
     // layer 1: Z1 = X W1
     if (tid == 0) {
-#pragma unroll 1
-      for (int k = 0; k < K1 / 16; ++k)
-        umma_bf16(tmem + T_Z1, umma_desc(sm + TS_X + 2 * k * CM, CM, 128),
-                  umma_desc(sm + TS_H1 + 2 * k * (H / 8) * 128, (H / 8) * 128, 128), IDK, k > 0);
+      umma_steps<K1 / 16>(tmem + T_Z1, umma_desc(sm + TS_X, CM, 128), 2 * CM,
+                          umma_desc(sm + TS_H1, (H / 8) * 128, 128), 2 * (H / 8) * 128, IDK);
       umma_commit(bar);
     }
     if (!(ok = train_wait(bar, ph))) break;
@@ -1081,10 +1076,8 @@ k_mlp_train_tc(const bf16* __restrict__ Xg, const float* __restrict__ Tg, const 
     train_sync();
     // layer 2: Z2 = H1 W2
     if (tid == 0) {
-#pragma unroll 1
-      for (int k = 0; k < H / 16; ++k)
-        umma_bf16(tmem + T_Z2, umma_desc(sm + TS_H1 + 2 * k * CM, CM, 128),
-                  umma_desc(sm + TS_W2 + 2 * k * (H / 8) * 128, (H / 8) * 128, 128), IDK, k > 0);
+      umma_steps<H / 16>(tmem + T_Z2, umma_desc(sm + TS_H1, CM, 128), 2 * CM,
+                         umma_desc(sm + TS_W2, (H / 8) * 128, 128), 2 * (H / 8) * 128, IDK);
       umma_commit(bar);
     }
     if (!(ok = train_wait(bar, ph))) break;
@@ -1103,10 +1096,8 @@ k_mlp_train_tc(const bf16* __restrict__ Xg, const float* __restrict__ Tg, const 
     train_sync();
     // layer 3: Y = H2 W3
     if (tid == 0) {
-#pragma unroll 1
-      for (int k = 0; k < H / 16; ++k)
-        umma_bf16(tmem + T_Y, umma_desc(sm + TS_H2 + 2 * k * CM, CM, 128),
-                  umma_desc(sm + TS_D + 2 * k * (N3P / 8) * 128, (N3P / 8) * 128, 128), ID3, k > 0);
+      umma_steps<H / 16>(tmem + T_Y, umma_desc(sm + TS_H2, CM, 128), 2 * CM,
+                         umma_desc(sm + TS_D, (N3P / 8) * 128, 128), 2 * (N3P / 8) * 128, ID3);
       umma_commit(bar);
     }
     if (!(ok = train_wait(bar, ph))) break;
@@ -1169,22 +1160,23 @@ k_mlp_train_tc(const bf16* __restrict__ Xg, const float* __restrict__ Tg, const 
     train_sync();
     // dW3 = H2^T dY, dH1 = dZ2 W2^T, dW2 = H1^T dZ2, each from the hi and the lo part
     if (tid == 0) {
-#pragma unroll 1
+      const uint64_t dh2 = umma_desc(sm + TS_H2, 128, CM), dw2 = umma_desc(sm + TS_W2, 128, CM);
+      const uint64_t dh1 = umma_desc(sm + TS_H1, 128, CM);
+      const uint64_t ddy[2] = {umma_desc(sm + TS_Y, (N3P / 8) * 128, 128), umma_desc(sm + TS_YLO, (N3P / 8) * 128, 128)};
+      const uint64_t ddzk[2] = {umma_desc(sm + TS_D, CM, 128), umma_desc(sm + TS_DLO, CM, 128)};
+      const uint64_t ddz[2] = {umma_desc(sm + TS_D, 128, CM), umma_desc(sm + TS_DLO, 128, CM)};
+#pragma unroll
       for (int k = 0; k < TBT / 16; ++k)
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
-          const unsigned char* dz = sm + (part ? TS_DLO : TS_D);
-          const unsigned char* dy = sm + (part ? TS_YLO : TS_Y);
           const unsigned acc = (k > 0 || part > 0) ? 1u : 0u;
+          const unsigned st = 2u * k * 128 / 16;  // MN-major operands: two core-matrix lines per step
           // A: H2 with the samples along K (MN-major); B: the dY tile (K-major)
-          umma_bf16(tmem + T_Y, umma_desc(sm + TS_H2 + 2 * k * 128, 128, CM),
-                    umma_desc(dy + 2 * k * (N3P / 8) * 128, (N3P / 8) * 128, 128), IDW3, acc);
+          umma_bf16(tmem + T_Y, dh2 + st, ddy[part] + 2u * k * (N3P / 8) * 128 / 16, IDW3, acc);
           // A: dZ2 (K = hidden column o, K-major); B: the W2 tile (rows o) read with N = i (MN-major)
-          umma_bf16(tmem + T_Z2, umma_desc(dz + 2 * k * CM, CM, 128), umma_desc(sm + TS_W2 + 2 * k * 128, 128, CM),
-                    IDH, acc);
+          umma_bf16(tmem + T_Z2, ddzk[part] + 2u * k * CM / 16, dw2 + st, IDH, acc);
           // A: H1, B: dZ2, both with the samples along K (MN-major)
-          umma_bf16(tmem + T_DW2, umma_desc(sm + TS_H1 + 2 * k * 128, 128, CM), umma_desc(dz + 2 * k * 128, 128, CM),
-                    IDW, acc);
+          umma_bf16(tmem + T_DW2, dh1 + st, ddz[part] + st, IDW, acc);
         }
       umma_commit(bar);
     }
@@ -1231,16 +1223,16 @@ k_mlp_train_tc(const bf16* __restrict__ Xg, const float* __restrict__ Tg, const 
     }
     // dW1 = X^T dZ1: rows k 0..127 (X chunks 0..15) and 80..207 (chunks 10..25)
     if (tid == 0) {
-#pragma unroll 1
+      const uint64_t dx0 = umma_desc(sm + TS_X, 128, CM), dx1 = umma_desc(sm + TS_X + 10 * CM, 128, CM);
+      const uint64_t ddz[2] = {umma_desc(sm + TS_D, 128, CM), umma_desc(sm + TS_DLO, 128, CM)};
+#pragma unroll
       for (int k = 0; k < TBT / 16; ++k)
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
-          const unsigned char* dz = sm + (part ? TS_DLO : TS_D);
           const unsigned acc = (k > 0 || part > 0) ? 1u : 0u;
-          umma_bf16(tmem + T_Z1, umma_desc(sm + TS_X + 2 * k * 128, 128, CM), umma_desc(dz + 2 * k * 128, 128, CM),
-                    IDW, acc);
-          umma_bf16(tmem + T_Z2, umma_desc(sm + TS_X + 10 * CM + 2 * k * 128, 128, CM),
-                    umma_desc(dz + 2 * k * 128, 128, CM), IDW, acc);
+          const unsigned st = 2u * k * 128 / 16;
+          umma_bf16(tmem + T_Z1, dx0 + st, ddz[part] + st, IDW, acc);
+          umma_bf16(tmem + T_Z2, dx1 + st, ddz[part] + st, IDW, acc);
         }
       umma_commit(bar);
     }
