@@ -317,20 +317,28 @@ __device__ __forceinline__ cplx<T> tw_at(const TwLane<T, N, E>& tw, int n, int p
 }
 
 // The three stages of a length N = 12 R2 R3 (see Len12); without PAD the slots are a + R3 c + NT k1.
+// A row buffer (PAD) serves NT lanes of a warp; lanes past its last whole row (360: NT = 30, lanes 30
+// and 31) run along as copies of a row's first lanes.  They only read it: stage 2 replaces the values
+// it has read, with no barrier in between, so a copy that is not in step with the lane it repeats
+// would transform values already transformed.
 template <typename T, int N, bool INV, bool PAD, class Tw, class Sync>
 __device__ __forceinline__ void fft_run_12(cplx<T>* a, cplx<T>* sbuf, int sstride, int j, const Tw& tw, Sync sync) {
   using L = Len12<T, N>;
   constexpr int NT = L::NT, R2 = L::R2, R3 = L::R3, Q2 = (12 + R2 - 1) / R2, Q3 = 12 / R3;
   auto S = [](int k1) { return PAD ? L::PITCH * k1 + (k1 >> L::SH) : NT * k1; };
+  bool own = true;
+  if constexpr (PAD && 32 % NT != 0) own = (int)(threadIdx.x & 31) < 32 / NT * NT;
   dft3p<T, 4, INV>(a);
+  if (own) {
 #pragma unroll
-  for (int k = 0; k < 12; ++k)
-    sbuf[(S(k) + j) * sstride] = k ? cmul(a[k], tw_at<T, N, 12, INV>(tw, k - 1, j * k)) : a[k];
+    for (int k = 0; k < 12; ++k)
+      sbuf[(S(k) + j) * sstride] = k ? cmul(a[k], tw_at<T, N, 12, INV>(tw, k - 1, j * k)) : a[k];
+  }
   sync();
 #pragma unroll
   for (int q = 0; q < Q2; ++q) {
     const int u = j + NT * q;
-    if (Q2 * R2 == 12 || u < 12 * R3) {
+    if (own && (Q2 * R2 == 12 || u < 12 * R3)) {
       const int i = u % R3;
       cplx<T>* p = sbuf + (S(u / R3) + i) * sstride;
       cplx<T> x[R2];
