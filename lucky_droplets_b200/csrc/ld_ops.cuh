@@ -80,9 +80,12 @@ template <typename T, int N> struct Ops {
       if constexpr (PAIRS) return colpass2<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
       else return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
     } else {
-      // untuned plans: one-shot tiles for short columns (right-hand side at 128^3 FP64 105 -> 95 us), except
-      // with two columns per thread (FP32 58 -> 61 us)
-      if (choice == 0 || (choice < 0 && N <= 128 && !PAIRS) || cdiv(ncols, TB) * (long long)nf * nouter >= (1LL << 31)) {
+      // untuned plans: one-shot tiles for short columns (right-hand side at 128^3 FP64 96 us, 104 with the
+      // pipelined pass; 16 boxes of it 1430 and 1480 us, 16 boxes of 96^3 758 and 830 us), except with two
+      // columns per thread (FP32 58 -> 61 us).  Their grid has the outer index as its second dimension,
+      // 65535 at most (682 boxes of 96^3); beyond it the pipelined pass, whose grid is linear, takes over.
+      const bool one_shot = choice == 0 || (choice < 0 && N <= 128 && !PAIRS);
+      if ((one_shot && nouter <= 65535) || cdiv(ncols, TB) * (long long)nf * nouter >= (1LL << 31)) {
         if constexpr (PAIRS) return colpass2<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
         else return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
       }

@@ -70,3 +70,23 @@ def test_large_grids_fp32_against_fp64(torch, N):
     ref = p64.velocity_rhs(uk.to(torch.complex128), 0.01, 1.0, (1, 2))
     assert float(torch.linalg.norm(got - ref) / torch.linalg.norm(ref)) < TOL
     assert np.isfinite(float(got.abs().max()))
+
+
+@pytest.mark.parametrize("tuning", [None, [0, 0]])
+def test_y_passes_of_more_planes_than_a_grid_dimension(torch, tuning):
+    """683 boxes of 96^3 are 65,568 outer indices of the y passes, more than a second grid dimension
+    takes: the same values as a box alone, whose y passes are one-shot tiles."""
+    from lucky_droplets_b200.spectral import Plan
+    torch.cuda.empty_cache()
+    N, nbox = 96, 683
+    many, one = Plan(N, "f64", nbox=nbox), Plan(N, "f64")
+    if tuning:
+        many.set_tuning(tuning)
+    uk = torch.zeros((nbox, 3, one.Mx, one.My, one.Mzp), dtype=one.cdtype, device="cuda")
+    for b in (0, nbox - 1):
+        uk[b] = _state(torch, one, b)
+    ku = torch.zeros_like(uk)
+    many.velocity_rhs(uk, 0.01, 1.0, (1, 2), ku=ku)
+    for b in (0, nbox - 1):
+        assert torch.equal(ku[b], one.velocity_rhs(uk[b].contiguous(), 0.01, 1.0, (1, 2)))
+    assert not torch.view_as_real(ku[1:-1]).any()
