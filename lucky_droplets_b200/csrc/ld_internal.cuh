@@ -104,7 +104,9 @@ cudaError_t launch_dep(bool early, void (*kernel)(KArgs...), dim3 grid, int bloc
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // returned here: the next launch check must not find it again
+  return e;
 }
 
 // Launch sequences of one (precision, N) instance; every pointer is a device pointer.

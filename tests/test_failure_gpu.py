@@ -124,3 +124,19 @@ def test_wait_timeout_in_tensor_core_forward(torch):
     assert p.status() == 0
     torch.cuda.synchronize()
     assert torch.equal(before, after)
+
+
+def test_a_refused_launch_is_reported_once(torch):
+    """More components than a grid dimension takes: the call returns the launch's error, and the next
+    launches, this library's or another's, do not find it again."""
+    from lucky_droplets_b200._lib import LDError
+    from lucky_droplets_b200.spectral import Plan
+    torch.cuda.empty_cache()
+    p = Plan(16, "f32")
+    u = torch.zeros((65536, 16, 16, 16), dtype=torch.float32, device="cuda")
+    fu = torch.zeros((65536, 16, 16, 9), dtype=torch.complex64, device="cuda")
+    torch.cuda.synchronize()
+    with pytest.raises(LDError, match="invalid"):
+        p.rfft_mpi(u, fu)
+    u[0].fill_(1.0)
+    assert float(p.rfft_mpi(u[:2].contiguous())[0, 0, 0, 0].real) == 16.0 ** 3
