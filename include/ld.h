@@ -177,7 +177,9 @@ LD_API int ld_rk4_stage(ld_plan* plan, int stage, void* uk, void* y, void* acc, 
 /* Autotuner of the plan's strided-row (y) transform passes (no counterpart in the reference):
  * times each launch variant on the plan's workspace - ms[8] = [inverse, forward] x [one-shot
  * tiles, pipelined with 1, 2, 3 CTAs per SM] (-1: not available) - and keeps the fastest;
- * choice[2] receives it (0 one-shot, k pipelined with k CTAs per SM).  Synchronises the stream.
+ * choice[2] receives it (0 one-shot, k pipelined with k CTAs per SM).  Grids of 16, 32, 64 and FP32
+ * 96, whose right-hand side has no separate y pass, have nothing to time: ms all -1, choice 0.
+ * Synchronises the stream.
  * ld_plan_set_tuning applies a choice found on another plan of the same N and precision. */
 LD_API int ld_plan_autotune(ld_plan* plan, double* ms, int32_t* choice, void* stream);
 LD_API int ld_plan_set_tuning(ld_plan* plan, const int32_t* choice);

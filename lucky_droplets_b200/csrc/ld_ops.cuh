@@ -264,7 +264,18 @@ template <typename T, int N> struct Ops {
   }
 
   // ---- autotuner of the y passes: every launch variant timed on the plan's workspace ------------
+  // (none where the right-hand side takes the plane pass: no y pass is launched)
   static int autotune(ld_plan* p, cudaStream_t s, double* ms) {
+    if constexpr (PlaneCfg<T, N>::OK) {
+      for (int v = 0; v < 8; ++v) ms[v] = -1.0;
+      p->tune_y[0] = p->tune_y[1] = 0;
+      LD_CUDA_CHECK(cudaStreamSynchronize(s));
+      return LD_OK;
+    } else {
+      return autotune_y(p, s, ms);
+    }
+  }
+  static int autotune_y(ld_plan* p, cudaStream_t s, double* ms) {
     const int My = p->My, Mzp = p->Mzp, kc = p->kc;
     const C* tw = (const C*)p->tw;
     C* W1 = (C*)p->W1;

@@ -177,7 +177,8 @@ class Plan:
 
     def autotune(self, stream=None):
         """Time every launch variant of the y passes on this plan and keep the fastest; returns
-        {"ms": {pass: [one-shot, pipelined 1..3 CTAs/SM]}, "choice": [inverse, forward]}."""
+        {"ms": {pass: [one-shot, pipelined 1..3 CTAs/SM]}, "choice": [inverse, forward]} (ms -1: no
+        such variant; none at all for 16, 32, 64 and FP32 96, which have no separate y pass)."""
         ms = (ctypes.c_double * 8)()
         ch = (ctypes.c_int32 * 2)()
         check(_lib.lib().ld_plan_autotune(self._h, ms, ch, stream_ptr(stream)))

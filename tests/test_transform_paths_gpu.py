@@ -90,3 +90,22 @@ def test_y_passes_of_more_planes_than_a_grid_dimension(torch, tuning):
     for b in (0, nbox - 1):
         assert torch.equal(ku[b], one.velocity_rhs(uk[b].contiguous(), 0.01, 1.0, (1, 2)))
     assert not torch.view_as_real(ku[1:-1]).any()
+
+
+@pytest.mark.parametrize("N,prec,nbox", [(64, "f32", 1), (96, "f32", 1), (16, "f64", 4096)])
+def test_autotune_where_the_plane_pass_runs(torch, N, prec, nbox):
+    """Grids whose right-hand side takes the plane pass have no y pass to time."""
+    from lucky_droplets_b200.spectral import Plan
+    p = Plan(N, prec, nbox=nbox)
+    assert p.autotune() == {"ms": {"inverse_y": [-1.0] * 4, "forward_y": [-1.0] * 4}, "choice": [0, 0]}
+
+
+@pytest.mark.parametrize("N,prec", [(96, "f64"), (128, "f32"), (128, "f64"), (192, "f64"), (360, "f32")])
+def test_y_pass_variants_give_identical_rhs(torch, N, prec):
+    from lucky_droplets_b200.spectral import Plan
+    p = Plan(N, prec)
+    uk = _state(torch, p, N)
+    ref = p.velocity_rhs(uk, 0.01, 1.0, (1, 2)).clone()
+    for choice in ([0, 0], [1, 1], [3, 3]):
+        p.set_tuning(choice)
+        assert torch.equal(p.velocity_rhs(uk, 0.01, 1.0, (1, 2)), ref)
