@@ -109,3 +109,55 @@ def test_y_pass_variants_give_identical_rhs(torch, N, prec):
     for choice in ([0, 0], [1, 1], [3, 3]):
         p.set_tuning(choice)
         assert torch.equal(p.velocity_rhs(uk, 0.01, 1.0, (1, 2)), ref)
+
+
+class _Guarded:
+    """A tensor `off` bytes past a 16-byte boundary between two stretches of NaN."""
+
+    def __init__(self, torch, shape, dtype, off):
+        n, item = int(np.prod(shape)), torch.empty(0, dtype=dtype).element_size()
+        self.torch, self.lo = torch, 64 + off // item
+        self.hi = self.lo + n
+        self.all = torch.full((self.hi + 64,), complex("nan+nanj"), dtype=dtype, device="cuda")
+        self.t = self.all[self.lo:self.hi].view(shape)
+        assert self.t.data_ptr() % 16 == off
+
+    def intact(self):
+        ends = self.torch.cat([self.all[:self.lo], self.all[self.hi:]])
+        return bool(self.torch.isnan(self.torch.view_as_real(ends)).all())
+
+
+@pytest.mark.parametrize("off", [(8, 8, 8), (0, 0, 8), (8, 0, 0), (0, 8, 0)])
+@pytest.mark.parametrize("N", [64, 128, 256])
+def test_stages_off_the_16_byte_grid_stay_inside(torch, N, off):
+    """RK2 and RK4 stages and the right-hand side with the state, the stage state or the accumulator 8
+    bytes past a 16-byte boundary: the values of aligned buffers to FP32 rounding, and nothing outside
+    the buffers is written, or read and used."""
+    import ctypes
+    from lucky_droplets_b200 import _lib
+    from lucky_droplets_b200._lib import check, ptr, stream_ptr
+    from lucky_droplets_b200.spectral import Plan, flow_params
+    p = Plan(N, "f32")
+    uk = _state(torch, p, N)
+    prm = ctypes.byref(flow_params(1e-3, 0.01, 1.0, (1, 2)))
+
+    def stages(offs, call, count):
+        bufs = [_Guarded(torch, uk.shape, uk.dtype, o) for o in offs]
+        bufs[0].t.copy_(uk)
+        for b in bufs[1:]:
+            b.t.zero_()
+        for s in range(1, count + 1):
+            check(call(p.handle, s, *[ptr(b.t) for b in bufs], None, prm, stream_ptr(None)))
+        assert all(b.intact() for b in bufs)
+        return [b.t for b in bufs]
+
+    L = _lib.lib()
+    for call, count in ((L.ld_rk2if_stage, 2), (L.ld_rk4_stage, 4)):
+        for got, ref in zip(stages(off, call, count), stages((0, 0, 0), call, count)):
+            assert float(torch.linalg.norm(got - ref) / torch.linalg.norm(ref)) < TOL
+    y, ku = (_Guarded(torch, uk.shape, uk.dtype, o) for o in off[:2])
+    y.t.copy_(uk)
+    p.velocity_rhs(y.t, 0.01, 1.0, (1, 2), ku=ku.t)
+    ref = p.velocity_rhs(uk, 0.01, 1.0, (1, 2))
+    assert y.intact() and ku.intact() and torch.equal(y.t, uk)
+    assert float(torch.linalg.norm(ku.t - ref) / torch.linalg.norm(ref)) < TOL
