@@ -14,7 +14,8 @@
 //   wide      droplets with 2 r > cell width ("wide"; none when the cell width is at least twice
 //             the largest radius) also search the cells within 2 r of them for the partners
 //             with ri + rj > cell width, which the neighbour search leaves out: counted by the
-//             warp of the count pass that meets them, emitted by the block of the emit pass
+//             warp of the count pass that meets them (those that reach far: listed by the sort
+//             and counted by blocks of their own), emitted by the block of the emit pass
 //   emit      pairs at offset + t in the fixed visiting order (copied from the record, or searched
 //             again for droplets with more partners), as droplet ids (i < j)
 // The FP64 arithmetic (wrap, cell index, minimum image, squared distance) is done with explicit
@@ -80,10 +81,20 @@ __global__ void k_cell_scatter(const unsigned* __restrict__ key, const unsigned*
     run[cs[key[i]] + rank[i]] = (unsigned)i;
 }
 
+// Sorted droplets whose search reaches three cells and further (far_counts), in no order.
+__device__ __forceinline__ bool reaches_far(double r, double cw) { return r >= cw; }
+struct FarList {
+  double cw;
+  unsigned *list, *count;
+  __device__ __forceinline__ void add(long long s, double r) const {
+    if (reaches_far(r, cw)) list[atomicAdd(count, 1u)] = (unsigned)s;
+  }
+};
+
 // Sorted copies of one sorted slot: cell key, wrapped FP64 position + radius, FP32 copy.
 __device__ __forceinline__ void sorted_slot(long long s, unsigned k, unsigned i, const double* __restrict__ pos,
                                             const double* __restrict__ rad, double L, unsigned* __restrict__ skey,
-                                            double4* __restrict__ sp, float4* __restrict__ spf) {
+                                            double4* __restrict__ sp, float4* __restrict__ spf, const FarList& far) {
   double4 q;
   q.x = wrapL(pos[3 * (long long)i], L);
   q.y = wrapL(pos[3 * (long long)i + 1], L);
@@ -92,6 +103,7 @@ __device__ __forceinline__ void sorted_slot(long long s, unsigned k, unsigned i,
   skey[s] = k;
   sp[s] = q;
   spf[s] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
+  far.add(s, q.w);
 }
 
 constexpr int kSmallCell = 64;  // cells up to this occupancy are placed by rank counting
@@ -106,7 +118,7 @@ __global__ void k_cell_place(const unsigned* __restrict__ key, const int* __rest
                              const unsigned* __restrict__ run, long long n, const double* __restrict__ pos,
                              const double* __restrict__ rad, double L, unsigned* __restrict__ sval,
                              unsigned* __restrict__ skey, double4* __restrict__ sp, float4* __restrict__ spf,
-                             unsigned* __restrict__ big, unsigned* __restrict__ nbig) {
+                             unsigned* __restrict__ big, unsigned* __restrict__ nbig, FarList far) {
   ld::grid_dep();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
     const unsigned i = run[t];
@@ -120,7 +132,7 @@ __global__ void k_cell_place(const unsigned* __restrict__ key, const int* __rest
     for (int j = s0; j < s1; ++j) r += run[j] < i ? 1 : 0;
     const int s = s0 + r;
     sval[s] = i;
-    sorted_slot(s, k, i, pos, rad, L, skey, sp, spf);
+    sorted_slot(s, k, i, pos, rad, L, skey, sp, spf, far);
   }
 }
 
@@ -130,7 +142,8 @@ __global__ void k_cell_place(const unsigned* __restrict__ key, const int* __rest
 __global__ void __launch_bounds__(512)
 k_cell_big(const int* __restrict__ cs, const unsigned* __restrict__ big, const unsigned* __restrict__ nbig,
            unsigned* __restrict__ run, const double* __restrict__ pos, const double* __restrict__ rad, double L,
-           unsigned* __restrict__ sval, unsigned* __restrict__ skey, double4* __restrict__ sp, float4* __restrict__ spf) {
+           unsigned* __restrict__ sval, unsigned* __restrict__ skey, double4* __restrict__ sp, float4* __restrict__ spf,
+           FarList far) {
   ld::grid_dep();
   const unsigned nb = *nbig;
   for (unsigned b = blockIdx.x; b < nb; b += gridDim.x) {
@@ -154,7 +167,7 @@ k_cell_big(const int* __restrict__ cs, const unsigned* __restrict__ big, const u
     }
     for (int x = threadIdx.x; x < m; x += blockDim.x) {
       sval[s0 + x] = v[x];
-      sorted_slot(s0 + x, k, v[x], pos, rad, L, skey, sp, spf);
+      sorted_slot(s0 + x, k, v[x], pos, rad, L, skey, sp, spf, far);
     }
     __syncthreads();
   }
@@ -306,7 +319,7 @@ __global__ void k_cell_starts(const unsigned* __restrict__ skey, long long n, lo
 
 __global__ void k_sorted_copy(const double* __restrict__ pos, const double* __restrict__ rad,
                               const unsigned* __restrict__ sval, long long n, double L, double4* __restrict__ sp,
-                              float4* __restrict__ spf) {
+                              float4* __restrict__ spf, FarList far) {
   for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < n; s += (long long)gridDim.x * blockDim.x) {
     const unsigned i = sval[s];
     double4 q;
@@ -316,6 +329,7 @@ __global__ void k_sorted_copy(const double* __restrict__ pos, const double* __re
     q.w = rad[i];
     sp[s] = q;
     spf[s] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
+    far.add(s, q.w);
   }
 }
 
@@ -446,9 +460,9 @@ constexpr int KEEP = 16;  // partners recorded per droplet (more: searched again
 // smaller sorted index), which is wide.  The owner s searches every cell within R = floor(2 rs /
 // cw) + 1 cells of its own along each axis (all nc when 2 R + 1 >= nc), since its partner is closer
 // than rs + rt <= 2 rs.  The owner's pairs follow the pairs of its neighbour-cell search in its
-// run of the output.  Work items of a wide droplet: the 14 cells of the neighbour search (emit
-// only), then the cells of the wide search in (x, y, z) order; the warp that meets a wide droplet
-// in the count pass, and the block of the emit pass, shares out its items.
+// run of the output.  Work items of a wide droplet: the 14 cells of the neighbour search (left out by
+// a warp of the count pass, which has searched them), then the cells of the wide search in (x, y, z)
+// order, shared out to the threads of a warp or a block.
 
 // droplet ids (i, j), i < j, at place o of the pair list
 __device__ __forceinline__ void put_pair(int* __restrict__ pairs, long long o, long long cap, unsigned a, unsigned b) {
@@ -549,18 +563,65 @@ __device__ unsigned wide_count(int s, const double4* __restrict__ sp, const floa
   return total;
 }
 
+// The partners of the droplets that reach far, neighbour search included, a block per droplet.  They
+// search 7^3 cells and more, which keeps the one warp that meets them in its own search long after the
+// rest of the pass is done, and few blocks may meet them all.  Whole search of 3e5 droplets in 120^3
+// cells, one warp each and a block each: 300 of 20 times the radius of the rest 1070 and 378 us, a
+// single one of 60 times 6570 and 2900 us; 1000 droplets that all reach seven cells 4320 and 1680 us;
+// without such droplets 70 us either way.  With the line at four cells, 3e5 droplets of lognormal radii
+// in 13^3 cells take 1980 instead of 1430 us; at two cells, 1e6 droplets that all reach two 5.9 ms
+// instead of 3.1.
+constexpr int kFarBlocks = 8 * kSMs;
+__device__ void far_counts(unsigned block, unsigned nblocks, const FarList& far, const double4* __restrict__ sp,
+                           const float4* __restrict__ spf, const unsigned* __restrict__ skey,
+                           const int* __restrict__ cs, int nc, double L, unsigned* __restrict__ cnt,
+                           int* __restrict__ scr, unsigned* sums) {
+  const float Lf = (float)L, hf = 0.5f * Lf, margin = (float)(1e-6 * L);
+  const unsigned n = *far.count;
+  for (unsigned e = block; e < n; e += nblocks) {
+    const int s = (int)far.list[e];
+    const double4 me = sp[s];
+    const float4 mf = spf[s];
+    const WideCell w = wide_cell(skey[s], nc, me.w, far.cw);
+    const int items = 14 + w.ax * w.ax * w.ax;
+    unsigned c = 0, total;
+    for (int it = (int)threadIdx.x; it < items; it += VISIT_THREADS)
+      c += wide_item<false>(it, true, s, w, me, mf, sp, spf, cs, nc, L, far.cw, Lf, hf, margin + 1e-6f * mf.w, nullptr,
+                            nullptr, 0, 0);
+    warp_excl_scan(c, &total);
+    __syncthreads();  // the sums of the droplet before have been read
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      total = 0;
+      for (int q = 0; q < VISIT_THREADS / 32; ++q) total += sums[q];
+      cnt[s] = total;
+      scr[(long long)KEEP * s] = -1;  // the emit pass writes its pairs by wide_emit
+    }
+  }
+}
+
+// The first fblocks blocks count the droplets that reach far, the others search for the rest.
 __global__ void __launch_bounds__(VISIT_THREADS, VISIT_BLOCKS)
 k_visit(const double4* __restrict__ sp, const float4* __restrict__ spf, const unsigned* __restrict__ skey,
         const int* __restrict__ cs, int nc, double L, double cw, int n, unsigned* __restrict__ cnt,
-        int* __restrict__ scr) {
+        int* __restrict__ scr, FarList far, unsigned fblocks) {
   ld::grid_dep();
   __shared__ int queue[KEEP][VISIT_THREADS];
+  if (blockIdx.x < fblocks) {
+    far_counts(blockIdx.x, fblocks, far, sp, spf, skey, cs, nc, L, cnt, scr, reinterpret_cast<unsigned*>(&queue[0][0]));
+    return;
+  }
   const int tid = threadIdx.x;
   unsigned c = 0;     // partners confirmed (the first KEEP in scr)
   bool wide = false;  // partners beyond the neighbour cells, counted by the warp below
-  const long long ii = (long long)blockIdx.x * VISIT_THREADS + tid;
+  const long long ii = (long long)(blockIdx.x - fblocks) * VISIT_THREADS + tid;
   if (ii == 0) cnt[n] = 0u;
-  if (ii < n) {
+  // wide droplets: FP32 radius first (rounding is monotone, r > cw / 2 implies float(r) >= float(cw / 2))
+  double r = 0.0;
+  if (ii < n && spf[ii].w >= (float)(0.5 * cw)) r = sp[ii].w;
+  if (ii < n && !reaches_far(r, cw)) {
+    wide = r > 0.5 * cw;
     const int i = (int)ii;
     const float Lf = (float)L, margin = (float)(1e-6 * L);
     // home cell: column (box, cx, cy) and height
@@ -638,8 +699,6 @@ k_visit(const double4* __restrict__ sp, const float4* __restrict__ spf, const un
     }
     flush();
     cnt[i] = c;
-    // FP32 radius first: rounding is monotone, r > cw / 2 implies float(r) >= float(cw / 2)
-    wide = mf.w >= (float)(0.5 * cw) && sp[i].w > 0.5 * cw;
   }
   for (unsigned m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1) {
     const int src = __ffs(m) - 1;
@@ -789,7 +848,9 @@ struct ld_collider {
   float4* spf = nullptr;
   int* scr = nullptr;  // first KEEP partners of each sorted droplet
   unsigned* status = nullptr;
-  unsigned* nbig = nullptr;  // number of cells above kSmallCell droplets (counting sort)
+  // number of cells above kSmallCell droplets (counting sort), number of droplets that reach far
+  unsigned* nbig = nullptr;
+  unsigned* far = nullptr;  // the latter's sorted indices
   unsigned* sums = nullptr;  // scan tile totals
   int nblocks = 0;
   ld_plan* trace = nullptr;  // plan whose event trace records this collider's launches
@@ -835,7 +896,8 @@ int ld_collider_create_boxes(ld_collider** out, int64_t nmax, int32_t nc, int32_
   A((void**)&c->spf, sizeof(float4) * nmax);
   A((void**)&c->scr, sizeof(int) * KEEP * nmax);
   A((void**)&c->status, sizeof(unsigned));
-  A((void**)&c->nbig, sizeof(unsigned));
+  A((void**)&c->nbig, 2 * sizeof(unsigned));
+  A((void**)&c->far, 4 * nmax);
   {
     long long m = (nmax + 1) > (long long)RADIX * c->nblocks ? (nmax + 1) : (long long)RADIX * c->nblocks;
     if (ncell + 1 > m) m = ncell + 1;
@@ -856,6 +918,7 @@ int ld_collider_destroy(ld_collider* c) {
   cudaFree(c->key); cudaFree(c->val); cudaFree(c->key2); cudaFree(c->val2); cudaFree(c->hist);
   cudaFree(c->cnt); cudaFree(c->start); cudaFree(c->sp); cudaFree(c->spf); cudaFree(c->scr); cudaFree(c->status);
   cudaFree(c->nbig);
+  cudaFree(c->far);
   cudaFree(c->sums);
   delete c;
   return LD_OK;
@@ -906,8 +969,10 @@ int ld_collide_boxes(ld_collider* c, const double* pos, const double* radius, co
     LD_CUDA_CHECK(cudaMemsetAsync(count, 0, sizeof(int64_t), s));
     return LD_OK;
   }
+  const FarList far{cw, c->far, c->nbig + 1};
   {
     ProfScope ps(c->trace, KID_COLL_SORT, s);
+    LD_CUDA_CHECK(cudaMemsetAsync(c->nbig, 0, 2 * sizeof(unsigned), s));
     if (ncell + 1 > (long long)SCAN_TILE * SCAN_TILE) {
       // more cells than one scan handles: stable radix sort of the keys, starts by binary search
       k_cell_keys<<<gridn(n, 256), 256, 0, s>>>(pos, n, L, cw, nc, c->key, c->val, box);
@@ -915,7 +980,7 @@ int ld_collide_boxes(ld_collider* c, const double* pos, const double* radius, co
       while ((1LL << bits) < ncell) ++bits;
       if (int rc = ld_radix_sort_u32(c, c->key, c->val, n, bits, stream)) return rc;
       k_cell_starts<<<gridn(ncell + 1, 256), 256, 0, s>>>(c->key, n, ncell, c->start);
-      k_sorted_copy<<<gridn(n, 256), 256, 0, s>>>(pos, radius, c->val, n, L, c->sp, c->spf);
+      k_sorted_copy<<<gridn(n, 256), 256, 0, s>>>(pos, radius, c->val, n, L, c->sp, c->spf, far);
     } else {
       // counting sort by cell (the same order): keys (c->key2) and arrival ranks (c->val2),
       // occupancies -> starts in c->start, unordered runs scattered into c->cnt, then every
@@ -923,22 +988,23 @@ int ld_collide_boxes(ld_collider* c, const double* pos, const double* radius, co
       // copies (cells above kSmallCell: listed in c->val2, sorted by k_cell_big)
       unsigned* occ = reinterpret_cast<unsigned*>(c->start);
       LD_CUDA_CHECK(cudaMemsetAsync(occ, 0, sizeof(unsigned) * (size_t)(ncell + 1), s));
-      LD_CUDA_CHECK(cudaMemsetAsync(c->nbig, 0, sizeof(unsigned), s));
       LD_CUDA_CHECK(launch_dep(true, k_cell_count, dim3(gridn(n, 256)), 256, 0, s, pos, n, L, cw, nc, c->key2, c->val2,
                                occ, box));
       if (int rc = scan_u32(c, occ, ncell + 1, s)) return rc;
       LD_CUDA_CHECK(launch_dep(true, k_cell_scatter, dim3(gridn(n, 256)), 256, 0, s, c->key2, c->val2, c->start, n,
                                c->cnt));
       LD_CUDA_CHECK(launch_dep(true, k_cell_place, dim3(gridn(n, 256)), 256, 0, s, c->key2, c->start, c->cnt, n, pos,
-                               radius, L, c->val, c->key, c->sp, c->spf, c->val2, c->nbig));
+                               radius, L, c->val, c->key, c->sp, c->spf, c->val2, c->nbig, far));
       LD_CUDA_CHECK(launch_dep(true, k_cell_big, dim3(kSMs), 512, 0, s, c->start, c->val2, c->nbig, c->cnt, pos, radius,
-                               L, c->val, c->key, c->sp, c->spf));
+                               L, c->val, c->key, c->sp, c->spf, far));
     }
   }
   ProfScope ps(c->trace, KID_COLL_PAIRS, s);
   if (nc >= 3) {
-    LD_CUDA_CHECK(launch_dep(true, k_visit, dim3((unsigned)((n + VISIT_THREADS - 1) / VISIT_THREADS)), VISIT_THREADS, 0,
-                             s, c->sp, c->spf, c->key, c->start, nc, L, cw, (int)n, c->cnt, c->scr));
+    const unsigned fblocks = (unsigned)(n < kFarBlocks ? n : kFarBlocks);
+    LD_CUDA_CHECK(launch_dep(true, k_visit, dim3(fblocks + (unsigned)((n + VISIT_THREADS - 1) / VISIT_THREADS)),
+                             VISIT_THREADS, 0, s, c->sp, c->spf, c->key, c->start, nc, L, cw, (int)n, c->cnt, c->scr,
+                             far, fblocks));
     if (int rc = scan_u32(c, c->cnt, n + 1, s)) return rc;
     LD_CUDA_CHECK(launch_dep(true, k_emit_pairs, dim3((unsigned)((n + EMIT_THREADS - 1) / EMIT_THREADS)), EMIT_THREADS,
                              0, s, c->sp, c->spf, c->key, c->val, c->start, nc, L, cw, (int)n, c->cnt, c->scr, pairs,

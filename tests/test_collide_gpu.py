@@ -331,3 +331,21 @@ def test_narrow_cells_multi_box_and_overflow(torch):
 def _lib_status_overflow():
     from lucky_droplets_b200 import _lib
     return _lib.STATUS_PAIR_OVERFLOW
+
+
+# wide droplets that reach two cells (counted by a warp), three and four (by a block), the whole box; more
+# of them than blocks that count them; more cells than the counting sort takes (sorted copies after the
+# radix sort)
+@pytest.mark.parametrize("n,nc,radii", [(5000, 40, (0.15, 0.158, 0.18)), (3000, 40, (0.18, 0.25)),
+                                        (2000, 40, (0.01, 1.3)), (3000, 260, (0.02, 0.03, 0.05, 0.001))])
+def test_wide_droplets_by_reach(torch, n, nc, radii):
+    rng = np.random.default_rng(nc + n)
+    pos = rng.uniform(-1.0, TWO_PI + 1.0, (n, 3))
+    rad = np.asarray(radii)[np.arange(n) % len(radii)]
+    if radii[-1] > 1.0:
+        rad = np.where(np.arange(n) < 5, radii[1], radii[0])
+    got, c = gpu_pairs(torch, pos, rad, TWO_PI / (nc + 0.5))
+    assert c.nc == nc
+    ref = K.collide(pos, rad, 2 * rad.max()) if 6 * rad.max() < TWO_PI else K.collide_bruteforce(pos, rad)
+    assert len(ref) > 10
+    assert got.shape == ref.shape and np.array_equal(got, ref)
