@@ -85,12 +85,25 @@ struct ProfScope {
 // prologue, two to three microseconds per launch.  That pays for short kernels only: blocks that
 // become resident beside a long predecessor pin the SM's split of L1 and shared memory (a right-hand
 // side at 32^3 FP64 23.6 -> 14.4 us, at 256^3 FP32 396 -> 442; 1e6 inferences 381 -> 612).  Hence:
-// the flow's passes with at most one x plane per SM (four boxes of 64^3: 637 us for five ensemble
-// steps without, 702 with it), per-droplet passes of at most 1024 droplets per SM, inference of at
-// most one tile per SM; the generic transforms and the collision search always (transforms at 96^3
-// FP64 78 -> 66 us, 256^3 FP32 503 -> 491; 1e6 droplets 228 -> 204 us).
+// - the flow's passes with at most one x plane per SM (four boxes of 64^3: 637 us for five ensemble
+//   steps without, 702 with it), its one-shot y passes up to 384^3 (four boxes of 128^3 FP64: a
+//   right-hand side of 381 us without, 376 with it; 512^3 FP64: 7915 and 8225);
+// - the cube-layout transforms; those in the reference layout up to 300 MB of spectrum (three fields of
+//   192^3 FP64, 172 MB, forward: 216 us without, 209 with it; of 256^3 FP64, 406 MB: 453 and 461;
+//   inverse of 384^3 FP64, 1.4 GB: 1862 and 1904);
+// - per-droplet passes: early_droplets; inference of at most one tile per two SMs, so that the feature
+//   and the forward kernel find SMs of their own (9000 droplets at 256^3 FP32: 16.5 us without, 12.1
+//   with it; 16,000: 18.6 and 20.2);
+// - the collision search always (1e6 droplets 228 -> 204 us).
 constexpr int kSMs = 148;
-inline bool early_droplets(long long n) { return n <= kSMs * 1024; }
+// Beside the flow's passes of small grids 1024 droplets per SM, 512 for the 64-point stencils;
+// 64 beside those of larger grids, whose blocks hold the shared memory that stencil loads want as L1.
+// A step without and with it: 64^3 FP32, 4e4 tricubic droplets 79 and 75 us, 1e5 trilinear ones 60 and
+// 55; 64^3 FP64, 1e5 tricubic ones 149 and 156; 128^3 FP32, 9000 tricubic droplets 170 and 165, 1e5 of
+// them 194 and 229.
+inline bool early_droplets(const ld_plan* p, long long n, bool stencil64 = false) {
+  return n <= kSMs * ((long long)p->N * p->nbox > 96 ? 64 : (stencil64 ? 512 : 1024));
+}
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dep(bool early, void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t s,
                        Args... args) {

@@ -1480,11 +1480,11 @@ int ld_mlp_infer_ws(ld_plan* p, const void* u4, const double* pos, int64_t n, co
                                          (int)SMEM_FWD));
       {
         ProfScope ps(p, KID_MLP_FEAT, s);
-        LD_CUDA_CHECK(launch_dep(tiles <= kSMs, k_mlp_features<float>, dim3((unsigned)gf), FTHREADS, 0, s, (const float4*)u4, p->N, L,
+        LD_CUDA_CHECK(launch_dep(tiles <= kSMs / 2, k_mlp_features<float>, dim3((unsigned)gf), FTHREADS, 0, s, (const float4*)u4, p->N, L,
                                  pos + 3 * b0, nb, params, (bf16*)X, aux));
       }
       ProfScope ps(p, KID_MLP_INFER, s);
-      LD_CUDA_CHECK(launch_dep(tiles <= kSMs, k_mlp_forward_tc<float>, dim3((unsigned)gm), FT_THREADS, SMEM_FWD, s, X, aux, nb,
+      LD_CUDA_CHECK(launch_dep(tiles <= kSMs / 2, k_mlp_forward_tc<float>, dim3((unsigned)gm), FT_THREADS, SMEM_FWD, s, X, aux, nb,
                                (const bf16*)packed, params, (float*)out + 3 * b0, p->status, p->wait_limit,
                                p->wait_stall));
     } else {
@@ -1492,11 +1492,11 @@ int ld_mlp_infer_ws(ld_plan* p, const void* u4, const double* pos, int64_t n, co
                                          (int)SMEM_FWD));
       {
         ProfScope ps(p, KID_MLP_FEAT, s);
-        LD_CUDA_CHECK(launch_dep(tiles <= kSMs, k_mlp_features<double>, dim3((unsigned)gf), FTHREADS, 0, s, (const double4*)u4, p->N, L,
+        LD_CUDA_CHECK(launch_dep(tiles <= kSMs / 2, k_mlp_features<double>, dim3((unsigned)gf), FTHREADS, 0, s, (const double4*)u4, p->N, L,
                                  pos + 3 * b0, nb, params, (bf16*)X, aux));
       }
       ProfScope ps(p, KID_MLP_INFER, s);
-      LD_CUDA_CHECK(launch_dep(tiles <= kSMs, k_mlp_forward_tc<double>, dim3((unsigned)gm), FT_THREADS, SMEM_FWD, s, X, aux, nb,
+      LD_CUDA_CHECK(launch_dep(tiles <= kSMs / 2, k_mlp_forward_tc<double>, dim3((unsigned)gm), FT_THREADS, SMEM_FWD, s, X, aux, nb,
                                (const bf16*)packed, params, (double*)out + 3 * b0, p->status, p->wait_limit,
                                p->wait_stall));
     }
@@ -1577,8 +1577,8 @@ int ld_droplet_predict(ld_plan* p, const double* pos, const void* vel, int64_t n
   if (!p || n < 0 || (n > 0 && (!pos || !vel || !xs))) return ld_fail(LD_ERR_ARG, "ld_droplet_predict: bad arguments");
   if (n == 0) return LD_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  if (p->prec == LD_F32) LD_CUDA_CHECK(launch_dep(early_droplets(n), k_droplet_predict<float>, dim3(gridn(3 * n, 256)), 256, 0, s, pos, (const float*)vel, n, h, xs));
-  else LD_CUDA_CHECK(launch_dep(early_droplets(n), k_droplet_predict<double>, dim3(gridn(3 * n, 256)), 256, 0, s, pos, (const double*)vel, n, h, xs));
+  if (p->prec == LD_F32) LD_CUDA_CHECK(launch_dep(early_droplets(p, n), k_droplet_predict<float>, dim3(gridn(3 * n, 256)), 256, 0, s, pos, (const float*)vel, n, h, xs));
+  else LD_CUDA_CHECK(launch_dep(early_droplets(p, n), k_droplet_predict<double>, dim3(gridn(3 * n, 256)), 256, 0, s, pos, (const double*)vel, n, h, xs));
   LD_LAUNCH_CHECK();
   return LD_OK;
 }
@@ -1591,10 +1591,10 @@ int ld_droplet_update(ld_plan* p, int stage, const void* up, double* pos, void* 
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope ps(p, stage == 1 ? KID_DROPLET1 : KID_DROPLET2, s);
   if (p->prec == LD_F32)
-    LD_CUDA_CHECK(launch_dep(early_droplets(n), k_droplet_given<float>, dim3(gridn(n, 256)), 256, 0, s, stage, (const float*)up, pos, (float*)vel,
+    LD_CUDA_CHECK(launch_dep(early_droplets(p, n), k_droplet_given<float>, dim3(gridn(n, 256)), 256, 0, s, stage, (const float*)up, pos, (float*)vel,
                              (const float*)tau, (float*)a1, n, h, (float)g));
   else
-    LD_CUDA_CHECK(launch_dep(early_droplets(n), k_droplet_given<double>, dim3(gridn(n, 256)), 256, 0, s, stage, (const double*)up, pos, (double*)vel,
+    LD_CUDA_CHECK(launch_dep(early_droplets(p, n), k_droplet_given<double>, dim3(gridn(n, 256)), 256, 0, s, stage, (const double*)up, pos, (double*)vel,
                              (const double*)tau, (double*)a1, n, h, (double)g));
   LD_LAUNCH_CHECK();
   return LD_OK;

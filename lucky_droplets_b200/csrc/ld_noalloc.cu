@@ -83,13 +83,14 @@ int na_run(const float2* fu, float* u, int ncomp, float2* W, const float2* tw, c
     auto xout = O::io(W, per, 0);
     // the loaders and storers of Ops::irfft_full (plain rows), so both paths run the same kernels
     if (int rc = O::template colpass<true>(nullptr, KID_XPASS, ld::LdRowsC<float, N, false, O::RS::XF>{xin},
-                                           ld::StRowsC<float, N, false, O::RS::XF>{xout}, N * Nf, 1, 1, tw, s))
+                                           ld::StRowsC<float, N, false, O::RS::XF>{xout}, N * Nf, 1, 1, tw, s,
+                                           true))
       return rc;
     auto yio = O::io(W, per, (long long)N * Nf);
     if (int rc = O::template colpass<true>(nullptr, KID_YINV, ld::LdRowsC<float, N, false, O::RS::YF>{yio},
-                                           ld::StRowsC<float, N, false, O::RS::YF>{yio}, Nf, 1, N, tw, s))
+                                           ld::StRowsC<float, N, false, O::RS::YF>{yio}, Nf, 1, N, tw, s, true))
       return rc;
-    if (int rc = O::z_c2r(nullptr, W, u + c * NN * N, NN, Nf, Nf, sc, NN * N, per, 1, tw, s)) return rc;
+    if (int rc = O::z_c2r(nullptr, W, u + c * NN * N, NN, Nf, Nf, sc, NN * N, per, 1, tw, s, true)) return rc;
   }
   return LD_OK;
 }

@@ -42,14 +42,17 @@ template <typename T, int N> struct Ops {
 
   // whether the flow's passes may begin early: at most one x plane per SM (launch_dep)
   static bool early(const ld_plan* p) { return (long long)N * p->nbox <= kSMs; }
+  // and those of a reference-layout transform of so many spectral elements
+  static bool early_transform(long long elems) { return elems * (long long)sizeof(C) <= 300LL << 20; }
 
   template <bool INV, class Ld, class St>
-  static int colpass(ld_plan* p, int kid, Ld ld, St st, int ncols, int nf, int nouter, const C* tw, cudaStream_t s) {
+  static int colpass(ld_plan* p, int kid, Ld ld, St st, int ncols, int nf, int nouter, const C* tw, cudaStream_t s,
+                     bool dep) {
     ProfScope ps(p, kid, s);
     auto k = colfft_kernel<T, N, INV, Ld, St>();
     if (int rc = set_smem(k, COL_SMEM)) return rc;
     dim3 grid((unsigned)(cdiv(ncols, TB) * nf), (unsigned)nouter);
-    LD_CUDA_CHECK(launch_dep(true, k, grid, Cfg<N>::COL_THREADS, COL_SMEM, s, ld, st, ncols, nf, tw));
+    LD_CUDA_CHECK(launch_dep(dep, k, grid, Cfg<N>::COL_THREADS, COL_SMEM, s, ld, st, ncols, nf, tw));
     return LD_OK;
   }
 
@@ -78,7 +81,7 @@ template <typename T, int N> struct Ops {
     const int choice = variant != -2 ? variant : p->tune_y[INV ? 0 : 1];
     if constexpr (!PIPE) {
       if constexpr (PAIRS) return colpass2<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
-      else return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
+      else return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s, N <= 384);
     } else {
       // untuned plans: one-shot tiles for short columns (right-hand side at 128^3 FP64 96 us, 104 with the
       // pipelined pass; 16 boxes of it 1430 and 1480 us, 16 boxes of 96^3 758 and 830 us), except with two
@@ -87,7 +90,7 @@ template <typename T, int N> struct Ops {
       const bool one_shot = choice == 0 || (choice < 0 && N <= 128 && !PAIRS);
       if ((one_shot && nouter <= 65535) || cdiv(ncols, TB) * (long long)nf * nouter >= (1LL << 31)) {
         if constexpr (PAIRS) return colpass2<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
-        else return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s);
+        else return colpass<INV>(p, kid, LdRowsC<T, N, IN_MAP, RS>{in}, st, ncols, nf, nouter, tw, s, N <= 384);
       }
       ProfScope ps(p, kid, s);
       constexpr int threads = PAIRS ? Col2<N>::THREADS : Cfg<N>::COL_THREADS;
@@ -114,22 +117,22 @@ template <typename T, int N> struct Ops {
   using RS = RowStride<N>;
 
   static int z_c2r(ld_plan* p, const C* X, T* x, long long nrows, int ss, int Kin, T sc, long long xfs, long long Xfs,
-                   int nf, const C* tw, cudaStream_t s) {
+                   int nf, const C* tw, cudaStream_t s, bool dep) {
     ProfScope ps(p, KID_ZC2R, s);
     auto k = k_z_c2r<T, N>;
     if (int rc = set_smem(k, Z_SMEM)) return rc;
     dim3 grid((unsigned)cdiv(nrows / 2, Z::UNITS1), (unsigned)nf);
-    LD_CUDA_CHECK(launch_dep(true, k, grid, Z::THREADS1, Z_SMEM, s, X, x, nrows, ss, Kin, sc, xfs, Xfs, tw));
+    LD_CUDA_CHECK(launch_dep(dep, k, grid, Z::THREADS1, Z_SMEM, s, X, x, nrows, ss, Kin, sc, xfs, Xfs, tw));
     return LD_OK;
   }
 
   static int z_r2c(ld_plan* p, const T* x, C* X, long long nrows, int ss, int Kout, int Kval, long long xfs, long long Xfs,
-                   int nf, const C* tw, cudaStream_t s) {
+                   int nf, const C* tw, cudaStream_t s, bool dep) {
     ProfScope ps(p, KID_ZR2C, s);
     auto k = k_z_r2c<T, N>;
     if (int rc = set_smem(k, Z_SMEM)) return rc;
     dim3 grid((unsigned)cdiv(nrows / 2, Z::UNITS1), (unsigned)nf);
-    LD_CUDA_CHECK(launch_dep(true, k, grid, Z::THREADS1, Z_SMEM, s, x, X, nrows, ss, Kout, Kval, xfs, Xfs, tw));
+    LD_CUDA_CHECK(launch_dep(dep, k, grid, Z::THREADS1, Z_SMEM, s, x, X, nrows, ss, Kout, Kval, xfs, Xfs, tw));
     return LD_OK;
   }
 
@@ -138,13 +141,14 @@ template <typename T, int N> struct Ops {
     const int Nf = p->Nf;
     const C* tw = (const C*)p->tw;
     const long long NN = (long long)N * N;
-    if (int rc = z_r2c(p, u, fu, NN, Nf, Nf, Nf, NN * N, NN * Nf, ncomp, tw, s)) return rc;
+    const bool dep = early_transform(ncomp * NN * Nf);
+    if (int rc = z_r2c(p, u, fu, NN, Nf, Nf, Nf, NN * N, NN * Nf, ncomp, tw, s, dep)) return rc;
     // y pass in place: columns kz (Nf), rows y, outer x
     auto yio = io(fu, NN * Nf, (long long)N * Nf);
-    if (int rc = colpass<false>(p, KID_YFWD, LdRowsC<T, N, false, RS::YF>{yio}, StRowsC<T, N, false, RS::YF>{yio}, Nf, ncomp, N, tw, s)) return rc;
+    if (int rc = colpass<false>(p, KID_YFWD, LdRowsC<T, N, false, RS::YF>{yio}, StRowsC<T, N, false, RS::YF>{yio}, Nf, ncomp, N, tw, s, dep)) return rc;
     // x pass in place: columns (ky, kz) flat, rows x
     auto xio = io(fu, NN * Nf, 0);
-    return colpass<false>(p, KID_XPASS, LdRowsC<T, N, false, RS::XF>{xio}, StRowsC<T, N, false, RS::XF>{xio}, N * Nf, ncomp, 1, tw, s);
+    return colpass<false>(p, KID_XPASS, LdRowsC<T, N, false, RS::XF>{xio}, StRowsC<T, N, false, RS::XF>{xio}, N * Nf, ncomp, 1, tw, s, dep);
   }
 
   static int irfft_full(ld_plan* p, const C* fu, T* u, int ncomp, cudaStream_t s) {
@@ -156,13 +160,14 @@ template <typename T, int N> struct Ops {
     C* W = (C*)p->W2;
     for (int c0 = 0; c0 < ncomp; c0 += chunk) {
       const int nc = ncomp - c0 < chunk ? ncomp - c0 : chunk;
+      const bool dep = early_transform(nc * per);
       auto xin = io(fu + c0 * per, per, 0);
       auto xout = io(W, per, 0);
-      if (int rc = colpass<true>(p, KID_XPASS, LdRowsC<T, N, false, RS::XF>{xin}, StRowsC<T, N, false, RS::XF>{xout}, N * Nf, nc, 1, tw, s)) return rc;
+      if (int rc = colpass<true>(p, KID_XPASS, LdRowsC<T, N, false, RS::XF>{xin}, StRowsC<T, N, false, RS::XF>{xout}, N * Nf, nc, 1, tw, s, dep)) return rc;
       auto yio = io(W, per, (long long)N * Nf);
-      if (int rc = colpass<true>(p, KID_YINV, LdRowsC<T, N, false, RS::YF>{yio}, StRowsC<T, N, false, RS::YF>{yio}, Nf, nc, N, tw, s)) return rc;
+      if (int rc = colpass<true>(p, KID_YINV, LdRowsC<T, N, false, RS::YF>{yio}, StRowsC<T, N, false, RS::YF>{yio}, Nf, nc, N, tw, s, dep)) return rc;
       const T sc = T(1.0 / (double(N) * N * N));
-      if (int rc = z_c2r(p, W, u + (long long)c0 * NN * N, NN, Nf, Nf, sc, NN * N, per, nc, tw, s)) return rc;
+      if (int rc = z_c2r(p, W, u + (long long)c0 * NN * N, NN, Nf, Nf, sc, NN * N, per, nc, tw, s, dep)) return rc;
     }
     return LD_OK;
   }
@@ -180,12 +185,12 @@ template <typename T, int N> struct Ops {
       const int nc = ncomp - c0 < 6 ? ncomp - c0 : 6;
       auto xin = io(uk + c0 * cs, cs, 0);
       auto xout = io(W1, w1s, 0);
-      if (int rc = colpass<true>(p, KID_XPASS, LdRowsC<T, N, true, RS::XC>{xin}, StRowsC<T, N, false, RS::XC>{xout}, My * Mzp, nc, 1, tw, s)) return rc;
+      if (int rc = colpass<true>(p, KID_XPASS, LdRowsC<T, N, true, RS::XC>{xin}, StRowsC<T, N, false, RS::XC>{xout}, My * Mzp, nc, 1, tw, s, true)) return rc;
       auto yin = io(W1, w1s, (long long)My * Mzp);
       auto yout = io(W2, w2s, (long long)N * Mzp);
-      if (int rc = colpass<true>(p, KID_YINV, LdRowsC<T, N, true, RS::YC>{yin}, StRowsC<T, N, false, RS::YC>{yout}, Mzp, nc, N, tw, s)) return rc;
+      if (int rc = colpass<true>(p, KID_YINV, LdRowsC<T, N, true, RS::YC>{yin}, StRowsC<T, N, false, RS::YC>{yout}, Mzp, nc, N, tw, s, true)) return rc;
       const T sc = T(1.0 / (double(N) * N * N));
-      if (int rc = z_c2r(p, W2, u + (long long)c0 * NN * N, NN, Mzp, kc + 1, sc, NN * N, w2s, nc, tw, s)) return rc;
+      if (int rc = z_c2r(p, W2, u + (long long)c0 * NN * N, NN, Mzp, kc + 1, sc, NN * N, w2s, nc, tw, s, true)) return rc;
     }
     return LD_OK;
   }
@@ -200,13 +205,13 @@ template <typename T, int N> struct Ops {
     const long long w1s = (long long)N * My * Mzp, w2s = NN * Mzp;
     for (int c0 = 0; c0 < ncomp; c0 += 6) {
       const int nc = ncomp - c0 < 6 ? ncomp - c0 : 6;
-      if (int rc = z_r2c(p, u + (long long)c0 * NN * N, W2, NN, Mzp, Mzp, kc + 1, NN * N, w2s, nc, tw, s)) return rc;
+      if (int rc = z_r2c(p, u + (long long)c0 * NN * N, W2, NN, Mzp, Mzp, kc + 1, NN * N, w2s, nc, tw, s, true)) return rc;
       auto yin = io(W2, w2s, (long long)N * Mzp);
       auto yout = io(W1, w1s, (long long)My * Mzp);
-      if (int rc = colpass<false>(p, KID_YFWD, LdRowsC<T, N, false, RS::YC>{yin}, StRowsC<T, N, true, RS::YC>{yout}, Mzp, nc, N, tw, s)) return rc;
+      if (int rc = colpass<false>(p, KID_YFWD, LdRowsC<T, N, false, RS::YC>{yin}, StRowsC<T, N, true, RS::YC>{yout}, Mzp, nc, N, tw, s, true)) return rc;
       auto xin = io(W1, w1s, 0);
       auto xout = io(uk + c0 * cs, cs, 0);
-      if (int rc = colpass<false>(p, KID_XPASS, LdRowsC<T, N, false, RS::XC>{xin}, StCube<T, N>{xout}, My * Mzp, nc, 1, tw, s)) return rc;
+      if (int rc = colpass<false>(p, KID_XPASS, LdRowsC<T, N, false, RS::XC>{xin}, StCube<T, N>{xout}, My * Mzp, nc, 1, tw, s, true)) return rc;
     }
     return LD_OK;
   }
@@ -436,7 +441,8 @@ template <typename T, int N> struct Ops {
     const double L = 2.0 * M_PI;
     const vec4<T>* u4 = reinterpret_cast<const vec4<T>*>(u);
     auto k = stage == 1 ? k_droplet_stage<T, M, 1> : k_droplet_stage<T, M, 2>;
-    LD_CUDA_CHECK(launch_dep(early_droplets(n), k, dim3(gr), th, 0, s, u4, N, L, pos, vel, tau, a1, n, h, T(g), box));
+    LD_CUDA_CHECK(launch_dep(early_droplets(p, n, M != LD_INTERP_TRILINEAR), k, dim3(gr), th, 0, s, u4, N, L, pos, vel, tau, a1, n,
+                             h, T(g), box));
     return LD_OK;
   }
 
