@@ -44,7 +44,11 @@ template <typename T> __device__ __forceinline__ T ldg(const T* p) { return __ld
 // this one runs; its threads wait in grid_dep_wait until this grid has completed and its writes are
 // visible.  Both are no-ops for a kernel launched without the attribute.  Kernels call grid_dep_wait
 // before they touch anything that another kernel writes or reads, and grid_dep_launch after it, so
-// that whatever runs before a kernel's own wait runs after its last predecessor but one.
+// that whatever runs before a kernel's own wait runs after its last predecessor but one.  The two
+// kernels of a training step, k_mlp_train_tc and k_mlp_reduce_adam, launch first: before its wait, the
+// kernel after one of them may run beside the training kernels before that one too, and must not touch
+// what training writes (weights, packed copies, moments, partial sums).  k_mlp_forward_tc, which loads
+// weights before its wait, always follows k_mlp_features, which waits first.
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep() {

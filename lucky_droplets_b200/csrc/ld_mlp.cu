@@ -1636,8 +1636,10 @@ int ld_mlp_train_epoch(const void* X, const float* T, const float* W, const uint
     const int64_t k = step0 + b + 1;  // Adam step of this batch
     const double lrk = lr_final > 0.0 ? lr * pow(lr_final / lr, (double)(k < total ? k : total) / (double)total) : lr;
     const float c1 = 1.f - powf(b1, (float)k), c2 = 1.f - powf(b2, (float)k);
-    // each launch may begin while the previous one finishes (programmatic dependent launch)
-    LD_CUDA_CHECK(launch_dep(true, k_mlp_train_tc, dim3(nblk), TR_THREADS, SMEM_TRAIN_TC, s, (const bf16*)X, T, W,
+    // each launch may begin while the previous one finishes (programmatic dependent launch), but for the
+    // first: it loads samples and their order before its wait, and the caller's kernel before it may
+    // have written them
+    LD_CUDA_CHECK(launch_dep(b > 0, k_mlp_train_tc, dim3(nblk), TR_THREADS, SMEM_TRAIN_TC, s, (const bf16*)X, T, W,
                              order + b * batch, (long long)batch, inv_norm, (const bf16*)packed, params, gpart,
                              lpart));
     LD_CUDA_CHECK(launch_dep(true, k_mlp_reduce_adam, dim3(gridn(OFF_FS, 256)), 256, 0, s, (const float*)gpart,

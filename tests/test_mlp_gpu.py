@@ -281,3 +281,37 @@ def test_packed_tile_copies(torch):
     t3 = tile(P_TW3, N3P, H)
     assert np.array_equal(t3[:N3], w3t[:, :H]) and not t3[N3:].any()
     assert np.array_equal(w1t[:, :M.D_IN], M.bf16(p["W1"]).T)  # W1t[o][k] = bf16(W1[k][o])
+
+
+def test_first_training_launch_waits_for_the_callers_kernel(torch):
+    """The training kernel loads samples and their order before it waits for its predecessor: right after
+    the update of the batch before, not after a kernel of the caller that may have written them.  Seen in
+    the edges of a captured epoch of two batches: only those between its own kernels are programmatic."""
+    import ctypes
+    from lucky_droplets_b200 import _lib
+    from lucky_droplets_b200._lib import check, ptr, stream_ptr
+    from lucky_droplets_b200.mlp import LearnedInterp
+    from lucky_droplets_b200.spectral import Plan
+    net = LearnedInterp(Plan(16, "f32"), seed=0)
+    L, batch = _lib.lib(), 128
+    X = torch.zeros((2 * batch, 208), dtype=torch.bfloat16, device="cuda")
+    T = torch.zeros((2 * batch, 3), dtype=torch.float32, device="cuda")
+    order = torch.arange(2 * batch, dtype=torch.int32, device="cuda")
+    work = torch.empty(int(L.ld_mlp_partial_floats(batch)), dtype=torch.float32, device="cuda")
+    acc = torch.zeros(1, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        order.add_(0)
+        check(L.ld_mlp_train_epoch(ptr(X), ptr(T), None, ptr(order), 2, batch, ptr(net.params), ptr(net.packed),
+                                   ptr(net.m), ptr(net.v), 0, 1e-3, 0.0, 2, ptr(work), ptr(acc), stream_ptr(None)))
+    handle, n = ctypes.c_void_p(int(graph.raw_cuda_graph())), ctypes.c_size_t(16)
+    ends, data = [(ctypes.c_void_p * 16)() for _ in range(2)], (ctypes.c_uint8 * (8 * 16))()
+    assert ctypes.CDLL("libcuda.so.1").cuGraphGetEdges_v2(handle, *ends, data, ctypes.byref(n)) == 0
+    edges = {ends[0][i]: (ends[1][i], data[8 * i + 2]) for i in range(n.value)}  # CUgraphEdgeData.type
+    (node,) = set(edges) - {to for to, _ in edges.values()}
+    kinds = []
+    while node in edges:
+        node, kind = edges[node]
+        kinds.append(kind)
+    assert kinds == [0, 1, 1, 1]  # 1: CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC
