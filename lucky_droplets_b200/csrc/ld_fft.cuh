@@ -19,6 +19,7 @@
 // The other lengths N = 12 R2 R3 (360 = 12 5 6, 384 = 12 8 4, 192 = 12 4 4, 96 = 12 4 2) take
 // twelve elements per thread and three in-place stages with two exchanges (fft_run_12).
 #pragma once
+#include <cmath>
 #include <type_traits>
 
 #include "ld_common.cuh"
@@ -38,12 +39,26 @@ template <int N, int E> struct FftShape {
   static __host__ __device__ constexpr int ns(int s) { return ipow(E, s); }
 };
 
-// W_16^m = exp(-2 pi i m / 16) for m = 0..7 (forward sign).  INV conjugates.
+// W_16^m, W_16 = exp(-2 pi i / 16): W = c2 (1 -+ i) for even m, c1 (+-1 -+ i t) or c1 (+-t -+ i) for odd
+// m, with c2 = cos(pi/4), c1 = cos(pi/8), t = tan(pi/8), s1 = c1 t.
+template <typename T> struct W16 {
+  static constexpr double C1 = 0.92387953251128675613;
+  static constexpr T c1 = T(C1), s1 = T(0.38268343236508977173), t = T(0.41421356237309504880),
+                     c2 = T(0.70710678118654752440);
+  // c1 rounded to FP32 is almost as far off as a rounded number can be (3.1e-8), in every second
+  // butterfly of the radix-16 steps, so rows of 128 = 16 x 8 and 256 = 16 x 16 add its remainder l1
+  // (EXACT below).  Error against 64 bits of a right-hand side at 256^3 / 128^3: 4.56e-7 / 3.55e-7 without
+  // it and without the fused products, 4.27e-7 / 3.38e-7 now, 4.40e-7 / 3.50e-7 with rows of 8 x 8 x 4 and
+  // 8 x 8 x 2; time 363 -> 365 us and 58.8 -> 59.1 us.  In the columns too: 3.92e-7, 367 us.
+  static constexpr T l1 = T(C1 - double(T(C1)));
+  static constexpr bool exact(int n, int e, bool row) { return sizeof(T) == 4 && row && e == 16 && n <= 256; }
+};
+
+// q W_16^m for m = 0..7 (INV: by its conjugate)
 template <typename T, bool INV> __device__ __forceinline__ cplx<T> w16mul(cplx<T> x, int m) {
-  constexpr T c1 = T(0.92387953251128675613);  // cos(pi/8)
-  constexpr T s1 = T(0.38268343236508977173);  // sin(pi/8)
-  constexpr T c2 = T(0.70710678118654752440);  // cos(pi/4)
-  const T sg = INV ? T(1) : T(-1);             // sign of the sine part
+  using W = W16<T>;
+  constexpr T c1 = W::c1, s1 = W::s1, c2 = W::c2;
+  const T sg = INV ? T(1) : T(-1);  // sign of the sine part
   switch (m) {
     case 0: return x;
     case 4: return INV ? cmk(-x.y, x.x) : cmk(x.y, -x.x);  // * (+-i)
@@ -65,6 +80,48 @@ template <typename T, bool INV> __device__ __forceinline__ cplx<T> w16mul(cplx<T
   }
 }
 
+// The odd products: W v = c1 (ka a, kb b).
+template <bool INV> struct OddW16 {
+  static constexpr float sg = INV ? -1.f : 1.f, st = sg * W16<float>::t;
+  float ta, ka, kb;
+  bool xy;  // a = v.x + ta v.y, b = v.y - ta v.x; else a = v.y + ta v.x, b = v.x - ta v.y
+  __device__ __forceinline__ explicit OddW16(int m)
+      : ta(m == 1 || m == 3 ? st : -st), ka(m == 1 ? 1.f : (m == 7 ? -1.f : sg)),
+        kb(m == 1 ? 1.f : (m == 7 ? -1.f : -sg)), xy(m == 1 || m == 7) {}
+};
+
+// Butterfly p, q <- p +- q W_16^m.  FP32: the products accumulated onto p by fused multiply-adds, six
+// operations for an odd m (ten with EXACT) instead of eight with the product rounded first.  FP64 keeps
+// the plain form: the fused one has a longer chain (one field forward at 128^3 24.4 -> 25.6 us).
+template <typename T, bool INV, bool EXACT> __device__ __forceinline__ void butterfly(cplx<T>& p, cplx<T>& q, int m) {
+  using W = W16<T>;
+  const cplx<T> u = p, v = q;
+  if (sizeof(T) == 8 || m == 0 || m == 4) {
+    const cplx<T> w = w16mul<T, INV>(v, m);
+    p = cadd(u, w);
+    q = csub(u, w);
+  } else if (m == 2 || m == 6) {
+    const T s = v.x + v.y, d = v.x - v.y;
+    // W^2 v = c2 (s, -d) forward, c2 (d, s) inverse; W^6 v = c2 (-d, -s) forward, c2 (-s, d) inverse
+    const T a = m == 2 ? (INV ? d : s) : (INV ? s : d), b = m == 2 ? (INV ? s : d) : (INV ? d : s);
+    const T ka = m == 2 ? W::c2 : -W::c2, kb = INV ? W::c2 : -W::c2;
+    p = cmk(std::fma(a, ka, u.x), std::fma(b, kb, u.y));
+    q = cmk(std::fma(a, -ka, u.x), std::fma(b, -kb, u.y));
+  } else {
+    const OddW16<INV> o(m);
+    const T ta = o.ta, ka = o.ka, kb = o.kb;
+    const T a = o.xy ? std::fma(v.y, ta, v.x) : std::fma(v.x, ta, v.y);
+    const T b = o.xy ? std::fma(v.x, -ta, v.y) : std::fma(v.y, -ta, v.x);
+    cplx<T> up = u, uq = u;
+    if constexpr (EXACT) {
+      up = cmk(std::fma(a, ka * W::l1, u.x), std::fma(b, kb * W::l1, u.y));
+      uq = cmk(std::fma(a, -ka * W::l1, u.x), std::fma(b, -kb * W::l1, u.y));
+    }
+    p = cmk(std::fma(a, ka * W::c1, up.x), std::fma(b, kb * W::c1, up.y));
+    q = cmk(std::fma(a, -ka * W::c1, uq.x), std::fma(b, -kb * W::c1, uq.y));
+  }
+}
+
 __host__ __device__ constexpr int bitrev(int i, int bits) {
   return bits == 0 ? 0 : ((i & 1) << (bits - 1)) | bitrev(i >> 1, bits - 1);
 }
@@ -73,19 +130,16 @@ __host__ __device__ constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n
 // One radix-2 pass (butterfly span LEN) of an in-place length-R DIT DFT, then the next pass.
 // LEN is a template constant so every loop has a compile-time trip count and every index into
 // a[] is static: the array stays in registers.
-template <typename T, int R, int LEN, bool INV> __device__ __forceinline__ void dft_pass(cplx<T>* a) {
+template <typename T, int R, int LEN, bool INV, bool EXACT> __device__ __forceinline__ void dft_pass(cplx<T>* a) {
   if constexpr (LEN <= R) {
 #pragma unroll
     for (int i = 0; i < R; i += LEN) {
 #pragma unroll
       for (int q = 0; q < LEN / 2; ++q) {
-        const cplx<T> u = a[i + q];
-        const cplx<T> v = w16mul<T, INV>(a[i + q + LEN / 2], q * (16 / LEN));
-        a[i + q] = cadd(u, v);
-        a[i + q + LEN / 2] = csub(u, v);
+        butterfly<T, INV, EXACT>(a[i + q], a[i + q + LEN / 2], q * (16 / LEN));
       }
     }
-    dft_pass<T, R, 2 * LEN, INV>(a);
+    dft_pass<T, R, 2 * LEN, INV, EXACT>(a);
   }
 }
 
@@ -103,10 +157,10 @@ template <typename T, int R, int I> __device__ __forceinline__ void bitrev_swaps
 }
 
 // In-place length-R DFT of a[0..R-1] (natural order in and out), R in {1,2,4,8,16}.
-template <typename T, int R, bool INV> __device__ __forceinline__ void dft(cplx<T>* a) {
+template <typename T, int R, bool INV, bool EXACT = false> __device__ __forceinline__ void dft(cplx<T>* a) {
   if constexpr (R > 1) {
     bitrev_swaps<T, R, 0>(a);
-    dft_pass<T, R, 2, INV>(a);
+    dft_pass<T, R, 2, INV, EXACT>(a);
   }
 }
 
@@ -388,7 +442,7 @@ __device__ __forceinline__ void fft_stage(cplx<T>* a, cplx<T>* sbuf, int sstride
 #pragma unroll
     for (int r = 1; r < R; ++r) x[q * R + r] = cmul(x[q * R + r], tw_at<T, N, E, INV>(tw, Pipe<N, E>::first(s) + q * (R - 1) + r - 1,
                                                                             r * k * (N / (Ns * R))));
-    dft<T, R, INV>(x + q * R);
+    dft<T, R, INV, W16<T>::exact(N, E, PAD)>(x + q * R);
     if constexpr (s < S - 1) {
       const int base = (b / Ns) * Ns * R + k;
 #pragma unroll
@@ -410,7 +464,7 @@ template <typename T, int N, int E, bool INV, bool PAD, class Tw, class Sync>
 __device__ __forceinline__ void fft_run(cplx<T>* a, cplx<T>* sbuf, int sstride, int j, const Tw& tw, Sync sync) {
   if constexpr (is_pow2(N)) {
     using Sh = FftShape<N, E>;
-    dft<T, E, INV>(a);  // stage 0: radix E, Ns = 1, no twiddles
+    dft<T, E, INV, W16<T>::exact(N, E, PAD)>(a);  // stage 0: radix E, Ns = 1, no twiddles
     if constexpr (Sh::S > 1) {
 #pragma unroll
       for (int r = 0; r < E; ++r) sbuf[sidx<T, N, E, PAD>(j * E + r) * sstride] = a[r];
@@ -436,11 +490,9 @@ struct C2 {
 __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
 
-// Butterfly u +- v W_16^m of both transforms.
-template <bool INV> __device__ __forceinline__ void butterfly2(C2& p, C2& q, int m) {
-  constexpr float c1 = 0.92387953251128675613f;  // cos(pi/8)
-  constexpr float s1 = 0.38268343236508977173f;  // sin(pi/8)
-  constexpr float c2 = 0.70710678118654752440f;  // cos(pi/4)
+// The butterfly of both transforms.
+template <bool INV, bool EXACT> __device__ __forceinline__ void butterfly2(C2& p, C2& q, int m) {
+  using W = W16<float>;
   const C2 u = p, v = q;
   if (m == 0) {
     p.x = __fadd2_rn(u.x, v.x);
@@ -456,29 +508,35 @@ template <bool INV> __device__ __forceinline__ void butterfly2(C2& p, C2& q, int
     q.y = INV ? sy : ay;
   } else if (m == 2 || m == 6) {
     const float2 s = __fadd2_rn(v.x, v.y), d = sub2(v.x, v.y);
-    // W^2 v = c2 (s, -d) forward, c2 (d, s) inverse; W^6 v = c2 (-d, -s) forward, c2 (-s, d) inverse
     const float2 a = m == 2 ? (INV ? d : s) : (INV ? s : d), b = m == 2 ? (INV ? s : d) : (INV ? d : s);
-    const float ka = m == 2 ? c2 : -c2, kb = m == 2 ? (INV ? c2 : -c2) : (INV ? c2 : -c2);
+    const float ka = m == 2 ? W::c2 : -W::c2, kb = INV ? W::c2 : -W::c2;
     p.x = __ffma2_rn(a, f2(ka), u.x);
     p.y = __ffma2_rn(b, f2(kb), u.y);
     q.x = __ffma2_rn(a, f2(-ka), u.x);
     q.y = __ffma2_rn(b, f2(-kb), u.y);
   } else {
-    const float wr = m == 1 ? c1 : (m == 3 ? s1 : (m == 5 ? -s1 : -c1));
-    const float wi = (INV ? 1.f : -1.f) * (m == 1 || m == 7 ? s1 : c1);
-    p.x = __ffma2_rn(v.x, f2(wr), __ffma2_rn(v.y, f2(-wi), u.x));
-    p.y = __ffma2_rn(v.y, f2(wr), __ffma2_rn(v.x, f2(wi), u.y));
-    q.x = __ffma2_rn(v.x, f2(-wr), __ffma2_rn(v.y, f2(wi), u.x));
-    q.y = __ffma2_rn(v.y, f2(-wr), __ffma2_rn(v.x, f2(-wi), u.y));
+    const OddW16<INV> o(m);
+    const float ka = o.ka, kb = o.kb;
+    const float2 a = o.xy ? __ffma2_rn(v.y, f2(o.ta), v.x) : __ffma2_rn(v.x, f2(o.ta), v.y);
+    const float2 b = o.xy ? __ffma2_rn(v.x, f2(-o.ta), v.y) : __ffma2_rn(v.y, f2(-o.ta), v.x);
+    C2 up = u, uq = u;
+    if constexpr (EXACT) {
+      up = C2{__ffma2_rn(a, f2(ka * W::l1), u.x), __ffma2_rn(b, f2(kb * W::l1), u.y)};
+      uq = C2{__ffma2_rn(a, f2(-ka * W::l1), u.x), __ffma2_rn(b, f2(-kb * W::l1), u.y)};
+    }
+    p.x = __ffma2_rn(a, f2(ka * W::c1), up.x);
+    p.y = __ffma2_rn(b, f2(kb * W::c1), up.y);
+    q.x = __ffma2_rn(a, f2(-ka * W::c1), uq.x);
+    q.y = __ffma2_rn(b, f2(-kb * W::c1), uq.y);
   }
 }
-template <int R, int LEN, bool INV> __device__ __forceinline__ void dft_pass2(C2* a) {
+template <int R, int LEN, bool INV, bool EXACT> __device__ __forceinline__ void dft_pass2(C2* a) {
   if constexpr (LEN <= R) {
 #pragma unroll
     for (int i = 0; i < R; i += LEN)
 #pragma unroll
-      for (int q = 0; q < LEN / 2; ++q) butterfly2<INV>(a[i + q], a[i + q + LEN / 2], q * (16 / LEN));
-    dft_pass2<R, 2 * LEN, INV>(a);
+      for (int q = 0; q < LEN / 2; ++q) butterfly2<INV, EXACT>(a[i + q], a[i + q + LEN / 2], q * (16 / LEN));
+    dft_pass2<R, 2 * LEN, INV, EXACT>(a);
   }
 }
 template <int R, int I> __device__ __forceinline__ void bitrev_swaps2(C2* a) {
@@ -492,10 +550,10 @@ template <int R, int I> __device__ __forceinline__ void bitrev_swaps2(C2* a) {
     bitrev_swaps2<R, I + 1>(a);
   }
 }
-template <int R, bool INV> __device__ __forceinline__ void dft2(C2* a) {
+template <int R, bool INV, bool EXACT> __device__ __forceinline__ void dft2(C2* a) {
   if constexpr (R > 1) {
     bitrev_swaps2<R, 0>(a);
-    dft_pass2<R, 2, INV>(a);
+    dft_pass2<R, 2, INV, EXACT>(a);
   }
 }
 
@@ -553,7 +611,7 @@ __device__ __forceinline__ void fft_stage2(C2* a, float4* sbuf, int j, const TwL
 #pragma unroll
     for (int r = 1; r < R; ++r)
       x[q * R + r] = cmul2<INV>(x[q * R + r], tw.p[(Pipe<N, E>::first(s) + q * (R - 1) + r - 1) * NT]);
-    dft2<R, INV>(x + q * R);
+    dft2<R, INV, W16<float>::exact(N, E, STRIDE == 1)>(x + q * R);
     if constexpr (s < S - 1) {
       const int base = (b / Ns) * Ns * R + k;
 #pragma unroll
@@ -575,7 +633,7 @@ __device__ __forceinline__ void fft_stage2(C2* a, float4* sbuf, int j, const TwL
 // Both transforms, powers of two: the register contract of fft_run().
 template <int N, int E, bool INV, int STRIDE, class Sync>
 __device__ __forceinline__ void fft_run2(C2* a, float4* sbuf, int j, const TwLane2<N, E>& tw, Sync sync) {
-  dft2<E, INV>(a);
+  dft2<E, INV, W16<float>::exact(N, E, STRIDE == 1)>(a);
 #pragma unroll
   for (int r = 0; r < E; ++r)
     sbuf[slot2<E, STRIDE>(j * E + r)] = make_float4(a[r].x.x, a[r].x.y, a[r].y.x, a[r].y.y);
