@@ -128,7 +128,12 @@ int ld_plan_create_boxes(ld_plan** out, int n, int precision, int nbox) {
     const int kc = p->kc, My = p->My, Mzp = p->Mzp, Nf = p->Nf;
     std::vector<int> cnt(Nf + 1, 0);
     const long long kmax2 = (long long)Nf * Nf - Nf;
-    auto shell_of = [&](long long k2) { int s = 0; while ((long long)s * s + s < k2) ++s; return s; };
+    // round(sqrt(k2)), the smallest s with s^2 + s >= k2.  (Counting s up from 0 made a plan of 256^3 in 84
+    // or in 129 ms, by where the loop fell in the library.)
+    auto shell_of = [](long long k2) {
+      const int s = (int)std::sqrt((double)k2);
+      return (long long)s * s + s < k2 ? s + 1 : s;
+    };
     std::vector<std::pair<int, int>> items;
     items.reserve((size_t)p->cube_elems());
     for (int ix = 0; ix < My; ++ix)
