@@ -78,7 +78,7 @@ __device__ __forceinline__ void mma_f64(double (&c)[4], double2 a, double b) {
 // pipe) for eight shared-memory wavefronts.  1e4 points at 256^3, FP32 spectrum: 30.4 ms with a
 // thread per point and a phase recurrence per mode (16 FP64 operations a mode), 6.25 ms here, 25 of
 // the 36.7 TFLOP/s that the pipe gives these products, tiles' padding not counted.  P = 128 reuses each staged row for 128 points and
-// still leaves room for the ring up to kc = 93; larger grids have columns of 64 points.
+// still leaves room for the ring up to kc = 89; larger grids have columns of 64 points.
 // Partial sums of the kx planes are added in block order afterwards (deterministic).
 template <int P>
 __global__ void __launch_bounds__(2 * P, 1)

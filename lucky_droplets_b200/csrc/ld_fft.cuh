@@ -283,10 +283,12 @@ __host__ __device__ constexpr bool is_pow2(int n) { return n > 0 && (n & (n - 1)
 // The exchange buffer holds (k1, a + R3 c) at slot S(k1) + a + R3 c.  Stage 3's butterflies t = k1 +
 // 12 c = j + NT q leave their outputs at j + NT (q + (12 / R3) d), the thread's own positions (the
 // register contract), and stage 2 works in place, so two barriers separate the three stages.
-// S(k1) = PITCH k1 + (k1 >> SH) makes the accesses of all stages free of bank conflicts (360 in
-// FP64: 10% more than conflict-free), found by enumerating the bank groups of each half-warp
-// (FP32) or quarter-warp (FP64) over pitches and skews; ROW is the row buffer's length, rows of a
-// warp side by side included in the enumeration.
+// S(k1) = PITCH k1 + (k1 >> SH), the pitch and skew from an enumeration of the bank groups of each
+// half-warp (FP32) or quarter-warp (FP64), rows of a warp side by side: stages 1 and 2 are free of bank
+// conflicts (stage 2 of 360 in FP64: 10% more wavefronts), stage 3, whose lanes wrap past k1 = 11, takes
+// 4/3 (FP64, FP32 96), 3/2 (FP64 360) or 2 (FP32) times as many.  A transform takes 1.08 (FP64, FP32 96),
+// 1.25 (FP32) and, with the copies of lanes 0 and 1 that 360 has in its last quarter-warp, 1.21 (FP64
+// 360) times the wavefronts without conflicts.  ROW is the row buffer's length.
 template <typename T, int N> struct Len12 {
   static_assert(N == 360 || N == 384 || N == 192 || N == 96, "length 12 R2 R3");
   static constexpr int NT = N / 12;

@@ -1,5 +1,5 @@
 // Launch sequences for one (precision, N) instance.  Included by the ld_inst_*.cu units, each
-// of which instantiates one OpsTable; compiling the twelve instances separately keeps the build
+// of which instantiates one OpsTable; compiling the twenty instances separately keeps the build
 // parallel.
 #pragma once
 #include <cmath>

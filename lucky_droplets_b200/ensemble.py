@@ -12,9 +12,9 @@ per-box forcing.  The droplets of all boxes live in one set of arrays, each drop
 box; one droplet launch per stage samples each droplet's own box, and one multi-box collider
 (cells keyed box-major) sorts, searches and counts the pairs of every box.  `steps_per_graph`
 steps are captured into one CUDA graph, so one graph launch advances every box by that many
-steps with no host work between the kernels.  `autotune()` picks the launch variants of the
-strided transform passes on the multi-box plan (one-shot tiles or pipelined CTAs, 1..3 per SM) and
-the steps per graph.  With several ranks the boxes are dealt out round-robin by box index; there
+steps with no host work between the kernels.  `autotune()` picks the steps per
+graph; construction times the launch variants of the strided y passes on the multi-box plan
+(one-shot tiles or pipelined CTAs, 1..3 per SM; grids up to 64 have none).  With several ranks the boxes are dealt out round-robin by box index; there
 is no exchange between boxes, per-box results are gathered on the host.
 
     python -m lucky_droplets_b200.ensemble [--boxes 64] [--N 64] [--steps 2000]
@@ -240,7 +240,8 @@ class Ensemble:
 
     def autotune(self, steps_per_graph=(5, 10, 20), trial_graphs=2):
         """The launch variants of the strided transform passes are timed on the multi-box plan at
-        construction (ld_plan_autotune: one-shot tiles, or pipelined with 1, 2, 3 CTAs per SM);
+        construction (ld_plan_autotune: one-shot tiles, or pipelined with 1, 2, 3 CTAs per SM; grids
+        up to 64, which have no separate y pass, report -1);
         here the steps per graph are picked by timing `trial_graphs` rounds of replays of each
         candidate (a round visits every phase of the re-sorting period once, after a first round
         that captures and uploads the graphs; the trial steps advance the boxes like any other
