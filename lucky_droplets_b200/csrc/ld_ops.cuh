@@ -281,7 +281,7 @@ template <typename T, int N> struct Ops {
     }
   }
   static int autotune_y(ld_plan* p, cudaStream_t s, double* ms) {
-    const int My = p->My, Mzp = p->Mzp, kc = p->kc;
+    const int My = p->My, Mzp = p->Mzp;
     const C* tw = (const C*)p->tw;
     C* W1 = (C*)p->W1;
     C* W2 = (C*)p->W2;

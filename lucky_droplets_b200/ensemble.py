@@ -12,10 +12,11 @@ per-box forcing.  The droplets of all boxes live in one set of arrays, each drop
 box; one droplet launch per stage samples each droplet's own box, and one multi-box collider
 (cells keyed box-major) sorts, searches and counts the pairs of every box.  `steps_per_graph`
 steps are captured into one CUDA graph, so one graph launch advances every box by that many
-steps with no host work between the kernels.  `autotune()` picks the steps per
-graph; construction times the launch variants of the strided y passes on the multi-box plan
-(one-shot tiles or pipelined CTAs, 1..3 per SM; grids up to 64 have none).  With several ranks the boxes are dealt out round-robin by box index; there
-is no exchange between boxes, per-box results are gathered on the host.
+steps with no host work between the kernels.  `autotune()` picks the steps per graph;
+construction times the launch variants of the strided y passes on the multi-box plan (one-shot
+tiles or pipelined CTAs, 1..3 per SM; grids up to 64 have none).  With several ranks the boxes are
+dealt out round-robin by box index; there is no exchange between boxes, per-box results are
+gathered on the host.
 
     python -m lucky_droplets_b200.ensemble [--boxes 64] [--N 64] [--steps 2000]
 """
